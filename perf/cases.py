@@ -13,6 +13,8 @@ Kinds of case:
   experts   the owner side of the expert-parallel layer: rows with their slots given, foreign slots -1
   dsa_bf16  sparse MLA decode on a bf16 cache; `ids` flat (physical rows) or paged (positions + block table +
             valid lengths)
+
+``exact`` states the result of a pass in 64-bit torch arithmetic, for measuring how far an implementation is off.
 """
 import importlib
 import math
@@ -102,9 +104,8 @@ def _normal(shape, seed, sigma, dtype=torch.float32):
     return b200.fill_normal_(t, seed, sigma)
 
 
-def _fp8_layer(c, seed):
-    """Weights of E experts ~ N(0, 0.02) in 128x128 blocks, router weights with unit-variance logits, and the
-    layer object a serving program keeps."""
+def _fp8_weights(c, seed):
+    """Weights of E experts ~ N(0, 0.02) in 128x128 blocks, router weights with unit-variance logits."""
     E, K, D, I = c["E"], c["K"], c["D"], c["I"]
     pow2 = c.get("option") == "pow2"
     w1q = torch.empty((E, 2 * I, D), dtype=torch.uint8, device=DEV)
@@ -115,8 +116,14 @@ def _fp8_layer(c, seed):
     b200.fill_normal_fp8_w128_(w2q, w2s, seed * 16 + 2, 0.02, pow2=pow2)
     gate_w = _normal((E, D), seed * 16 + 3, D ** -0.5)
     bias = _normal((E,), seed * 16 + 4, 0.01)
+    return gate_w, bias, w1q, w1s, w2q, w2s
+
+
+def _fp8_layer(c, seed):
+    """The layer object a serving program keeps."""
+    gate_w, bias, w1q, w1s, w2q, w2s = _fp8_weights(c, seed)
     flags = {"pow2": b200.MOE_POW2_SCALES, "fixed_order": b200.MOE_DETERMINISTIC}.get(c.get("option"), 0)
-    layer = b200.MoeFp8Layer(gate_w, bias, w1q, w1s, w2q, w2s, K, b200.SCORE_SIGMOID_GROUPED, N_GROUP, TOPK_GROUP,
+    layer = b200.MoeFp8Layer(gate_w, bias, w1q, w1s, w2q, w2s, c["K"], b200.SCORE_SIGMOID_GROUPED, N_GROUP, TOPK_GROUP,
                              ROUTED_SCALE, flags=flags)
     if c["layout"] == "packed":
         layer.pack(free_unpacked=True)
@@ -218,6 +225,113 @@ def run(s):
     b200.dsa_forward_bf16_paged(s["qn"], s["qp"], s["kc"], s["kp"], s["v"], s["pos"], s["table"], s["out"], s["cfg"],
                                 valid_len=s["valid"])
     return s["out"]
+
+
+# ---------------------------------------------------------------------------------------------
+# the same results in 64 bits
+# ---------------------------------------------------------------------------------------------
+def _blocks128(x, pow2):
+    """1x128 blocks: e4m3 values and their scale (amax / 448, or the smallest power of two not below it)."""
+    b = x.double().reshape(x.shape[0], -1, 128)
+    s = (b.abs().amax(-1) / 448.0).float().double()
+    if pow2:
+        s = torch.exp2(torch.ceil(torch.log2(s)))
+    s = torch.where(s > 0, s, torch.ones_like(s))
+    q = (b / s[..., None]).float().clamp(-448.0, 448.0).to(torch.float8_e4m3fn).double()
+    return q.reshape(x.shape), s
+
+
+def _times_scale(q, s):
+    return (q.reshape(*s.shape, 128) * s[..., None]).reshape(q.shape)
+
+
+def _weight64(q, s):
+    n, k = q.shape
+    return (q.view(torch.float8_e4m3fn).double().reshape(n // 128, 128, k // 128, 128) * s.double()[:, None, :, None]).reshape(n, k)
+
+
+def _grouped_choice64(x, gate_w, bias, K):
+    s = torch.sigmoid(x @ gate_w.double().T)
+    c = s + bias.double()
+    E = c.shape[1]
+    groups = c.reshape(-1, N_GROUP, E // N_GROUP)
+    kept = groups.topk(min(2, E // N_GROUP), dim=2).values.sum(2).topk(TOPK_GROUP, dim=1).indices
+    open_ = torch.zeros(groups.shape[:2], dtype=torch.bool, device=DEV).scatter_(1, kept, True)
+    c = torch.where(open_.repeat_interleave(E // N_GROUP, dim=1), c, torch.full_like(c, -math.inf))
+    ids = c.topk(K, dim=1).indices
+    w = s.gather(1, ids)
+    return ids, w / w.sum(1, keepdim=True) * ROUTED_SCALE
+
+
+def _experts64(x, ids, w, weights, pow2=None):
+    """sum over a row's experts of w * W2 quant(silu(W1g x) * W1u x); pow2 None: no quantisation in between."""
+    out = torch.zeros_like(x)
+    for e in range(len(weights)):
+        row, slot = (ids == e).nonzero(as_tuple=True)
+        if len(row) == 0:
+            continue
+        w1, w2 = weights[e]
+        h = x[row] @ w1.T
+        I = h.shape[1] // 2
+        a = torch.nn.functional.silu(h[:, :I]) * h[:, I:]
+        if pow2 is not None:
+            a = _times_scale(*_blocks128(a, pow2))
+        out.index_add_(0, row, (a @ w2.T) * w[row, slot][:, None])
+    return out
+
+
+class _Fp8Experts:
+    def __init__(self, w1q, w1s, w2q, w2s):
+        self.t = (w1q, w1s, w2q, w2s)
+
+    def __len__(self):
+        return self.t[0].shape[0]
+
+    def __getitem__(self, e):
+        w1q, w1s, w2q, w2s = self.t
+        return _weight64(w1q[e], w1s[e]), _weight64(w2q[e], w2s[e])
+
+
+def _attend64(q, k, v):
+    p = torch.softmax((q @ k.T) / math.sqrt(q.shape[1]), dim=1)
+    return p @ v
+
+
+def exact(case, seed):
+    c = case
+    kind = c["kind"]
+    if kind == "moe_f32":
+        s = prepare(c, seed)
+        x = s["x"].double()
+        p, ids = torch.softmax(x @ s["wg"].double().T, dim=1).topk(c["K"], dim=1)
+        return _experts64(x, ids, p / p.sum(1, keepdim=True), [(a.double(), b.double()) for a, b in zip(s["w1"], s["w2"])])
+    if kind == "dsa_f32":
+        s = prepare(c, seed)
+        k, v = torch.cat([s["kc"], s["kp"]], 1).double(), s["v"].double()
+        q = torch.cat([s["qn"], s["qp"]], 2).double()
+        return torch.stack([_attend64(q[i], k[s["idx"][i].long()], v[s["idx"][i].long()]) for i in range(c["Q"])])
+    if kind == "moe_fp8":
+        gate_w, bias, *experts = _fp8_weights(c, seed)
+        pow2 = c["option"] == "pow2"
+        xq, xs = _blocks128(_normal((c["T"], c["D"]), seed * 16 + 5, 1.0), pow2)
+        x = _times_scale(xq, xs)
+        ids, w = _grouped_choice64(x, gate_w, bias, c["K"])
+        return None, xs, _experts64(x, ids, w, _Fp8Experts(*experts), pow2)
+    if kind == "experts":
+        s = prepare(c, seed)
+        _, _, *experts = _fp8_weights(c, seed)
+        x = _times_scale(s["xq"].view(torch.float8_e4m3fn).double(), s["xs"].double())
+        return _experts64(x, s["rid"], s["rw"].double(), _Fp8Experts(*experts), False)
+    valid, table, pos, N = _decode_ids(c, seed)
+    s = prepare(c, seed)
+    kc, kp, v = (_normal((N, d), seed * 16 + i, 0.5, torch.bfloat16) for i, d in enumerate((512, 64, 512)))
+    out = []
+    for i in range(c["Q"]):
+        p = pos[i][pos[i] >= 0]
+        r = table[i][p // 64].long() * 64 + p % 64
+        q = torch.cat([s["qn"][i], s["qp"][i]], 1).double()
+        out.append(_attend64(q, torch.cat([kc[r], kp[r]], 1).double(), v[r].double()))
+    return torch.stack(out)
 
 
 # ---------------------------------------------------------------------------------------------
