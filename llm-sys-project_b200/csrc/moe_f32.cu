@@ -8,7 +8,11 @@
 //                      scatter-add fused; replaces tiled_gemm_bt_kernel + scatter_kernel,
 //                      naive_moe.cu:458-468, :315-335)
 // Rows are addressed through the row -> (token, slot) map, so no gathered copy of the
-// activations is made and the host never learns the per-expert counts.
+// activations is made and the host never learns the per-expert counts.  Aligned shapes take the kernels of the
+// vector path below; these two serve the rest.
+#include <cfloat>
+
+#include "cluster_f32.cuh"
 #include "common.cuh"
 #include "moe_internal.cuh"
 
@@ -113,6 +117,320 @@ grouped_gemm_f32_kernel(const float* __restrict__ a_src,     // MODE 1: x [T,D];
     }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Vector path (D % 4 == 0, I % 4 == 0, 16-byte aligned tensors).  At these sizes (tens of tokens, weights of a few
+// MB to 100 MB) the layer is bound by launches, by latency and by how much of the weights is in flight, so:
+//   * three launches instead of eight: gate + selection + zero-fill of the output | GEMM1 | GEMM2, the later two
+//     launched with programmatic stream serialisation (their first weight tiles are on the way before the kernel
+//     in front of them has finished);
+//   * no permutation kernel when the id list is short (T * K <= GV_PAIRS): every GEMM block reads the ids and
+//     lists its expert's rows itself (a kilobyte against its 100 KB of weights);
+//   * weights stream through a four-stage cp.async ring; thread = (MT / 4) x 4 outputs of one quarter of each
+//     k-tile, operands read as 16-byte vectors along k from rows of 36 floats (odd multiple of 16 bytes: no bank
+//     conflicts), the four quarters are added at the end;
+//   * where the tiles do not fill the machine the reduction is split over a cluster of up to four CTAs and added in
+//     rank order through distributed shared memory, so an output still receives one addition per (token, expert).
+// T = 32, E = 8, K = 2, D = 128, I = 256: 66 -> 16 us a call; T = 128, E = 16, K = 2, D = 512, I = 1024: 355 -> 68 us
+// (100 MB of weights); error against 64-bit arithmetic 9.2e-7 -> 5.2e-7.
+// ---------------------------------------------------------------------------------------------
+constexpr int GV_KT = 32, GV_LD = GV_KT + 4, GV_ST = 4, GV_N = 64, GV_THREADS = 256, GV_PAIRS = 2048;
+
+__device__ __forceinline__ void gv_cp16(float* dst, const float* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ptx::smem_u32(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
+struct GvParams {
+    const float* a;          // MODE 1: x [T,D];  MODE 2: act [rows,I]
+    const float* w;          // MODE 1: W1 [E,2I,D]; MODE 2: W2 [E,D,I]
+    const int* ids;          // [T*K]
+    const int* offsets;      // with row_pair: permutation made beforehand (long id lists)
+    const int* row_pair;
+    const float* wts;        // MODE 2
+    float* dst;              // MODE 1: act [rows,I]; MODE 2: out [T,D]
+    int TK, K, D, I;
+};
+
+template <int MT>
+constexpr size_t gv_smem_bytes() { return sizeof(float) * (size_t)GV_ST * (GV_N + MT) * GV_LD; }
+
+// grid: (ceil(N / tile columns), row-tile walkers, E * cluster size); MT rows x 64 weight rows per tile
+template <int MODE, int MT>
+__global__ void __launch_bounds__(GV_THREADS)
+grouped_gemm_f32_vec_kernel(const GvParams p) {
+    extern __shared__ __align__(16) float gv_smem[];
+    __shared__ int s_pair[GV_PAIRS];
+    __shared__ int s_warp[GV_THREADS / 32];
+    constexpr int RT = MT / 4;                               // rows per thread
+    constexpr int STG = (GV_N + MT) * GV_LD;                 // floats per stage: weights, then activations
+    static_assert(4 * MT * GV_N <= GV_ST * STG, "the k-quarter sums reuse the ring");
+    uint32_t crank, csize;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(csize));
+    const int e = blockIdx.z / csize;
+    const int Kd = (MODE == 1) ? p.D : p.I, N = (MODE == 1) ? p.I : p.D;
+    const int n0 = blockIdx.x * ((MODE == 1) ? GV_N / 2 : GV_N);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nkt = (Kd + GV_KT - 1) / GV_KT, per = (nkt + (int)csize - 1) / (int)csize;
+    const int kt_b = min(nkt, (int)crank * per), nk = min(nkt, kt_b + per) - kt_b;
+
+    const float* we = p.w + (size_t)e * ((MODE == 1) ? (size_t)2 * p.I * p.D : (size_t)p.D * p.I);
+    // this thread's two 16-byte pieces of a weight tile: tile rows tid / 8 and tid / 8 + 32
+    const int lr = tid >> 3, lk = (tid & 7) * 4;
+    const float* wsrc[2];
+    bool wok[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int c = lr + 32 * i;
+        const int n = (MODE == 1) ? n0 + (c & 31) : n0 + c;
+        wok[i] = n < N;
+        wsrc[i] = we + (size_t)((MODE == 1 && c >= 32) ? p.I + (wok[i] ? n : 0) : (wok[i] ? n : 0)) * Kd;
+    }
+    auto load_w = [&](int j) {                               // k-tile kt_b + j into ring slot j % GV_ST
+        const int k = (kt_b + j) * GV_KT + lk;
+        float* d = gv_smem + (j % GV_ST) * STG + lr * GV_LD + lk;
+#pragma unroll
+        for (int i = 0; i < 2; i++) gv_cp16(d + 32 * i * GV_LD, wsrc[i] + (k < Kd ? k : 0), wok[i] && k < Kd);
+    };
+    // the weights do not depend on the kernel in front: the first tiles are requested before waiting for it
+    const bool early = blockIdx.y == 0;
+    if (early)
+        for (int j = 0; j < GV_ST - 1; j++)
+            if (j < nk) load_w(j);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+    // rows of this expert (ascending pairs) and, for the sorted position, the rows of lower experts
+    int cnt = 0, base = 0;
+    const int* rows = s_pair;
+    if (p.row_pair) {
+        base = p.offsets[e];
+        cnt = p.offsets[e + 1] - base;
+        rows = p.row_pair + base;
+    } else {
+        int lower = 0;
+        for (int p0 = 0; p0 < p.TK; p0 += GV_THREADS) {
+            const int id = (p0 + tid < p.TK) ? p.ids[p0 + tid] : -1;
+            const unsigned hit = __ballot_sync(0xffffffffu, id == e);
+            lower += (id >= 0 && id < e) ? 1 : 0;
+            if (lane == 0) s_warp[warp] = __popc(hit);
+            __syncthreads();
+            int before = 0, total = 0;
+#pragma unroll
+            for (int w = 0; w < GV_THREADS / 32; w++) {
+                const int n = s_warp[w];
+                before += (w < warp) ? n : 0;
+                total += n;
+            }
+            if (id == e) s_pair[cnt + before + __popc(hit & ((1u << lane) - 1))] = p0 + tid;
+            cnt += total;
+            __syncthreads();
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) lower += __shfl_xor_sync(0xffffffffu, lower, o);
+        if (lane == 0) s_warp[warp] = lower;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < GV_THREADS / 32; w++) base += s_warp[w];
+    }
+
+    const int tx = tid & 15, ty = (tid >> 4) & 3, kq = tid >> 6;
+    bool first = early;
+    for (int m0 = blockIdx.y * MT; m0 < cnt; m0 += gridDim.y * MT) {
+        const float* asrc = nullptr;
+        if (tid < MT * 8 && m0 + lr < cnt)
+            asrc = p.a + ((MODE == 1) ? (size_t)(rows[m0 + lr] / p.K) * Kd : (size_t)(base + m0 + lr) * Kd);
+        auto load_a = [&](int j) {
+            if (tid < MT * 8) {
+                const int k = (kt_b + j) * GV_KT + lk;
+                const bool ok = asrc != nullptr && k < Kd;
+                gv_cp16(gv_smem + (j % GV_ST) * STG + (GV_N + lr) * GV_LD + lk, ok ? asrc + k : p.a, ok);
+            }
+        };
+#pragma unroll
+        for (int j = 0; j < GV_ST - 1; j++) {
+            if (j < nk) {
+                if (!first) load_w(j);
+                load_a(j);
+            }
+            ptx::cp_async_commit();
+        }
+        first = false;
+        float acc[RT][4];
+#pragma unroll
+        for (int i = 0; i < RT; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
+        for (int j = 0; j < nk; j++) {
+            ptx::cp_async_wait<GV_ST - 2>();
+            __syncthreads();
+            const float* sb = gv_smem + (j % GV_ST) * STG;
+            const float* sa = sb + GV_N * GV_LD;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int k = (kq + 4 * h) * 4;
+                float4 b[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++) b[c] = *reinterpret_cast<const float4*>(sb + (tx + 16 * c) * GV_LD + k);
+#pragma unroll
+                for (int i = 0; i < RT; i++) {
+                    const float4 a = *reinterpret_cast<const float4*>(sa + (ty + 4 * i) * GV_LD + k);
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        acc[i][c] = fmaf(a.x, b[c].x, acc[i][c]); acc[i][c] = fmaf(a.y, b[c].y, acc[i][c]);
+                        acc[i][c] = fmaf(a.z, b[c].z, acc[i][c]); acc[i][c] = fmaf(a.w, b[c].w, acc[i][c]);
+                    }
+                }
+            }
+            if (j + GV_ST - 1 < nk) { load_w(j + GV_ST - 1); load_a(j + GV_ST - 1); }
+            ptx::cp_async_commit();
+        }
+        ptx::cp_async_wait<0>();
+        __syncthreads();                                     // the ring is free: quarter sums [kq][row][column]
+#pragma unroll
+        for (int i = 0; i < RT; i++)
+#pragma unroll
+            for (int c = 0; c < 4; c++) gv_smem[(kq * MT + ty + 4 * i) * GV_N + tx + 16 * c] = acc[i][c];
+        __syncthreads();
+        // add the quarters in place; thread = 4 consecutive columns
+        for (int o = tid; o < MT * GV_N / 4; o += GV_THREADS) {
+            float4* q = reinterpret_cast<float4*>(gv_smem) + o;
+            float4 s = q[0];
+#pragma unroll
+            for (int g = 1; g < 4; g++) {
+                const float4 v = q[g * MT * GV_N / 4];
+                s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+            }
+            q[0] = s;
+        }
+        if (csize > 1) cluster_sync(); else __syncthreads();
+        auto total4 = [&](int o) -> float4 {                 // the CTAs of the cluster in rank order
+            if (csize == 1) return reinterpret_cast<const float4*>(gv_smem)[o];
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (uint32_t r = 0; r < csize; r++) {
+                const float4 v = cluster_ld_f32x4(cluster_map(gv_smem + 4 * o, r));
+                s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+            }
+            return s;
+        };
+        if (MODE == 1) {
+            for (int o = (int)crank * GV_THREADS + tid; o < MT * GV_N / 8; o += (int)csize * GV_THREADS) {
+                const int m = o >> 3, c4 = o & 7;            // row, 4 activation columns: gate at 4 c4, up 32 further
+                if (m0 + m >= cnt || n0 + 4 * c4 >= N) continue;
+                const float4 g = total4(m * (GV_N / 4) + c4), u = total4(m * (GV_N / 4) + 8 + c4);
+                float4 r;
+                r.x = __fdiv_rn(g.x, 1.0f + expf(-g.x)) * u.x;   // silu as naive_moe.cu:308
+                r.y = __fdiv_rn(g.y, 1.0f + expf(-g.y)) * u.y;
+                r.z = __fdiv_rn(g.z, 1.0f + expf(-g.z)) * u.z;
+                r.w = __fdiv_rn(g.w, 1.0f + expf(-g.w)) * u.w;
+                *reinterpret_cast<float4*>(p.dst + (size_t)(base + m0 + m) * p.I + n0 + 4 * c4) = r;
+            }
+        } else {
+            for (int o = (int)crank * GV_THREADS + tid; o < MT * GV_N / 4; o += (int)csize * GV_THREADS) {
+                const int m = o >> 4, c4 = o & 15;
+                if (m0 + m >= cnt || n0 + 4 * c4 >= N) continue;
+                const float4 s = total4(o);
+                const int pair = rows[m0 + m];
+                const float wv = p.wts[pair];
+                float* d = p.dst + (size_t)(pair / p.K) * p.D + n0 + 4 * c4;
+                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(d), "f"(wv * s.x), "f"(wv * s.y), "f"(wv * s.z), "f"(wv * s.w)
+                             : "memory");
+            }
+        }
+        // the ring is refilled (and the CTA may leave) only when nobody reads the sums any more
+        if (csize > 1) cluster_sync(); else __syncthreads();
+    }
+    ptx::cp_async_wait<0>();                                 // tiles requested early for an expert without rows
+}
+
+// Router of the vector path: block = 8 tokens x all (at most 32) experts, thread = one (token, expert) chain in the
+// reference's order (multiply, then add, ascending d; naive_moe.cu:102-106), then one warp per token selects; the
+// exponentials and divisions are spread over the lanes, sums and the K-slot scan stay in the reference's order.
+// Also clears the block's output rows (GEMM2 adds into them).
+constexpr int GR_T = 8, GR_KT = 128, GR_LD = GR_KT + 4, GR_ST = 4, GR_MAXE = 32;
+constexpr size_t gr_smem_bytes(int E) { return sizeof(float) * (size_t)GR_ST * (E + GR_T) * GR_LD; }
+
+__global__ void __launch_bounds__(GR_T * GR_MAXE)
+gate_select_f32_kernel(const float* __restrict__ x, const float* __restrict__ wg, int* __restrict__ ids,
+                       float* __restrict__ wts, float* __restrict__ out, int T, int E, int K, int D) {
+    extern __shared__ __align__(16) float gr_smem[];
+    __shared__ float s_p[GR_T][GR_MAXE];
+    __shared__ float s_c[GR_T][GR_MAXE];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, t0 = blockIdx.x * GR_T;
+    const int rowsz = E + GR_T, nkt = (D + GR_KT - 1) / GR_KT;
+    auto load = [&](int j) {
+        float* st = gr_smem + (size_t)(j % GR_ST) * rowsz * GR_LD;
+        for (int i = tid; i < rowsz * (GR_KT / 4); i += blockDim.x) {
+            const int r = i / (GR_KT / 4), k = j * GR_KT + (i % (GR_KT / 4)) * 4;
+            const bool ok = k < D && (r < E || t0 + r - E < T);
+            const float* src = r < E ? wg + (size_t)r * D + k : x + (size_t)(t0 + r - E) * D + k;
+            gv_cp16(st + r * GR_LD + (i % (GR_KT / 4)) * 4, ok ? src : wg, ok);
+        }
+    };
+#pragma unroll
+    for (int j = 0; j < GR_ST - 1; j++) {
+        if (j < nkt) load(j);
+        ptx::cp_async_commit();
+    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int nrow = min(GR_T, T - t0);
+    for (int i = tid; i < nrow * (D / 4); i += blockDim.x)
+        reinterpret_cast<float4*>(out + (size_t)t0 * D)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int tok = tid / E, ex = tid - tok * E;
+    const bool on = tok < GR_T;
+    float acc = 0.0f;
+    for (int j = 0; j < nkt; j++) {
+        ptx::cp_async_wait<GR_ST - 2>();
+        __syncthreads();
+        if (on) {
+            const float* st = gr_smem + (size_t)(j % GR_ST) * rowsz * GR_LD;
+            const float *wr = st + ex * GR_LD, *xr = st + (E + tok) * GR_LD;
+            const int kn = min(GR_KT, D - j * GR_KT);
+#pragma unroll 8
+            for (int k = 0; k < kn; k += 4) {
+                const float4 a = *reinterpret_cast<const float4*>(xr + k), b = *reinterpret_cast<const float4*>(wr + k);
+                acc = __fadd_rn(acc, __fmul_rn(a.x, b.x)); acc = __fadd_rn(acc, __fmul_rn(a.y, b.y));
+                acc = __fadd_rn(acc, __fmul_rn(a.z, b.z)); acc = __fadd_rn(acc, __fmul_rn(a.w, b.w));
+            }
+        }
+        if (j + GR_ST - 1 < nkt) load(j + GR_ST - 1);
+        ptx::cp_async_commit();
+    }
+    ptx::cp_async_wait<0>();
+    if (on) s_p[tok][ex] = acc;
+    __syncthreads();
+    for (int tt = warp; tt < nrow; tt += blockDim.x / 32) {
+        // naive_moe.cu:109-141
+        const float lg = lane < E ? s_p[tt][lane] : -FLT_MAX;
+        float mx = -FLT_MAX;
+        for (int i = 0; i < E; i++) mx = fmaxf(mx, s_p[tt][i]);
+        __syncwarp();
+        const float pe = (float)exp((double)__fsub_rn(lg, mx));      // correctly rounded expf
+        if (lane < E) s_p[tt][lane] = pe;
+        __syncwarp();
+        float sum = 0.0f;
+        for (int i = 0; i < E; i++) sum = __fadd_rn(sum, s_p[tt][i]);
+        __syncwarp();
+        if (lane < E) s_p[tt][lane] = __fdiv_rn(pe, sum);
+        __syncwarp();
+        if (lane == 0) {
+            int* oi = ids + (size_t)(t0 + tt) * K;
+            float* ow = wts + (size_t)(t0 + tt) * K;
+            float* c = s_c[tt];
+            for (int k = 0; k < K; k++) { c[k] = -FLT_MAX; oi[k] = -1; }
+            for (int i = 0; i < E; i++) {
+                const float pv = s_p[tt][i];
+                int min_k = 0;
+                for (int k = 1; k < K; k++)
+                    if (c[k] < c[min_k]) min_k = k;
+                if (pv > c[min_k]) { c[min_k] = pv; oi[min_k] = i; }
+            }
+            float tot = 0.0f;
+            for (int k = 0; k < K; k++) tot = __fadd_rn(tot, c[k]);
+            for (int k = 0; k < K; k++) ow[k] = (tot > 0.0f) ? __fdiv_rn(c[k], tot) : c[k];
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // stage kernels (the reference's per-stage launchers; not on the fused path)
 // ---------------------------------------------------------------------------
@@ -195,6 +513,38 @@ __global__ void scatter_f32_kernel(const float* __restrict__ expert_out, const i
     atomicAdd(&out[(size_t)t * D + d], w * expert_out[(size_t)i * D + d]);
 }
 
+// one grouped GEMM launch of the vector path
+template <int MODE, int MT>
+static int launch_gemm_vec(const GvParams& p, int T, int E, int sm_count, cudaStream_t stream) {
+    static bool attr_done[64] = {false};
+    if (b200_first_call_on_device(attr_done))
+        B200_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_f32_vec_kernel<MODE, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)gv_smem_bytes<MT>()));
+    const int Kd = (MODE == 1) ? p.D : p.I, N = (MODE == 1) ? p.I : p.D;
+    const int nx = ceil_div(N, (MODE == 1) ? GV_N / 2 : GV_N);
+    // walkers over an expert's row tiles: the mean and a half (a block loops over the tiles beyond)
+    const int ny = max(1, min(ceil_div(T, MT), ceil_div(3 * (p.TK / E + 1), 2 * MT)));
+    // cluster over k: until there are about two blocks per SM, at least two k-tiles each
+    const int nkt = ceil_div(Kd, GV_KT);
+    int cs = 1;
+    while (cs < 4 && (long long)nx * E * cs * 2 <= 2ll * sm_count && nkt / (2 * cs) >= 2) cs *= 2;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(nx, ny, E * cs);
+    lc.blockDim = dim3(GV_THREADS);
+    lc.dynamicSmemBytes = gv_smem_bytes<MT>();
+    lc.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = cs;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr; lc.numAttrs = 2;
+    B200_CUDA_TRY(cudaLaunchKernelEx(&lc, grouped_gemm_f32_vec_kernel<MODE, MT>, p));
+    b200_count_launch(1);
+    B200_CUDA_TRY(cudaGetLastError());
+    return B200_OK;
+}
+
 extern "C" {
 
 int b200_moe_forward_f32(b200_ws* ws, const float* x, const float* gate_w, const float* w1, const float* w2,
@@ -227,14 +577,43 @@ int b200_moe_forward_f32(b200_ws* ws, const float* x, const float* gate_w, const
     WsCarver cv(ws->base);
     carve(cv, partials, ids, wts, counts, offsets, row_pair, act);
 
-    st = launch_gate_logits(x, nullptr, gate_w, partials, T, E, D, false, stream);
-    if (st) return st;
-    st = launch_route_select(partials, 1, nullptr, ids, wts, nullptr, nullptr, T, E, K, B200_SCORE_SOFTMAX, 1, 1,
-                             1.0f, stream);
-    if (st) return st;
-    st = launch_permute(ids, T, K, E, nullptr, true, counts, offsets, row_pair, stream);
-    if (st) return st;
-    B200_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(float) * (size_t)T * D, stream));   // naive_moe.cu:413
+    const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gate_w) | reinterpret_cast<uintptr_t>(w1) |
+                          reinterpret_cast<uintptr_t>(w2) | reinterpret_cast<uintptr_t>(out);
+    const bool vec = D % 4 == 0 && I % 4 == 0 && (all & 15) == 0 && (long long)E * 4 <= 65535;
+    const bool short_ids = vec && (long long)T * K <= GV_PAIRS;      // the GEMM blocks list their rows themselves
+    if (vec && E <= GR_MAXE && short_ids) {
+        static bool attr_done[64] = {false};
+        if (b200_first_call_on_device(attr_done))
+            B200_CUDA_TRY(cudaFuncSetAttribute(gate_select_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)gr_smem_bytes(GR_MAXE)));
+        gate_select_f32_kernel<<<ceil_div(T, GR_T), GR_T * GR_MAXE, gr_smem_bytes(E), stream>>>(x, gate_w, ids, wts, out, T, E, K, D);
+        b200_count_launch(1);
+        B200_CUDA_TRY(cudaGetLastError());
+    } else {
+        st = launch_gate_logits(x, nullptr, gate_w, partials, T, E, D, false, stream);
+        if (st) return st;
+        st = launch_route_select(partials, 1, nullptr, ids, wts, nullptr, nullptr, T, E, K, B200_SCORE_SOFTMAX, 1, 1,
+                                 1.0f, stream);
+        if (st) return st;
+        if (!short_ids) {
+            st = launch_permute(ids, T, K, E, nullptr, true, counts, offsets, row_pair, stream);
+            if (st) return st;
+        }
+        B200_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(float) * (size_t)T * D, stream));   // naive_moe.cu:413
+    }
+    if (vec) {
+        GvParams p{};
+        p.ids = ids; p.wts = wts; p.TK = T * K; p.K = K; p.D = D; p.I = I;
+        if (!short_ids) { p.offsets = offsets; p.row_pair = row_pair; }
+        // Row tiles of 16 or 32: an expert's rows should mostly fit one tile (each tile streams the weights again),
+        // and a half-empty tile of 32 costs as many multiply-adds as a full one.
+        const bool wide = (long long)T * K > 16ll * E;
+        p.a = x; p.w = w1; p.dst = act;
+        st = wide ? launch_gemm_vec<1, 32>(p, T, E, ws->sm_count, stream) : launch_gemm_vec<1, 16>(p, T, E, ws->sm_count, stream);
+        if (st) return st;
+        p.a = act; p.w = w2; p.dst = out;
+        return wide ? launch_gemm_vec<2, 32>(p, T, E, ws->sm_count, stream) : launch_gemm_vec<2, 16>(p, T, E, ws->sm_count, stream);
+    }
     dim3 g1(ceil_div(I, G_TN), ceil_div(T, G_TM), E);
     grouped_gemm_f32_kernel<1><<<g1, 256, 0, stream>>>(x, w1, offsets, row_pair, nullptr, act, K, D, I);
     dim3 g2(ceil_div(D, G_TN), ceil_div(T, G_TM), E);

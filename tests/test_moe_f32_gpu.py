@@ -160,3 +160,18 @@ def test_permute_counts_a_token_once_per_expert(b200, cuda):
     assert np.array_equal(counts.cpu().numpy(), oc)
     assert np.array_equal(offsets.cpu().numpy(), oo)
     assert np.array_equal(row_pair.cpu().numpy()[: oo[E]], orp)
+
+
+@pytest.mark.parametrize("T,E,K,D,I", [(1, 4, 2, 4, 4), (33, 16, 4, 68, 132), (128, 4, 4, 512, 1024), (9, 32, 2, 36, 40),
+                                       (700, 8, 3, 64, 64), (64, 40, 2, 128, 64), (17, 3, 1, 100, 260), (5, 2, 2, 33, 20)])
+def test_vector_path_edges(b200, cuda, T, E, K, D, I):
+    """Row tiles of 16 and 32 with remainders, column tiles and k-tiles cut short, split reductions, experts without
+    rows, a long id list (permutation kernel), more than 32 experts (general router) and an unaligned shape."""
+    rng = np.random.default_rng(T * 7 + E)
+    x = rng.normal(0, 1, (T, D)).astype(np.float32)
+    wg = rng.normal(0, D ** -0.5, (E, D)).astype(np.float32)
+    w1 = rng.normal(0, D ** -0.5, (E, 2 * I, D)).astype(np.float32)
+    w2 = rng.normal(0, I ** -0.5, (E, D, I)).astype(np.float32)
+    ids, wts, ref = oracle.moe_forward_f32(x, wg, w1, w2, K)
+    out = _run_forward(b200, cuda, x, wg, w1, w2, K)
+    assert np.abs(out - ref).max() < 1e-5 * max(1.0, np.abs(ref).max())
