@@ -193,27 +193,40 @@ __global__ void fill_normal_fp8_w128_kernel(uint8_t* q, float* scales, long long
 }
 
 // Quantisers over fp32 inputs.
+// Activations: the 1x128 blocks of a row-major matrix are contiguous, so the matrix is a plain list of blocks.  Bound by
+// memory; a warp takes QA_BLOCKS consecutive blocks so that their loads are in flight together.  4096 x 7168:
+// 45 -> 27 us (146 MB: 5.4 TB/s) with one block per warp before.
+constexpr int QA_BLOCKS = 4;
 template <bool POW2>
-__global__ void quant_act_1x128_kernel(const float* x, uint8_t* q, float* scales, long long rows, int cols) {
-    // one warp per 1x128 block; lane holds 4 consecutive values
-    int nb = cols / 128;
-    long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    long long total = rows * nb;
-    if (gw >= total) return;
-    long long r = gw / nb;
-    int b = (int)(gw % nb);
-    const float4 v = *reinterpret_cast<const float4*>(x + r * cols + (long long)b * 128 + lane * 4);
-    float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    float s = block_scale_of<POW2>(amax);
-    if (lane == 0) scales[gw] = s;
-    uchar4 o4;
-    o4.x = to_e4m3(__fdiv_rn(v.x, s));
-    o4.y = to_e4m3(__fdiv_rn(v.y, s));
-    o4.z = to_e4m3(__fdiv_rn(v.z, s));
-    o4.w = to_e4m3(__fdiv_rn(v.w, s));
-    *reinterpret_cast<uchar4*>(q + r * cols + (long long)b * 128 + lane * 4) = o4;
+__global__ void __launch_bounds__(256)
+quant_act_1x128_kernel(const float* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scales, long long total) {
+    const int lane = threadIdx.x & 31;
+    const long long b0 = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * QA_BLOCKS;
+    if (b0 >= total) return;
+    const int n = (int)(total - b0 < QA_BLOCKS ? total - b0 : QA_BLOCKS);
+    float4 v[QA_BLOCKS];
+#pragma unroll
+    for (int i = 0; i < QA_BLOCKS; i++)
+        v[i] = i < n ? __ldcs(reinterpret_cast<const float4*>(x + (b0 + i) * 128) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float s[QA_BLOCKS];
+#pragma unroll
+    for (int i = 0; i < QA_BLOCKS; i++) {
+        // non-negative floats order like their bits; fmaxf drops NaN, as the maximum always has here
+        const float m = fmaxf(fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))), 0.0f);
+        s[i] = block_scale_of<POW2>(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m))));
+    }
+#pragma unroll
+    for (int i = 0; i < QA_BLOCKS; i++) {
+        if (i < n) {
+            uchar4 o4;
+            o4.x = to_e4m3(__fdiv_rn(v[i].x, s[i]));
+            o4.y = to_e4m3(__fdiv_rn(v[i].y, s[i]));
+            o4.z = to_e4m3(__fdiv_rn(v[i].z, s[i]));
+            o4.w = to_e4m3(__fdiv_rn(v[i].w, s[i]));
+            reinterpret_cast<uchar4*>(q + (b0 + i) * 128)[lane] = o4;
+            if (lane == i) scales[b0 + i] = s[i];
+        }
+    }
 }
 
 template <bool POW2>
@@ -294,11 +307,11 @@ static int quant_act_1x128_impl(const float* x, uint8_t* q, float* scales, long 
     if (!x || !q || !scales) return B200_BAD_ARG;
     if (rows < 0 || cols <= 0 || cols % 128) return B200_BAD_SHAPE;
     if (rows == 0) return B200_OK;
-    long long warps = rows * (cols / 128);
-    long long blocks = (warps + 7) / 8;
-    if (blocks > 0x7fffffffLL) return B200_BAD_SHAPE;
-    if (pow2) quant_act_1x128_kernel<true><<<(unsigned)blocks, 256, 0, stream>>>(x, q, scales, rows, cols);
-    else      quant_act_1x128_kernel<false><<<(unsigned)blocks, 256, 0, stream>>>(x, q, scales, rows, cols);
+    const long long total = rows * (cols / 128);
+    const long long blocks = (total + 8 * QA_BLOCKS - 1) / (8 * QA_BLOCKS);
+    if ((total + 7) / 8 > 0x7fffffffLL) return B200_BAD_SHAPE;
+    if (pow2) quant_act_1x128_kernel<true><<<(unsigned)blocks, 256, 0, stream>>>(x, q, scales, total);
+    else      quant_act_1x128_kernel<false><<<(unsigned)blocks, 256, 0, stream>>>(x, q, scales, total);
     b200_count_launch(1);
     B200_CUDA_TRY(cudaGetLastError());
     return B200_OK;
