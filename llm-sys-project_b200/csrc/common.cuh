@@ -77,7 +77,27 @@ static inline bool b200_first_call_on_device(bool* done_by_device) {
     return true;
 }
 
+// Launch with programmatic stream serialisation: the kernel may start while the kernel in front of it in the stream
+// drains (launch latency and prologue overlap), and must call ptx::grid_wait() before it touches global memory that a
+// kernel in front writes, or writes anything.  Every kernel launched this way waits, so completion stays transitive along
+// the stream.
+template <typename... P, typename... A>
+static inline cudaError_t b200_launch_after(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
+                                            A... args) {
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = grid; lc.blockDim = dim3(threads); lc.dynamicSmemBytes = smem; lc.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = attr; lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, kernel, static_cast<P>(args)...);
+}
+
 namespace ptx {
+
+// programmatic dependent launch: wait for the kernels in front / let the next kernel start (no-ops otherwise)
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));

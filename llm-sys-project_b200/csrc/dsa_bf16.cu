@@ -340,11 +340,15 @@ done:
 __global__ void __launch_bounds__(128) dsa_merge_kernel(const float* __restrict__ part_o,
                                                         const float* __restrict__ part_ml, float* __restrict__ out,
                                                         int H, int NS) {
+    ptx::grid_wait();
+    ptx::grid_release();
     const int b = blockIdx.y, h = blockIdx.x;
     float M = -1e30f;
+#pragma unroll 8
     for (int s = 0; s < NS; s++) M = fmaxf(M, part_ml[(((size_t)b * NS + s) * HEADS + h) * 2]);
     float L = 0.0f;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
     for (int s = 0; s < NS; s++) {
         const float* ml = part_ml + (((size_t)b * NS + s) * HEADS + h) * 2;
         const float w = exp2f(ml[0] - M);
@@ -419,7 +423,7 @@ int dsa_bf16_impl(b200_ws* ws, const uint16_t* q_nope, const uint16_t* q_pe, con
                                       pair_tile, stream);
         if (st) return st;
         if (NS > 1) {
-            dsa_merge_kernel<<<dim3(H, Q), 128, 0, stream>>>(part_o, part_ml, out, H, NS);
+            B200_CUDA_TRY(b200_launch_after(dsa_merge_kernel, dim3(H, Q), 128, 0, stream, part_o, part_ml, out, H, NS));
             b200_count_launch(1);
             B200_CUDA_TRY(cudaGetLastError());
         }
@@ -444,7 +448,7 @@ int dsa_bf16_impl(b200_ws* ws, const uint16_t* q_nope, const uint16_t* q_pe, con
     b200_count_launch(1);
     B200_CUDA_TRY(cudaGetLastError());
     if (NS > 1) {
-        dsa_merge_kernel<<<dim3(H, Q), 128, 0, stream>>>(part_o, part_ml, out, H, NS);
+        B200_CUDA_TRY(b200_launch_after(dsa_merge_kernel, dim3(H, Q), 128, 0, stream, part_o, part_ml, out, H, NS));
         b200_count_launch(1);
         B200_CUDA_TRY(cudaGetLastError());
     }
@@ -598,7 +602,7 @@ extern "C" int b200_dsa_forward_bf16_static(const uint16_t* q_nope, const uint16
     b200_count_launch(1);
     B200_CUDA_TRY(cudaGetLastError());
     if (NS > 1) {
-        dsa_merge_kernel<<<dim3(H, Q), 128, 0, stream>>>(p.part_o, p.part_ml, out, H, NS);
+        B200_CUDA_TRY(b200_launch_after(dsa_merge_kernel, dim3(H, Q), 128, 0, stream, p.part_o, p.part_ml, out, H, NS));
         b200_count_launch(1);
         B200_CUDA_TRY(cudaGetLastError());
     }

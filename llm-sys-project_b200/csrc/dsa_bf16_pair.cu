@@ -221,10 +221,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) dsa_deco
                 asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0) : "memory");
             }
         }
-        ptx::cp_async_commit();
-        ptx::cp_async_wait<0>();
-        ptx::fence_proxy_async_smem();
-        ptx::mbar_arrive(&sm->q_full);
+        __threadfence_block();
+        ptx::cp_async_arrive_noinc(&sm->q_full);     // signals by itself when the copies land, as the tiles' copies do
 
         // Row ids of the next tile are fetched one tile ahead; the copies of a unit signal its
         // barrier by themselves when they land, so this thread never waits for data and up to two
@@ -581,6 +579,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS128, 1) dsa_d
     if (warp >= 5) {
         // ===================== gather producers: NKW warps for K rows, NVW warps for V rows =====================
         const int pt = threadIdx.x - 160;
+        const int s_begin = t_begin * TKV;
+        // the ids of the first tile are looked up (up to four dependent loads with a block table) behind the copies of Q
+        constexpr int RPW = KROWS / NKW;                          // K rows per warp
+        const int kw = pt >> 5;                                   // K warp: rows RPW kw .. RPW kw + RPW - 1 of this CTA's 64
+        constexpr int VPW = TKV / NVW;                            // V rows per warp
+        static_assert(VPW == 32, "one V row id per lane");
+        const int vw = (pt - 32 * NKW) >> 5;                      // V warp: rows vw, vw + NVW, ... of the tile's 128
+        const bool k_warp = pt < 32 * NKW;
+        const int my = k_warp ? (int)rank * KROWS + RPW * kw + (lane % RPW) : vw + NVW * lane;
+        int id_n = (nt > 0) ? dsa_resolve(p.ix, b, s_begin + my) : -1;
         // Q: this CTA's 64 heads x 72 sixteen-byte chunks; heads >= H are zero
         for (int i = pt; i < HPC * 72; i += NPROD) {
             const int r = i / 72, ch = i - r * 72;
@@ -594,21 +602,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS128, 1) dsa_d
                 asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dst), "r"(0) : "memory");
             }
         }
-        ptx::cp_async_commit();
-        ptx::cp_async_wait<0>();
-        ptx::fence_proxy_async_smem();
-        ptx::mbar_arrive(&sm->q_full);
+        // the copies signal q_full when they land (as the tiles' copies do): the first K and V rows are requested
+        // while Q is on its way
+        __threadfence_block();
+        ptx::cp_async_arrive_noinc(&sm->q_full);
 
         // A warp instruction always covers 512 contiguous bytes of one row (DRAM serves such pieces at
         // more than twice the rate of scattered 128-byte ones).  Each lane fetches the ids of the rows
         // its warp owns one tile ahead and hands them round by shuffle; the copies of a tile signal its
         // barrier by themselves when they land, so these threads never wait for data.
-        const int s_begin = t_begin * TKV;
-        if (pt < 32 * NKW) {
-            constexpr int RPW = KROWS / NKW;                      // K rows per warp
-            const int kw = pt >> 5;                               // rows RPW kw .. RPW kw + RPW - 1 of this CTA's 64
-            const int my = (int)rank * KROWS + RPW * kw + (lane % RPW);
-            int id_n = (nt > 0) ? dsa_resolve(p.ix, b, s_begin + my) : -1;
+        if (k_warp) {
             const uint32_t kst = ptx::smem_u32(sK);
             for (int j = 0; j < nt; j++) {
                 const int id = id_n;
@@ -664,26 +667,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS128, 1) dsa_d
                 }
             }
         } else {
-            constexpr int VPW = TKV / NVW;                        // V rows per warp (32 or 64)
-            const int vw = (pt - 32 * NKW) >> 5;                  // V rows vw, vw + NVW, ... of the tile's 128
-            const int my0 = vw + NVW * lane, my1 = (VPW > 32) ? vw + NVW * (lane + 32) : my0;
-            int id0_n = -1, id1_n = -1;
-            if (nt > 0) { id0_n = dsa_resolve(p.ix, b, s_begin + my0); id1_n = dsa_resolve(p.ix, b, s_begin + my1); }
             // this CTA's 512 contiguous bytes of a V row: columns [256 rank, 256 rank + 256);
             // 64-column chunk q = lane / 8 (MMA q/2, half q%2)
             const int q = lane >> 3, v16 = lane & 7;
             const uint32_t chunk = ptx::smem_u32(sV) + q * VCHUNK_BYTES;
             for (int j = 0; j < nt; j++) {
-                const int id0 = id0_n, id1 = id1_n;
-                if (j + 1 < nt) {
-                    id0_n = dsa_resolve(p.ix, b, s_begin + (j + 1) * TKV + my0);
-                    id1_n = dsa_resolve(p.ix, b, s_begin + (j + 1) * TKV + my1);
-                }
+                const int id = id_n;
+                if (j + 1 < nt) id_n = dsa_resolve(p.ix, b, s_begin + (j + 1) * TKV + my);
                 if (!ptx::mbar_wait(&sm->v_empty, (uint32_t)((j & 1) ^ 1), abort_flag)) goto done;
-                if (__all_sync(0xffffffffu, (id0 >= 0) && (id1 >= 0))) {
+                if (__all_sync(0xffffffffu, id >= 0)) {
 #pragma unroll 8
                     for (int x = 0; x < VPW; x++) {
-                        const size_t rid = (size_t)__shfl_sync(0xffffffffu, (x < 32) ? id0 : id1, x & 31);
+                        const size_t rid = (size_t)__shfl_sync(0xffffffffu, id, x);
                         const int r = vw + NVW * x;
                         ptx::cp_async_16(chunk + (r >> 3) * 1024 + (r & 7) * 128 + ((v16 ^ (r & 7)) << 4),
                                          p.v + rid * DC + 256 * (int)rank + lane * 8);
@@ -691,7 +686,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS128, 1) dsa_d
                 } else {
 #pragma unroll 4
                     for (int x = 0; x < VPW; x++) {
-                        const long long rid = __shfl_sync(0xffffffffu, (x < 32) ? id0 : id1, x & 31);
+                        const long long rid = __shfl_sync(0xffffffffu, id, x);
                         const int r = vw + NVW * x;
                         fetch16(chunk + (r >> 3) * 1024 + (r & 7) * 128 + ((v16 ^ (r & 7)) << 4), p.v, rid, DC,
                                 256 * (int)rank + lane * 8);
@@ -699,12 +694,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS128, 1) dsa_d
                     __threadfence_block();
                 }
                 ptx::cp_async_arrive_noinc(&sm->v_full);
-                if (j + 1 < nt) {
-                    if (id0_n >= 0)
-                        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.v + (size_t)id0_n * DC + 256 * (int)rank), "r"(512) : "memory");
-                    if (VPW > 32 && id1_n >= 0)
-                        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.v + (size_t)id1_n * DC + 256 * (int)rank), "r"(512) : "memory");
-                }
+                if (j + 1 < nt && id_n >= 0)
+                    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.v + (size_t)id_n * DC + 256 * (int)rank), "r"(512) : "memory");
             }
         }
         ptx::cp_async_commit();
@@ -743,7 +734,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS128, 1) dsa_d
                 commit_both(&sm->p_empty);
                 return true;
             };
-            if (!ptx::mbar_wait(&sm->q_full, 0, abort_flag)) goto done;
+            if (!ptx::mbar_wait(&sm->q_full, 0, abort_flag)) goto done;     // (fenced with the first K stage below)
             for (int j = 0; j < nt; j++) {
                 const int sb = j & 1;
                 if (!ptx::mbar_wait(&sm->s_empty[sb], (uint32_t)(((j >> 1) & 1) ^ 1), abort_flag)) goto done;
