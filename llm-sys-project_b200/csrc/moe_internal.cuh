@@ -72,6 +72,10 @@ int moe_route_fp8_run(const RouteScratch& rs, const uint8_t* xq, const float* xs
 // this library's router (an expert appears at most once per token), so the duplicate check is skipped.
 int launch_permute(const int* ids, int T, int K, int E, const int* counts_in, bool trusted, int* counts,
                    int* offsets, int* row_pair, cudaStream_t stream);
+// Same result with scratch of permute_ranges_scratch_ints integers: two launches whose work does not grow with E.
+size_t permute_ranges_scratch_ints(int T, int K, int E);
+int launch_permute_ranges(const int* ids, int T, int K, int E, bool trusted, int* range_hist, int* counts, int* offsets,
+                          int* row_pair, cudaStream_t stream);
 int check_route_cfg(int T, int E, int K, int D, int scoring, int n_group, int topk_group);
 
 // b200_moe_fp8_experts without the zero-fill of `out` (the caller keeps the rows that receive

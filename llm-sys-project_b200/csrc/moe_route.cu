@@ -163,6 +163,19 @@ __device__ __forceinline__ ValIdx warp_argmax(ValIdx x) {
     return x;
 }
 
+// The same result in three warp-wide steps instead of ten dependent shuffles, for lanes that hold ascending runs of
+// indices (ties: the lowest lane, and inside a lane the caller kept the lowest index).  x.i < 0: no candidate.
+__device__ __forceinline__ ValIdx warp_argmax_ordered(ValIdx x) {
+    const unsigned u = __float_as_uint(x.v + 0.0f);                       // -0 counts as +0
+    const unsigned key = x.i < 0 ? 0u : ((u & 0x80000000u) ? ~u : (u | 0x80000000u));
+    const unsigned top = __reduce_max_sync(0xffffffffu, key);
+    const int src = __ffs(__ballot_sync(0xffffffffu, key == top)) - 1;
+    ValIdx r;
+    r.v = __shfl_sync(0xffffffffu, x.v, src);
+    r.i = __shfl_sync(0xffffffffu, x.i, src);
+    return r;
+}
+
 // One token's selection, executed by one warp.  s / c: E floats each of this warp's shared memory.
 __device__ __forceinline__ void
 route_select_row(const float* __restrict__ partials, int n_chunks, const float* __restrict__ bias,
@@ -340,7 +353,7 @@ __device__ __forceinline__ void load_run(const float* p, float* v) {
     }
 }
 
-template <int PER>
+template <int PER, int FLY>
 __device__ __forceinline__ void
 route_select_row_regs(const float* __restrict__ partials, int n_chunks, const float* __restrict__ bias,
                       int* __restrict__ ids, float* __restrict__ wts, int* __restrict__ counts,
@@ -349,14 +362,14 @@ route_select_row_regs(const float* __restrict__ partials, int n_chunks, const fl
     const int e_lo = lane * PER;
     if (cert.plan.L > 0) n_chunks = tc_slots_before(cert.plan, row / 128, (row / 128 + 1) * cert.plan.nblk);
     float lg[PER];
-    // logit = the partial sums added in chunk order (loads of four chunks in flight, adds in order)
-    for (int ch0 = 0; ch0 < n_chunks; ch0 += 4) {
-        float v[4][PER];
+    // logit = the partial sums added in chunk order (loads of FLY chunks in flight, adds in order)
+    for (int ch0 = 0; ch0 < n_chunks; ch0 += FLY) {
+        float v[FLY][PER];
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < FLY; i++)
             if (ch0 + i < n_chunks) load_run<PER>(partials + ((size_t)(ch0 + i) * T + row) * E + e_lo, v[i]);
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < FLY; i++)
             if (ch0 + i < n_chunks) {
 #pragma unroll
                 for (int j = 0; j < PER; j++) lg[j] = (ch0 + i == 0) ? v[i][j] : __fadd_rn(lg[j], v[i][j]);
@@ -428,7 +441,7 @@ route_select_row_regs(const float* __restrict__ partials, int n_chunks, const fl
 #pragma unroll
         for (int j = 0; j < PER; j++)
             if (!((taken >> j) & 1u)) b = better(b, ValIdx{c[j], e_lo + j});
-        b = warp_argmax(b);
+        b = warp_argmax_ordered(b);
         if (cert.tau > 0.0f && b.i >= 0) {
             if (k > 0) min_margin = fminf(min_margin, prev_v - b.v);
             prev_v = b.v;
@@ -474,6 +487,8 @@ route_select_kernel(const float* __restrict__ partials, int n_chunks, const floa
                     float* __restrict__ logits_out, int T, int E, int K, int scoring, int n_group,
                     int topk_group, float routed_scale, RouteCert cert) {
     extern __shared__ float sm[];
+    ptx::grid_wait();
+    ptx::grid_release();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float* s = sm + (size_t)warp * 2 * E;
     float* c = s + E;
@@ -487,18 +502,21 @@ route_select_kernel(const float* __restrict__ partials, int n_chunks, const floa
 }
 
 // The register path as a kernel of its own (fewer registers than the generic kernel: more resident warps).  Seven
-// blocks per SM (72 registers, a few spilled words): 148 x 7 x 4 warps take 4096 tokens in one wave.
-template <int PER>
-__global__ void __launch_bounds__(128, 7)
+// blocks per SM (72 registers, a few spilled words): 148 x 7 x 4 warps take 4096 tokens in one wave.  Small batches are
+// one chain of latencies instead: there the loads of eight partial sums are in flight (FLY = 8, more registers).
+template <int PER, int FLY>
+__global__ void __launch_bounds__(128, FLY == 8 ? 3 : 7)
 route_select_regs_kernel(const float* __restrict__ partials, int n_chunks, const float* __restrict__ bias,
                          int* __restrict__ ids, float* __restrict__ wts, int* __restrict__ counts,
                          float* __restrict__ logits_out, int T, int E, int K, int n_group, int topk_group,
                          float routed_scale, RouteCert cert) {
+    ptx::grid_wait();
+    ptx::grid_release();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rows = cert.list ? min(*cert.list_n, T) : T;
     for (int row = blockIdx.x * 4 + warp; row < rows; row += gridDim.x * 4) {
         const int t = cert.list ? cert.list[row] : row;
-        route_select_row_regs<PER>(partials, n_chunks, bias, ids, wts, counts, logits_out, T, E, K, n_group, topk_group,
+        route_select_row_regs<PER, FLY>(partials, n_chunks, bias, ids, wts, counts, logits_out, T, E, K, n_group, topk_group,
                                    routed_scale, cert, row, t, lane);
     }
 }
@@ -541,6 +559,8 @@ template <bool CHECK_DUP>
 __global__ void __launch_bounds__(PERMUTE_THREADS)
 permute_kernel(const int* __restrict__ ids, int TK, int K, int E, const int* __restrict__ counts_in,
                int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ row_pair) {
+    ptx::grid_wait();
+    ptx::grid_release();
     constexpr int NW = PERMUTE_THREADS / 32;
     __shared__ int warp_sums[NW];
     __shared__ int s_base;
@@ -608,6 +628,100 @@ permute_kernel(const int* __restrict__ ids, int TK, int K, int E, const int* __r
         offsets[e] = base;
         if (e == E - 1) offsets[E] = base + running;
     }
+}
+
+// The same permutation for callers with scratch, in two launches whose work does not grow with E: the list is cut
+// into ranges of PR_PAIRS pairs, one block each.  permute_ranges_count_kernel writes a range's rows per expert;
+// permute_ranges_kernel adds the experts' totals and the earlier ranges' rows itself (E x ranges integers) and gives
+// every pair of its range its row: a warp owns 128 consecutive pairs, equal ids of a 32-pair step find each other by
+// match, and per-warp counters (scanned over the warps) keep the order stable.  The kernel above scans the whole
+// list once per expert: 131072 ids x 32 experts 67 us.  Here 12 us together (a
+// layer of 32 experts and 16384 rows: 2530 -> 2475 us).
+constexpr int PR_PAIRS = 4096, PR_THREADS = 1024;
+static_assert(PR_PAIRS == (PR_THREADS / 32) * 128, "128 pairs per warp");
+
+template <bool CHECK_DUP>
+__global__ void __launch_bounds__(PR_THREADS)
+permute_ranges_count_kernel(const int* __restrict__ ids, int TK, int K, int E, int* __restrict__ range_hist) {
+    ptx::grid_wait();
+    ptx::grid_release();
+    extern __shared__ int s_hist[];
+    for (int e = threadIdx.x; e < E; e += PR_THREADS) s_hist[e] = 0;
+    __syncthreads();
+    const int p1 = min(TK, ((int)blockIdx.x + 1) * PR_PAIRS);
+    for (int p = blockIdx.x * PR_PAIRS + threadIdx.x; p < p1; p += PR_THREADS) {
+        const int id = ids[p];
+        if (id >= 0 && id < E && (!CHECK_DUP || pair_selects(ids, p, K, id))) atomicAdd(&s_hist[id], 1);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += PR_THREADS) range_hist[(size_t)blockIdx.x * E + e] = s_hist[e];
+}
+
+template <bool CHECK_DUP>
+__global__ void __launch_bounds__(PR_THREADS)
+permute_ranges_kernel(const int* __restrict__ ids, int TK, int K, int E, const int* __restrict__ range_hist,
+                      int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ row_pair) {
+    ptx::grid_wait();
+    ptx::grid_release();
+    extern __shared__ int s_first[];                          // [E] first row of this range, then [32][E] 16-bit counters
+    unsigned short* wh = reinterpret_cast<unsigned short*>(s_first + E);
+    __shared__ int s_sum[PR_THREADS / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // experts' totals and first rows (thread = expert; E <= PR_THREADS)
+    int tot = 0, earlier = 0;
+    if (tid < E)
+        for (int r = 0; r < (int)gridDim.x; r++) {
+            const int n = range_hist[(size_t)r * E + tid];
+            earlier += (r < (int)blockIdx.x) ? n : 0;
+            tot += n;
+        }
+    int incl = tot;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int n = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += n;
+    }
+    if (lane == 31) s_sum[warp] = incl;
+    for (int i = tid; i < 32 * E; i += PR_THREADS) wh[i] = 0;
+    __syncthreads();
+    int base = incl - tot;
+    for (int w = 0; w < warp; w++) base += s_sum[w];
+    if (tid < E) {
+        s_first[tid] = base + earlier;
+        if (blockIdx.x == 0) {
+            offsets[tid] = base;
+            counts[tid] = tot;
+            if (tid == E - 1) offsets[E] = base + tot;
+        }
+    }
+    // ranks of equal ids inside the warp's 128 pairs
+    int id[4], rank[4];
+    unsigned short* mine = wh + warp * E;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int p = blockIdx.x * PR_PAIRS + warp * 128 + i * 32 + lane;
+        id[i] = (p < TK) ? ids[p] : -1;
+        if (id[i] >= E || (CHECK_DUP && id[i] >= 0 && !pair_selects(ids, p, K, id[i]))) id[i] = -1;
+        const unsigned same = __match_any_sync(0xffffffffu, id[i]);
+        const int before = id[i] >= 0 ? mine[id[i]] : 0;
+        rank[i] = before + __popc(same & ((1u << lane) - 1));
+        __syncwarp();
+        if (id[i] >= 0 && lane == __ffs(same) - 1) mine[id[i]] = (unsigned short)(before + __popc(same));
+        __syncwarp();
+    }
+    __syncthreads();
+    if (tid < E) {
+        int run = 0;
+        for (int w = 0; w < PR_THREADS / 32; w++) {
+            const int n = wh[w * E + tid];
+            wh[w * E + tid] = (unsigned short)run;
+            run += n;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        if (id[i] >= 0) row_pair[s_first[id[i]] + mine[id[i]] + rank[i]] = blockIdx.x * PR_PAIRS + warp * 128 + i * 32 + lane;
 }
 
 // FP8 router logits, tuned variant of the kernel above for aligned inputs (rows 16-byte aligned,
@@ -717,148 +831,142 @@ gate_logits_fp8_kernel(const uint8_t* __restrict__ xq, const float* __restrict__
     }
 }
 
-// FP8 router logits for decode-sized batches (T <= 32): the register-tiled kernels above would run
-// 14 CTAs of mostly padding.  Block = 32 experts x one chunk of d; thread = (expert, token slot);
-// every logit is still one fused multiply-add chain over the chunk's d in ascending order, so the
-// bits are those of the other kernels.  k-tiles of 128 d are double-buffered in shared memory.
-constexpr int GS_E = 32, GS_K = 128, GS_T = 8;
-__global__ void __launch_bounds__(GS_E * GS_T)
-gate_logits_fp8_small_kernel(const uint8_t* __restrict__ xq, const float* __restrict__ xs, const float* __restrict__ wg,
-                             float* __restrict__ partials, int T, int E, int D, int chunk) {
-    __shared__ float w_s[2][GS_E][GS_K + 1];
-    __shared__ float x_s[2][GS_T][GS_K];
-    const int e0 = blockIdx.x * GS_E, c = blockIdx.y;
-    const int d_begin = c * chunk, d_end = min(D, d_begin + chunk);
-    const int el = threadIdx.x & 31, ts = threadIdx.x >> 5;
-    const int nb = D / 128;
-    for (int t0 = 0; t0 < T; t0 += GS_T) {
-        auto stage = [&](int buf, int d0) {
-            // expert tile: 32 rows x 128 floats, coalesced along d; token tile: up to 8 rows, dequantised
-            for (int i = threadIdx.x; i < GS_E * GS_K; i += GS_E * GS_T) {
-                const int r = i / GS_K, k = i - r * GS_K;
-                w_s[buf][r][k] = (e0 + r < E && d0 + k < d_end) ? wg[(size_t)(e0 + r) * D + d0 + k] : 0.0f;
-            }
-            for (int i = threadIdx.x; i < GS_T * GS_K; i += GS_E * GS_T) {
-                const int r = i / GS_K, k = i - r * GS_K, t = t0 + r;
-                float v = 0.0f;
-                if (t < T && d0 + k < d_end) {
-                    __nv_fp8_e4m3 q;
-                    q.__x = xq[(size_t)t * D + d0 + k];
-                    v = __fmul_rn(float(q), xs[(size_t)t * nb + (d0 + k) / 128]);
+// FP8 router logits for decode-sized batches (T < 256) and for a list of tokens (the exact pass of the tensor-core
+// router).  Same chains, hence the same bits as the kernels above: every logit is one fused multiply-add chain over
+// the chunk's d in ascending order.  Such a call reads 7 MB of weights for a few chains per SM, so what counts is
+// how many blocks share the work and how early their loads are out: block = 16 experts x 32 tokens x one chunk of d
+// (E = 256, D = 7168: 112 blocks for up to 32 tokens), thread = 2 experts x 2 tokens (four independent chains; four
+// 16-byte shared-memory reads per sixteen multiply-adds), k-tiles of 128 d in a four-stage ring: weights by cp.async
+// three tiles ahead, activations through registers (dequantised once per block) one tile ahead.
+// E = 256, D = 7168: T = 1 35 -> 11 us, T = 16 67 -> 12 us (one expert x token chain per thread, 56 blocks, before).
+constexpr int GT_E = 16, GT_T = 32, GT_K = 128, GT_LD = GT_K + 4, GT_ST = 4, GT_THREADS = 128;
+constexpr size_t GT_SMEM = sizeof(float) * (size_t)GT_ST * (GT_E + GT_T) * GT_LD;
+template <bool LIST>
+__global__ void __launch_bounds__(GT_THREADS)
+gate_logits_fp8_tile_kernel(const uint8_t* __restrict__ xq, const float* __restrict__ xs, const float* __restrict__ wg,
+                            float* __restrict__ partials, const int* __restrict__ list, const int* __restrict__ list_n,
+                            int T, int E, int D, int chunk) {
+    extern __shared__ __align__(16) float gt_smem[];
+    ptx::grid_wait();
+    ptx::grid_release();
+    const int n = LIST ? min(*list_n, T) : T;
+    const int e0 = blockIdx.x * GT_E, c = blockIdx.y;
+    const int d_begin = c * chunk, nk = (min(D, d_begin + chunk) - d_begin) / GT_K;      // D % 128 == 0
+    const int tid = threadIdx.x, nb = D / 128;
+    const int el = tid & 7, tg = tid >> 3;               // experts el, el + 8; entries tg, tg + 16 (also: loader row and piece)
+    auto w_tile = [&](int j) { return gt_smem + (size_t)(j % GT_ST) * (GT_E + GT_T) * GT_LD; };
+    auto load_w = [&](int j) {
+        float* dst = w_tile(j);
+#pragma unroll
+        for (int i = 0; i < GT_E * GT_K / 4 / GT_THREADS; i++) {
+            const int p = tid + i * GT_THREADS, r = p >> 5, k = (p & 31) * 4;
+            const bool ok = e0 + r < E;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ptx::smem_u32(dst + r * GT_LD + k)),
+                         "l"(wg + (size_t)(ok ? e0 + r : 0) * D + d_begin + j * GT_K + k), "r"(ok ? 16 : 0)
+                         : "memory");
+        }
+    };
+    for (int i0 = blockIdx.z * GT_T; i0 < n; i0 += gridDim.z * GT_T) {
+#pragma unroll
+        for (int j = 0; j < GT_ST - 1; j++) {
+            if (j < nk) load_w(j);
+            ptx::cp_async_commit();
+        }
+        int tok[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int i = i0 + tg + 16 * h;
+            tok[h] = (i < n) ? (LIST ? list[i] : i) : -1;
+            if (tok[h] >= T) tok[h] = -1;
+        }
+        uint4 raw[2];
+        float sc[2];
+        auto fetch_x = [&](int j) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                raw[h] = make_uint4(0, 0, 0, 0);
+                sc[h] = 0.0f;
+                if (tok[h] >= 0) {
+                    raw[h] = __ldg(reinterpret_cast<const uint4*>(xq + (size_t)tok[h] * D + d_begin + j * GT_K + el * 16));
+                    sc[h] = xs[(size_t)tok[h] * nb + (d_begin + j * GT_K) / 128];
                 }
-                x_s[buf][r][k] = v;
             }
         };
-        float acc = 0.0f;
-        int buf = 0;
-        stage(0, d_begin);
-        __syncthreads();
-        for (int d0 = d_begin; d0 < d_end; d0 += GS_K) {
-            if (d0 + GS_K < d_end) stage(buf ^ 1, d0 + GS_K);
-            const int kmax = min(GS_K, d_end - d0);
-#pragma unroll 8
-            for (int k = 0; k < kmax; k++) acc = __fmaf_rn(x_s[buf][ts][k], w_s[buf][el][k], acc);
+        fetch_x(0);
+        const bool warp_live = i0 + (tg & ~3) < n;           // a warp holds entries 4 w .. 4 w + 3 and those + 16
+        const bool both = i0 + (tg & ~3) + 16 < n;
+        float acc[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};       // [entry][expert]
+        for (int j = 0; j < nk; j++) {
+            float* xt = w_tile(j) + GT_E * GT_LD;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                if (h == 1 && !both) break;
+                const uint32_t words[4] = {raw[h].x, raw[h].y, raw[h].z, raw[h].w};
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    float v[4];
+#pragma unroll
+                    for (int b = 0; b < 4; b++) {
+                        __nv_fp8_e4m3 f;
+                        f.__x = (unsigned char)((words[q] >> (8 * b)) & 0xFF);
+                        v[b] = tok[h] >= 0 ? __fmul_rn(float(f), sc[h]) : 0.0f;
+                    }
+                    *reinterpret_cast<float4*>(xt + (tg + 16 * h) * GT_LD + el * 16 + 4 * q) = make_float4(v[0], v[1], v[2], v[3]);
+                }
+            }
+            if (j + 1 < nk) fetch_x(j + 1);
+            ptx::cp_async_wait<GT_ST - 2>();
             __syncthreads();
-            buf ^= 1;
+            if (warp_live) {
+                const float *w0 = w_tile(j) + el * GT_LD, *w1 = w0 + 8 * GT_LD, *x0 = xt + tg * GT_LD, *x1 = x0 + 16 * GT_LD;
+                if (both) {
+#pragma unroll 8
+                    for (int k = 0; k < GT_K; k += 4) {
+                        const float4 wa = *reinterpret_cast<const float4*>(w0 + k), wb = *reinterpret_cast<const float4*>(w1 + k);
+                        const float4 xa = *reinterpret_cast<const float4*>(x0 + k), xb = *reinterpret_cast<const float4*>(x1 + k);
+                        acc[0][0] = __fmaf_rn(xa.x, wa.x, acc[0][0]); acc[0][1] = __fmaf_rn(xa.x, wb.x, acc[0][1]);
+                        acc[1][0] = __fmaf_rn(xb.x, wa.x, acc[1][0]); acc[1][1] = __fmaf_rn(xb.x, wb.x, acc[1][1]);
+                        acc[0][0] = __fmaf_rn(xa.y, wa.y, acc[0][0]); acc[0][1] = __fmaf_rn(xa.y, wb.y, acc[0][1]);
+                        acc[1][0] = __fmaf_rn(xb.y, wa.y, acc[1][0]); acc[1][1] = __fmaf_rn(xb.y, wb.y, acc[1][1]);
+                        acc[0][0] = __fmaf_rn(xa.z, wa.z, acc[0][0]); acc[0][1] = __fmaf_rn(xa.z, wb.z, acc[0][1]);
+                        acc[1][0] = __fmaf_rn(xb.z, wa.z, acc[1][0]); acc[1][1] = __fmaf_rn(xb.z, wb.z, acc[1][1]);
+                        acc[0][0] = __fmaf_rn(xa.w, wa.w, acc[0][0]); acc[0][1] = __fmaf_rn(xa.w, wb.w, acc[0][1]);
+                        acc[1][0] = __fmaf_rn(xb.w, wa.w, acc[1][0]); acc[1][1] = __fmaf_rn(xb.w, wb.w, acc[1][1]);
+                    }
+                } else {
+#pragma unroll 8
+                    for (int k = 0; k < GT_K; k += 4) {
+                        const float4 wa = *reinterpret_cast<const float4*>(w0 + k), wb = *reinterpret_cast<const float4*>(w1 + k);
+                        const float4 xa = *reinterpret_cast<const float4*>(x0 + k);
+                        acc[0][0] = __fmaf_rn(xa.x, wa.x, acc[0][0]); acc[0][1] = __fmaf_rn(xa.x, wb.x, acc[0][1]);
+                        acc[0][0] = __fmaf_rn(xa.y, wa.y, acc[0][0]); acc[0][1] = __fmaf_rn(xa.y, wb.y, acc[0][1]);
+                        acc[0][0] = __fmaf_rn(xa.z, wa.z, acc[0][0]); acc[0][1] = __fmaf_rn(xa.z, wb.z, acc[0][1]);
+                        acc[0][0] = __fmaf_rn(xa.w, wa.w, acc[0][0]); acc[0][1] = __fmaf_rn(xa.w, wb.w, acc[0][1]);
+                    }
+                }
+            }
+            if (j + GT_ST - 1 < nk) load_w(j + GT_ST - 1);
+            ptx::cp_async_commit();
         }
-        const int t = t0 + ts, e = e0 + el;
-        if (t < T && e < E) partials[((size_t)c * T + t) * E + e] = acc;
-        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int i = i0 + tg + 16 * h;
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+                if (i < n && e0 + el + 8 * q < E) partials[((size_t)c * T + i) * E + e0 + el + 8 * q] = acc[h][q];
+        }
+        __syncthreads();                                     // the ring is refilled for the next entries
     }
 }
 
-// The same chains for a list of tokens (the exact pass of the tensor-core router).  Block = 64 threads = 32
-// experts x 8 list entries per round x one chunk of d; thread = one expert x four entries, so that one 16-byte
-// read of the expert's weights serves sixteen multiply-adds (the entries' activations are warp-wide broadcasts).
-// k-tiles of 128 d: the next tile is fetched into registers while the current one is multiplied.  A bounded
-// grid walks the list, whose length is known only on the device.
-constexpr int GL2_E = 32, GL2_K = 128, GL2_T = 8, GL2_LDW = GL2_K + 4, GL2_THREADS = 64;
-__global__ void __launch_bounds__(GL2_THREADS)
-gate_logits_fp8_list_kernel(const uint8_t* __restrict__ xq, const float* __restrict__ xs, const float* __restrict__ wg,
-                            float* __restrict__ partials, const int* __restrict__ list, const int* __restrict__ list_n,
-                            int T, int E, int D, int chunk) {
-    __shared__ __align__(16) float w_s[GL2_E][GL2_LDW];
-    __shared__ __align__(16) float x_s[GL2_T][GL2_K];
-    __shared__ int tok_s[GL2_T];
-    const int n = min(*list_n, T);
-    const int e0 = blockIdx.x * GL2_E, c = blockIdx.y;
-    const int d_begin = c * chunk, d_end = min(D, d_begin + chunk);      // multiples of 128 (D % 128 == 0)
-    const int el = threadIdx.x & 31, tg = threadIdx.x >> 5;
-    const int nb = D / 128;
-    constexpr int WREP = GL2_E * GL2_K / 4 / GL2_THREADS;                 // 16 float4 of the weight tile per thread
-    const int xr = threadIdx.x >> 3, xp = threadIdx.x & 7;               // activation tile: entry xr, bytes 16*xp..
-    // The block's slab of weights (32 experts x the chunk's d) is walked in eight dependent steps; asking L2 for
-    // all of it up front pays the DRAM latency once instead of once per step.
-    if (blockIdx.z * GL2_T < n) {
-        const int lines_per_row = (d_end - d_begin) / 32;                // 128-byte lines of one expert's chunk
-        for (int i = threadIdx.x; i < GL2_E * lines_per_row; i += GL2_THREADS) {
-            const int r = i / lines_per_row, l = i - r * lines_per_row;
-            if (e0 + r < E)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(wg + (size_t)(e0 + r) * D + d_begin + l * 32));
-        }
+constexpr int GT_MAX_T = 256;
+static int gate_tile_attr() {
+    static bool attr_done[64] = {false};
+    if (b200_first_call_on_device(attr_done)) {
+        B200_CUDA_TRY(cudaFuncSetAttribute(gate_logits_fp8_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM));
+        B200_CUDA_TRY(cudaFuncSetAttribute(gate_logits_fp8_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM));
     }
-    for (int i0 = blockIdx.z * GL2_T; i0 < n; i0 += gridDim.z * GL2_T) {
-        __syncthreads();
-        if (threadIdx.x < GL2_T) tok_s[threadIdx.x] = (i0 + threadIdx.x < n) ? list[i0 + threadIdx.x] : -1;
-        __syncthreads();
-        const int xt = tok_s[xr];
-        const bool x_live = xt >= 0 && xt < T;
-        float4 w_reg[WREP];
-        uint4 x_raw = make_uint4(0, 0, 0, 0);
-        float x_sc = 0.0f;
-        auto fetch = [&](int d0) {
-#pragma unroll
-            for (int rep = 0; rep < WREP; rep++) {
-                const int idx = threadIdx.x + rep * GL2_THREADS, r = idx >> 5, kq = (idx & 31) * 4;
-                w_reg[rep] = (e0 + r < E) ? __ldg(reinterpret_cast<const float4*>(wg + (size_t)(e0 + r) * D + d0 + kq))
-                                          : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-            if (x_live) {
-                x_raw = __ldg(reinterpret_cast<const uint4*>(xq + (size_t)xt * D + d0 + xp * 16));
-                x_sc = xs[(size_t)xt * nb + d0 / 128];
-            }
-        };
-        auto stage = [&]() {
-#pragma unroll
-            for (int rep = 0; rep < WREP; rep++) {
-                const int idx = threadIdx.x + rep * GL2_THREADS, r = idx >> 5, kq = (idx & 31) * 4;
-                *reinterpret_cast<float4*>(&w_s[r][kq]) = w_reg[rep];
-            }
-            const uint8_t* b = reinterpret_cast<const uint8_t*>(&x_raw);
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                __nv_fp8_e4m3 q;
-                q.__x = b[i];
-                x_s[xr][xp * 16 + i] = x_live ? __fmul_rn(float(q), x_sc) : 0.0f;
-            }
-        };
-        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        fetch(d_begin);
-        for (int d0 = d_begin; d0 < d_end; d0 += GL2_K) {
-            __syncthreads();                      // the previous tile has been read
-            stage();
-            __syncthreads();
-            if (d0 + GL2_K < d_end) fetch(d0 + GL2_K);
-#pragma unroll 8
-            for (int k = 0; k < GL2_K; k += 4) {
-                const float4 w4 = *reinterpret_cast<const float4*>(&w_s[el][k]);
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const float4 x4 = *reinterpret_cast<const float4*>(&x_s[tg * 4 + i][k]);
-                    acc[i] = __fmaf_rn(x4.x, w4.x, acc[i]);
-                    acc[i] = __fmaf_rn(x4.y, w4.y, acc[i]);
-                    acc[i] = __fmaf_rn(x4.z, w4.z, acc[i]);
-                    acc[i] = __fmaf_rn(x4.w, w4.w, acc[i]);
-                }
-            }
-        }
-        const int e = e0 + el;
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int li = i0 + tg * 4 + i;
-            if (li < n && e < E) partials[((size_t)c * T + li) * E + e] = acc[i];
-        }
-    }
+    return B200_OK;
 }
 
 template <int TY>
@@ -884,10 +992,14 @@ int launch_gate_logits(const void* x, const float* xs, const float* wg, float* p
     const int n_chunks = moe_gate_chunks(D, fp8);
     const bool vec = (D % 16 == 0) && (chunk % 16 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0) &&
                      ((reinterpret_cast<uintptr_t>(wg) & 15) == 0);
-    if (fp8 && T <= 32 && D % 128 == 0) {
-        dim3 grid(ceil_div(E, GS_E), n_chunks);
-        gate_logits_fp8_small_kernel<<<grid, GS_E * GS_T, 0, stream>>>(static_cast<const uint8_t*>(x), xs, wg, partials,
-                                                                      T, E, D, chunk);
+    // Small batches: the 64 .. 128-token tiles below would leave most of the SMs idle (T = 128, E = 256, D = 7168: 28
+    // tiles), the 16 x 32 ones give 448 blocks.
+    if (fp8 && T < GT_MAX_T && vec && D % 128 == 0) {
+        const int st = gate_tile_attr();
+        if (st) return st;
+        dim3 grid(ceil_div(E, GT_E), n_chunks, ceil_div(T, GT_T));
+        gate_logits_fp8_tile_kernel<false><<<grid, GT_THREADS, GT_SMEM, stream>>>(static_cast<const uint8_t*>(x), xs, wg, partials,
+                                                                                nullptr, nullptr, T, E, D, chunk);
         b200_count_launch(1);
         B200_CUDA_TRY(cudaGetLastError());
         return B200_OK;
@@ -952,9 +1064,14 @@ int launch_gate_logits_list(const uint8_t* xq, const float* xs, const float* wg,
                             const int* list_n, int T, int E, int D, cudaStream_t stream) {
     if (D % 128) return B200_BAD_SHAPE;
     if ((reinterpret_cast<uintptr_t>(xq) & 15) || (reinterpret_cast<uintptr_t>(wg) & 15)) return B200_BAD_ARG;
-    dim3 grid(ceil_div(E, GL2_E), moe_gate_chunks(D, true), min(ceil_div(T, GL2_T), 32));
-    gate_logits_fp8_list_kernel<<<grid, GL2_THREADS, 0, stream>>>(xq, xs, wg, partials, list, list_n, T, E, D, MOE_GATE_CHUNK);
+    const int st = gate_tile_attr();
+    if (st) return st;
+    // the list's length is known only on the device: blocks beyond it leave at once, longer lists are walked
+    dim3 grid(ceil_div(E, GT_E), moe_gate_chunks(D, true), min(ceil_div(T, GT_T), 8));
+    const cudaError_t err = b200_launch_after(gate_logits_fp8_tile_kernel<true>, grid, GT_THREADS, GT_SMEM, stream, xq, xs, wg, partials,
+                                              list, list_n, T, E, D, MOE_GATE_CHUNK);
     b200_count_launch(1);
+    B200_CUDA_TRY(err);
     B200_CUDA_TRY(cudaGetLastError());
     return B200_OK;
 }
@@ -970,23 +1087,21 @@ int launch_route_select(const float* partials, int n_chunks, const float* bias, 
     // list mode: the length of the list is known only on the device; a modest grid walks it with a stride
     const int blocks = cert.list ? min(ceil_div(T, 4), 4 * 148) : ceil_div(T, 4);
     const int per = route_regs_per(E, K, scoring, n_group);
-    if (per == 8)
-        route_select_regs_kernel<8><<<blocks, 128, 0, stream>>>(partials, n_chunks, bias, ids, wts, counts, logits_out, T, E, K,
-                                                                n_group, topk_group, routed_scale, cert);
-    else if (per == 4)
-        route_select_regs_kernel<4><<<blocks, 128, 0, stream>>>(partials, n_chunks, bias, ids, wts, counts, logits_out, T, E, K,
-                                                                n_group, topk_group, routed_scale, cert);
-    else if (per == 2)
-        route_select_regs_kernel<2><<<blocks, 128, 0, stream>>>(partials, n_chunks, bias, ids, wts, counts, logits_out, T, E, K,
-                                                                n_group, topk_group, routed_scale, cert);
-    else if (per == 1)
-        route_select_regs_kernel<1><<<blocks, 128, 0, stream>>>(partials, n_chunks, bias, ids, wts, counts, logits_out, T, E, K,
-                                                                n_group, topk_group, routed_scale, cert);
+    const bool small = !cert.list && T <= 3 * 4 * 148;        // one wave at three blocks per SM
+    cudaError_t err = cudaSuccess;
+    auto regs = [&](auto kernel) {
+        err = b200_launch_after(kernel, dim3(blocks), 128, 0, stream, partials, n_chunks, bias, ids, wts, counts, logits_out, T, E, K,
+                                n_group, topk_group, routed_scale, cert);
+    };
+    if (per == 8)      small ? regs(route_select_regs_kernel<8, 8>) : regs(route_select_regs_kernel<8, 4>);
+    else if (per == 4) small ? regs(route_select_regs_kernel<4, 8>) : regs(route_select_regs_kernel<4, 4>);
+    else if (per == 2) small ? regs(route_select_regs_kernel<2, 8>) : regs(route_select_regs_kernel<2, 4>);
+    else if (per == 1) small ? regs(route_select_regs_kernel<1, 8>) : regs(route_select_regs_kernel<1, 4>);
     else
-        route_select_kernel<<<blocks, 128, smem, stream>>>(partials, n_chunks, bias, ids, wts, counts,
-                                                           logits_out, T, E, K, scoring, n_group, topk_group,
-                                                           routed_scale, cert);
+        err = b200_launch_after(route_select_kernel, dim3(blocks), 128, smem, stream, partials, n_chunks, bias, ids, wts, counts,
+                                logits_out, T, E, K, scoring, n_group, topk_group, routed_scale, cert);
     b200_count_launch(1);
+    B200_CUDA_TRY(err);
     B200_CUDA_TRY(cudaGetLastError());
     return B200_OK;
 }
@@ -1054,9 +1169,32 @@ int launch_permute(const int* ids, int T, int K, int E, const int* counts_in, bo
         B200_CUDA_TRY(cudaGetLastError());
         counts_in = counts;       // each block rewrites its own entry with the same value at the end
     }
-    if (trusted) permute_kernel<false><<<E, PERMUTE_THREADS, 0, stream>>>(ids, TK, K, E, counts_in, counts, offsets, row_pair);
-    else         permute_kernel<true><<<E, PERMUTE_THREADS, 0, stream>>>(ids, TK, K, E, counts_in, counts, offsets, row_pair);
+    const cudaError_t err = b200_launch_after(trusted ? permute_kernel<false> : permute_kernel<true>, dim3(E), PERMUTE_THREADS, 0, stream,
+                                              ids, TK, K, E, counts_in, counts, offsets, row_pair);
     b200_count_launch(1);
+    B200_CUDA_TRY(err);
+    B200_CUDA_TRY(cudaGetLastError());
+    return B200_OK;
+}
+
+size_t permute_ranges_scratch_ints(int T, int K, int E) { return (size_t)ceil_div(T * K, PR_PAIRS) * E; }
+
+int launch_permute_ranges(const int* ids, int T, int K, int E, bool trusted, int* range_hist, int* counts, int* offsets,
+                          int* row_pair, cudaStream_t stream) {
+    if (E > PR_THREADS) return B200_UNSUPPORTED;
+    const int TK = T * K, ranges = ceil_div(TK, PR_PAIRS);
+    const size_t smem = (size_t)E * sizeof(int) + (size_t)(PR_THREADS / 32) * E * sizeof(unsigned short);
+    static bool attr_done[64] = {false};
+    if (b200_first_call_on_device(attr_done)) {
+        const int most = PR_THREADS * (int)(sizeof(int) + (PR_THREADS / 32) * sizeof(unsigned short));
+        B200_CUDA_TRY(cudaFuncSetAttribute(permute_ranges_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+        B200_CUDA_TRY(cudaFuncSetAttribute(permute_ranges_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    }
+    B200_CUDA_TRY(b200_launch_after(trusted ? permute_ranges_count_kernel<false> : permute_ranges_count_kernel<true>, dim3(ranges),
+                                    PR_THREADS, sizeof(int) * (size_t)E, stream, ids, TK, K, E, range_hist));
+    B200_CUDA_TRY(b200_launch_after(trusted ? permute_ranges_kernel<false> : permute_ranges_kernel<true>, dim3(ranges), PR_THREADS,
+                                    smem, stream, ids, TK, K, E, range_hist, counts, offsets, row_pair));
+    b200_count_launch(2);
     B200_CUDA_TRY(cudaGetLastError());
     return B200_OK;
 }

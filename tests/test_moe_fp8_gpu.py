@@ -286,3 +286,51 @@ def test_host_pipeline_matches_synchronous_call(b200, cuda):
         b200.HostPipeline.wait(t)
     for w, o in zip(want, outs):
         assert torch.allclose(w, o, rtol=1e-5, atol=1e-6)      # scatter-add order may differ between runs
+
+
+@pytest.mark.parametrize("T,E,K", [(1, 40, 8), (512, 40, 8), (513, 40, 8), (1100, 3, 2), (1500, 1024, 8)])
+def test_permutation_ranges(b200, cuda, T, E, K):
+    """Sorted rows of ids from outside (repeated within a token, negative, beyond E): one range of the list, a whole
+    number of ranges, one more pair than that, few and many experts.  Integers, so equal to the oracle's."""
+    rng = np.random.default_rng(T + E)
+    D, I = 256, 128
+    ids = rng.integers(-2, E + 2, (T, K)).astype(np.int32)
+    cfg = b200.MoeFp8Config(T, E, K, D, I, b200.SCORE_SIGMOID_GROUPED, 1, 1, 1.0)
+    act_q = torch.empty((T * K, I), dtype=torch.uint8, device=cuda)
+    act_s = torch.empty((T * K, I // 128), dtype=torch.float32, device=cuda)
+    offs = torch.empty(E + 1, dtype=torch.int32, device=cuda)
+    rp = torch.empty(T * K, dtype=torch.int32, device=cuda)
+    z = lambda *s: torch.zeros(s, dtype=torch.uint8, device=cuda)
+    one = lambda *s: torch.ones(s, dtype=torch.float32, device=cuda)
+    b200.moe_fp8_gemm1_stage(z(T, D), one(T, D // 128), _dev(ids, cuda), z(E, 2 * I, D), one(E, 2 * I // 128, D // 128),
+                             act_q, act_s, offs, rp, cfg)
+    torch.cuda.synchronize()
+    assert b200.device_status() == 0
+    kept = np.where((ids >= 0) & (ids < E), ids, -1)
+    for k in range(1, K):
+        kept[:, k] = np.where((kept[:, :k] == kept[:, k:k + 1]).any(1), -1, kept[:, k])
+    flat = kept.reshape(-1)
+    want = np.concatenate([np.nonzero(flat == e)[0] for e in range(E)])
+    assert np.array_equal(offs.cpu().numpy(), np.concatenate([[0], np.cumsum(np.bincount(flat[flat >= 0], minlength=E))]))
+    assert np.array_equal(rp.cpu().numpy()[: len(want)], want)
+
+
+@pytest.mark.parametrize("T,E,D", [(1, 256, 1024), (31, 40, 1152), (33, 72, 2304), (255, 256, 7168)])
+def test_small_batch_router_bits(b200, cuda, T, E, D):
+    """The 16 x 32 router tiles: one token, a partial tile of experts, a short last chunk of d, several token tiles.
+    Logits are the oracle's fixed-order chains bit for bit, hence the same ids."""
+    rng = np.random.default_rng(T * 3 + E)
+    x = rng.normal(0, 1, (T, D)).astype(np.float32)
+    wg = rng.normal(0, D ** -0.5, (E, D)).astype(np.float32)
+    bias = rng.normal(0, 0.01, E).astype(np.float32)
+    xq, xs = oracle.quant_act(x)
+    cfg = b200.MoeFp8Config(T, E, 4, D, 128, b200.SCORE_SIGMOID_GROUPED, 4, 2, 2.5)
+    ids = torch.empty((T, 4), dtype=torch.int32, device=cuda)
+    wts = torch.empty((T, 4), dtype=torch.float32, device=cuda)
+    logits = torch.empty((T, E), dtype=torch.float32, device=cuda)
+    b200.moe_route_fp8(_dev(xq, cuda), _dev(xs, cuda), _dev(wg, cuda), _dev(bias, cuda), ids, wts, cfg, logits_out=logits)
+    torch.cuda.synchronize()
+    assert np.array_equal(logits.cpu().numpy(), oracle.gate_logits_fp8(xq, xs, wg))
+    oids, owts = oracle.route_grouped(xq, xs, wg, bias, 4, 4, 2, 2.5)
+    assert np.array_equal(ids.cpu().numpy(), oids)
+    assert np.abs(wts.cpu().numpy() - owts).max() <= 5e-7
