@@ -11,6 +11,7 @@
 // activations is made and the host never learns the per-expert counts.  Aligned shapes take the kernels of the
 // vector path below; these two serve the rest.
 #include <cfloat>
+#include <type_traits>
 
 #include "cluster_f32.cuh"
 #include "common.cuh"
@@ -125,15 +126,18 @@ grouped_gemm_f32_kernel(const float* __restrict__ a_src,     // MODE 1: x [T,D];
 //     in front of them has finished);
 //   * no permutation kernel when the id list is short (T * K <= GV_PAIRS): every GEMM block reads the ids and
 //     lists its expert's rows itself (a kilobyte against its 100 KB of weights);
-//   * weights stream through a four-stage cp.async ring; thread = (MT / 4) x 4 outputs of one quarter of each
-//     k-tile, operands read as 16-byte vectors along k from rows of 36 floats (odd multiple of 16 bytes: no bank
-//     conflicts), the four quarters are added at the end;
+//   * weights stream through a four-stage cp.async ring; a warp takes an eighth of every k-tile for the whole MT x 64
+//     tile, thread = (MT / 4) x 8 outputs, operands read as 16-byte vectors along k from rows of 68 floats (odd
+//     multiple of 16 bytes: no bank conflicts), the eight warps' sums are added at the end.  The multiply-adds of a
+//     shared-memory read are what bounds the large case: with (MT / 4) x 4 outputs of a quarter of a 32-deep k-tile
+//     per thread the T = 128 case below took 68 us;
 //   * where the tiles do not fill the machine the reduction is split over a cluster of up to four CTAs and added in
 //     rank order through distributed shared memory, so an output still receives one addition per (token, expert).
 // T = 32, E = 8, K = 2, D = 128, I = 256: 66 -> 16 us a call; T = 128, E = 16, K = 2, D = 512, I = 1024: 355 -> 68 us
 // (100 MB of weights); error against 64-bit arithmetic 9.2e-7 -> 5.2e-7.
 // ---------------------------------------------------------------------------------------------
-constexpr int GV_KT = 32, GV_LD = GV_KT + 4, GV_ST = 4, GV_N = 64, GV_THREADS = 256, GV_PAIRS = 2048;
+constexpr int GV_KT = 64, GV_LD = GV_KT + 4, GV_ST = 4, GV_N = 64, GV_THREADS = 256, GV_PAIRS = 2048;
+constexpr int GV_W = GV_THREADS / 32, GV_RLD = GV_N + 8;      // warps; row stride of the warps' sums
 
 __device__ __forceinline__ void gv_cp16(float* dst, const float* src, bool ok) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ptx::smem_u32(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
@@ -155,14 +159,14 @@ constexpr size_t gv_smem_bytes() { return sizeof(float) * (size_t)GV_ST * (GV_N 
 
 // grid: (ceil(N / tile columns), row-tile walkers, E * cluster size); MT rows x 64 weight rows per tile
 template <int MODE, int MT>
-__global__ void __launch_bounds__(GV_THREADS)
+__global__ void __launch_bounds__(GV_THREADS, 2)
 grouped_gemm_f32_vec_kernel(const GvParams p) {
     extern __shared__ __align__(16) float gv_smem[];
     __shared__ int s_pair[GV_PAIRS];
     __shared__ int s_warp[GV_THREADS / 32];
     constexpr int RT = MT / 4;                               // rows per thread
     constexpr int STG = (GV_N + MT) * GV_LD;                 // floats per stage: weights, then activations
-    static_assert(4 * MT * GV_N <= GV_ST * STG, "the k-quarter sums reuse the ring");
+    static_assert(GV_W * MT * GV_RLD <= GV_ST * STG, "the warps' sums reuse the ring");
     uint32_t crank, csize;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(csize));
@@ -174,13 +178,13 @@ grouped_gemm_f32_vec_kernel(const GvParams p) {
     const int kt_b = min(nkt, (int)crank * per), nk = min(nkt, kt_b + per) - kt_b;
 
     const float* we = p.w + (size_t)e * ((MODE == 1) ? (size_t)2 * p.I * p.D : (size_t)p.D * p.I);
-    // this thread's two 16-byte pieces of a weight tile: tile rows tid / 8 and tid / 8 + 32
-    const int lr = tid >> 3, lk = (tid & 7) * 4;
-    const float* wsrc[2];
-    bool wok[2];
+    // this thread's 16-byte pieces of a weight tile: tile rows tid / 16 + 16 i
+    const int lr = tid >> 4, lk = (tid & 15) * 4;
+    const float* wsrc[4];
+    bool wok[4];
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
-        const int c = lr + 32 * i;
+    for (int i = 0; i < 4; i++) {
+        const int c = lr + 16 * i;
         const int n = (MODE == 1) ? n0 + (c & 31) : n0 + c;
         wok[i] = n < N;
         wsrc[i] = we + (size_t)((MODE == 1 && c >= 32) ? p.I + (wok[i] ? n : 0) : (wok[i] ? n : 0)) * Kd;
@@ -189,7 +193,7 @@ grouped_gemm_f32_vec_kernel(const GvParams p) {
         const int k = (kt_b + j) * GV_KT + lk;
         float* d = gv_smem + (j % GV_ST) * STG + lr * GV_LD + lk;
 #pragma unroll
-        for (int i = 0; i < 2; i++) gv_cp16(d + 32 * i * GV_LD, wsrc[i] + (k < Kd ? k : 0), wok[i] && k < Kd);
+        for (int i = 0; i < 4; i++) gv_cp16(d + 16 * i * GV_LD, wsrc[i] + (k < Kd ? k : 0), wok[i] && k < Kd);
     };
     // the weights do not depend on the kernel in front: the first tiles are requested before waiting for it
     const bool early = blockIdx.y == 0;
@@ -233,18 +237,26 @@ grouped_gemm_f32_vec_kernel(const GvParams p) {
         for (int w = 0; w < GV_THREADS / 32; w++) base += s_warp[w];
     }
 
-    const int tx = tid & 15, ty = (tid >> 4) & 3, kq = tid >> 6;
+    const int tx = lane & 7, ty = lane >> 3;
+    constexpr int AR = (MT + 15) / 16;                       // activation rows per loader thread
     bool first = early;
     for (int m0 = blockIdx.y * MT; m0 < cnt; m0 += gridDim.y * MT) {
-        const float* asrc = nullptr;
-        if (tid < MT * 8 && m0 + lr < cnt)
-            asrc = p.a + ((MODE == 1) ? (size_t)(rows[m0 + lr] / p.K) * Kd : (size_t)(base + m0 + lr) * Kd);
+        const float* asrc[AR];
+#pragma unroll
+        for (int i = 0; i < AR; i++) {
+            const int r = m0 + lr + 16 * i;
+            asrc[i] = nullptr;
+            if (lr + 16 * i < MT && r < cnt)
+                asrc[i] = p.a + ((MODE == 1) ? (size_t)(rows[r] / p.K) * Kd : (size_t)(base + r) * Kd);
+        }
         auto load_a = [&](int j) {
-            if (tid < MT * 8) {
-                const int k = (kt_b + j) * GV_KT + lk;
-                const bool ok = asrc != nullptr && k < Kd;
-                gv_cp16(gv_smem + (j % GV_ST) * STG + (GV_N + lr) * GV_LD + lk, ok ? asrc + k : p.a, ok);
-            }
+            const int k = (kt_b + j) * GV_KT + lk;
+#pragma unroll
+            for (int i = 0; i < AR; i++)
+                if (lr + 16 * i < MT) {
+                    const bool ok = asrc[i] != nullptr && k < Kd;
+                    gv_cp16(gv_smem + (j % GV_ST) * STG + (GV_N + lr + 16 * i) * GV_LD + lk, ok ? asrc[i] + k : p.a, ok);
+                }
         };
 #pragma unroll
         for (int j = 0; j < GV_ST - 1; j++) {
@@ -255,27 +267,27 @@ grouped_gemm_f32_vec_kernel(const GvParams p) {
             ptx::cp_async_commit();
         }
         first = false;
-        float acc[RT][4];
+        float acc[RT][8];
 #pragma unroll
         for (int i = 0; i < RT; i++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
+            for (int j = 0; j < 8; j++) acc[i][j] = 0.0f;
         for (int j = 0; j < nk; j++) {
             ptx::cp_async_wait<GV_ST - 2>();
             __syncthreads();
             const float* sb = gv_smem + (j % GV_ST) * STG;
             const float* sa = sb + GV_N * GV_LD;
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int k = (kq + 4 * h) * 4;
-                float4 b[4];
+            for (int h = 0; h < GV_KT / 4 / GV_W; h++) {
+                const int k = (warp + GV_W * h) * 4;
+                float4 b[8];
 #pragma unroll
-                for (int c = 0; c < 4; c++) b[c] = *reinterpret_cast<const float4*>(sb + (tx + 16 * c) * GV_LD + k);
+                for (int c = 0; c < 8; c++) b[c] = *reinterpret_cast<const float4*>(sb + (tx + 8 * c) * GV_LD + k);
 #pragma unroll
                 for (int i = 0; i < RT; i++) {
                     const float4 a = *reinterpret_cast<const float4*>(sa + (ty + 4 * i) * GV_LD + k);
 #pragma unroll
-                    for (int c = 0; c < 4; c++) {
+                    for (int c = 0; c < 8; c++) {
                         acc[i][c] = fmaf(a.x, b[c].x, acc[i][c]); acc[i][c] = fmaf(a.y, b[c].y, acc[i][c]);
                         acc[i][c] = fmaf(a.z, b[c].z, acc[i][c]); acc[i][c] = fmaf(a.w, b[c].w, acc[i][c]);
                     }
@@ -285,29 +297,30 @@ grouped_gemm_f32_vec_kernel(const GvParams p) {
             ptx::cp_async_commit();
         }
         ptx::cp_async_wait<0>();
-        __syncthreads();                                     // the ring is free: quarter sums [kq][row][column]
+        __syncthreads();                                     // the ring is free: sums [warp][row][column]
 #pragma unroll
         for (int i = 0; i < RT; i++)
 #pragma unroll
-            for (int c = 0; c < 4; c++) gv_smem[(kq * MT + ty + 4 * i) * GV_N + tx + 16 * c] = acc[i][c];
+            for (int c = 0; c < 8; c++) gv_smem[(warp * MT + ty + 4 * i) * GV_RLD + tx + 8 * c] = acc[i][c];
         __syncthreads();
-        // add the quarters in place; thread = 4 consecutive columns
+        // add the warps' sums in place; thread = 4 consecutive columns
         for (int o = tid; o < MT * GV_N / 4; o += GV_THREADS) {
-            float4* q = reinterpret_cast<float4*>(gv_smem) + o;
-            float4 s = q[0];
+            float* q = gv_smem + (o >> 4) * GV_RLD + 4 * (o & 15);
+            float4 s = *reinterpret_cast<const float4*>(q);
 #pragma unroll
-            for (int g = 1; g < 4; g++) {
-                const float4 v = q[g * MT * GV_N / 4];
+            for (int g = 1; g < GV_W; g++) {
+                const float4 v = *reinterpret_cast<const float4*>(q + g * MT * GV_RLD);
                 s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
             }
-            q[0] = s;
+            *reinterpret_cast<float4*>(q) = s;
         }
         if (csize > 1) cluster_sync(); else __syncthreads();
-        auto total4 = [&](int o) -> float4 {                 // the CTAs of the cluster in rank order
-            if (csize == 1) return reinterpret_cast<const float4*>(gv_smem)[o];
+        auto total4 = [&](int m, int c4) -> float4 {         // the CTAs of the cluster in rank order
+            const float* q = gv_smem + m * GV_RLD + 4 * c4;
+            if (csize == 1) return *reinterpret_cast<const float4*>(q);
             float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
             for (uint32_t r = 0; r < csize; r++) {
-                const float4 v = cluster_ld_f32x4(cluster_map(gv_smem + 4 * o, r));
+                const float4 v = cluster_ld_f32x4(cluster_map(q, r));
                 s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
             }
             return s;
@@ -316,7 +329,7 @@ grouped_gemm_f32_vec_kernel(const GvParams p) {
             for (int o = (int)crank * GV_THREADS + tid; o < MT * GV_N / 8; o += (int)csize * GV_THREADS) {
                 const int m = o >> 3, c4 = o & 7;            // row, 4 activation columns: gate at 4 c4, up 32 further
                 if (m0 + m >= cnt || n0 + 4 * c4 >= N) continue;
-                const float4 g = total4(m * (GV_N / 4) + c4), u = total4(m * (GV_N / 4) + 8 + c4);
+                const float4 g = total4(m, c4), u = total4(m, 8 + c4);
                 float4 r;
                 r.x = __fdiv_rn(g.x, 1.0f + expf(-g.x)) * u.x;   // silu as naive_moe.cu:308
                 r.y = __fdiv_rn(g.y, 1.0f + expf(-g.y)) * u.y;
@@ -328,7 +341,7 @@ grouped_gemm_f32_vec_kernel(const GvParams p) {
             for (int o = (int)crank * GV_THREADS + tid; o < MT * GV_N / 4; o += (int)csize * GV_THREADS) {
                 const int m = o >> 4, c4 = o & 15;
                 if (m0 + m >= cnt || n0 + 4 * c4 >= N) continue;
-                const float4 s = total4(o);
+                const float4 s = total4(m, c4);
                 const int pair = rows[m0 + m];
                 const float wv = p.wts[pair];
                 float* d = p.dst + (size_t)(pair / p.K) * p.D + n0 + 4 * c4;
@@ -522,12 +535,13 @@ static int launch_gemm_vec(const GvParams& p, int T, int E, int sm_count, cudaSt
                                            (int)gv_smem_bytes<MT>()));
     const int Kd = (MODE == 1) ? p.D : p.I, N = (MODE == 1) ? p.I : p.D;
     const int nx = ceil_div(N, (MODE == 1) ? GV_N / 2 : GV_N);
-    // walkers over an expert's row tiles: the mean and a half (a block loops over the tiles beyond)
-    const int ny = max(1, min(ceil_div(T, MT), ceil_div(3 * (p.TK / E + 1), 2 * MT)));
-    // cluster over k: until there are about two blocks per SM, at least two k-tiles each
+    // walkers over an expert's row tiles: one where the tile was chosen to hold the expert, else the mean and a half (a
+    // block loops over the tiles beyond)
+    const int ny = MT < 32 ? 1 : max(1, min(ceil_div(T, MT), ceil_div(3 * (p.TK / E + 1), 2 * MT)));
+    // cluster over k: until there are about two blocks per SM (what fits at a time)
     const int nkt = ceil_div(Kd, GV_KT);
     int cs = 1;
-    while (cs < 4 && (long long)nx * E * cs * 2 <= 2ll * sm_count && nkt / (2 * cs) >= 2) cs *= 2;
+    while (cs < 4 && (long long)nx * E * cs * 2 <= 2ll * sm_count && nkt >= 2 * cs) cs *= 2;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(nx, ny, E * cs);
     lc.blockDim = dim3(GV_THREADS);
@@ -605,14 +619,22 @@ int b200_moe_forward_f32(b200_ws* ws, const float* x, const float* gate_w, const
         GvParams p{};
         p.ids = ids; p.wts = wts; p.TK = T * K; p.K = K; p.D = D; p.I = I;
         if (!short_ids) { p.offsets = offsets; p.row_pair = row_pair; }
-        // Row tiles of 16 or 32: an expert's rows should mostly fit one tile (each tile streams the weights again),
-        // and a half-empty tile of 32 costs as many multiply-adds as a full one.
-        const bool wide = (long long)T * K > 16ll * E;
+        // Row tiles of 8 .. 32: the smallest that holds the mean row count and twice its spread (binomial: at most
+        // sqrt(mean)), because a second tile streams the weights again and an empty row costs as much as a full one.
+        const float mean = (float)T * K / E;
+        const int fit = min(T, (int)(mean + 2.0f * sqrtf(mean) + 0.999f));
+        auto gemm = [&](auto mode) -> int {
+            constexpr int M = decltype(mode)::value;
+            if (fit <= 8) return launch_gemm_vec<M, 8>(p, T, E, ws->sm_count, stream);
+            if (fit <= 16) return launch_gemm_vec<M, 16>(p, T, E, ws->sm_count, stream);
+            if (fit <= 24) return launch_gemm_vec<M, 24>(p, T, E, ws->sm_count, stream);
+            return launch_gemm_vec<M, 32>(p, T, E, ws->sm_count, stream);
+        };
         p.a = x; p.w = w1; p.dst = act;
-        st = wide ? launch_gemm_vec<1, 32>(p, T, E, ws->sm_count, stream) : launch_gemm_vec<1, 16>(p, T, E, ws->sm_count, stream);
+        st = gemm(std::integral_constant<int, 1>{});
         if (st) return st;
         p.a = act; p.w = w2; p.dst = out;
-        return wide ? launch_gemm_vec<2, 32>(p, T, E, ws->sm_count, stream) : launch_gemm_vec<2, 16>(p, T, E, ws->sm_count, stream);
+        return gemm(std::integral_constant<int, 2>{});
     }
     dim3 g1(ceil_div(I, G_TN), ceil_div(T, G_TM), E);
     grouped_gemm_f32_kernel<1><<<g1, 256, 0, stream>>>(x, w1, offsets, row_pair, nullptr, act, K, D, I);
