@@ -218,6 +218,54 @@ __device__ __forceinline__ void mma2_f8(uint32_t d_tmem, uint64_t adesc, uint64_
         : "memory");
 }
 
+// Four e4m3 bytes, two per conversion instruction.  The epilogue runs once per tile, from a cold instruction cache (7700 of
+// a decode tile's 72000 cycles, 9500 of a full one's 84000): what counts is how many instructions it has.
+__device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float d) {
+    return (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3) |
+           ((uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E4M3) << 16);
+}
+
+// tile_prefix[e] = tiles of experts < e.  Every CTA starts with this, so the offsets are fetched by all threads at once
+// and scanned from shared memory (a warp that walked the global array 32 experts at a time spent 3 us on 256 of them).
+__device__ __forceinline__ void count_tiles(GemmSmem* sm, const GemmParams& p, int rows_per_tile, int n_tiles) {
+    for (int e = threadIdx.x; e < p.E; e += GEMM_THREADS)
+        sm->tile_prefix[e] = ((p.offsets[e + 1] - p.offsets[e] + rows_per_tile - 1) / rows_per_tile) * n_tiles;
+}
+__device__ __forceinline__ void scan_tiles(GemmSmem* sm, int E) {
+    __syncthreads();                                          // the counts are there
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x, per = (E + 31) / 32, b = min(E, lane * per), n = min(E, b + per);
+        int sum = 0;
+        for (int e = b; e < n; e++) sum += sm->tile_prefix[e];
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        int before = incl - sum;
+        for (int e = b; e < n; e++) {
+            const int t = sm->tile_prefix[e];
+            sm->tile_prefix[e] = before;
+            before += t;
+        }
+        if (lane == 31) { sm->tile_prefix[E] = incl; sm->total_tiles = incl; }
+    }
+}
+
+// The rows of an A tile that exist, in whole groups of 32 (what a promotion warp owns): a decode batch has a few rows
+// per expert, and a full box of 128 would bring the next experts' rows along, a third of the stage's bytes.  The rows of
+// the stage that are not loaded hold older bytes; their products go to accumulator rows that nobody reads.
+// E = 256, K = 8, D = 7168 layer: T = 1 129 -> 116 us, T = 333 2105 -> 2065 us; equal where the experts are full.
+__device__ __forceinline__ uint32_t a_tile_bytes(int rows) { return rows > BM - 32 ? (uint32_t)A_BYTES : (uint32_t)((rows + 31) >> 5) * 32u * BK; }
+__device__ __forceinline__ void load_a_rows(uint8_t* dst, const CUtensorMap* map128, const CUtensorMap* map32, uint64_t* bar, int x,
+                                            int row0, uint32_t bytes) {
+    if (bytes == A_BYTES) {
+        ptx::tma_load_2d(dst, map128, bar, x, row0);
+    } else {
+        for (uint32_t o = 0; o < bytes; o += 32 * BK) ptx::tma_load_2d(dst + o, map32, bar, x, row0 + (int)(o / BK));
+    }
+}
 // acc[0..N-1] += v[0..N-1] * s  (B200_GEMM_PACKED_FMA: as N/2 fma.rn.f32x2, same bits)
 template <int N>
 __device__ __forceinline__ void promote(float* acc, const uint32_t (&v)[N], float s) {
@@ -256,8 +304,8 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[N]) {
 // the leader's `tmem_empty` barrier, and tcgen05.commit signals `empty` / `tmem_full` in both CTAs.
 template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                        const GemmParams p) {
+grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_a32,
+                        const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
     constexpr int TM = PAIR ? 2 * BM : BM;        // rows of a tile
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -288,33 +336,18 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         sm->abort_flag = 0;
         ptx::fence_mbar_init();
     }
-    if (warp == 0) {
-        // tile_prefix[e] = tiles of experts < e (warp scan over the expert counts)
-        int running = 0;
-        for (int e0 = 0; e0 < p.E; e0 += 32) {
-            const int e = e0 + lane;
-            int t = 0;
-            if (e < p.E) t = ((p.offsets[e + 1] - p.offsets[e] + TM - 1) / TM) * NT;
-            int incl = t;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
-            }
-            if (e < p.E) sm->tile_prefix[e] = running + incl - t;
-            running += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (lane == 0) { sm->tile_prefix[p.E] = running; sm->total_tiles = running; }
-    }
+    count_tiles(sm, p, TM, NT);
     if (warp == W_MMA0) {
         if (PAIR) { tmem_alloc2(&sm->tmem_base, 512); tmem_relinquish2(); }
         else      { ptx::tmem_alloc(&sm->tmem_base, 512); ptx::tmem_relinquish(); }
     }
     if (warp == W_TMA && lane == 0) {
         ptx::prefetch_tensormap(&tmap_a);
+        ptx::prefetch_tensormap(&tmap_a32);
         ptx::prefetch_tensormap(&tmap_b);
     }
     ptx::tc_fence_before();
+    scan_tiles(sm, p.E);
     __syncthreads();
     if (PAIR || duo) cluster_sync_all();      // the peer's barriers are initialised before anyone signals them
     ptx::tc_fence_after();
@@ -355,6 +388,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                     go_ph ^= 1;
                 }
                 const int row0 = p.offsets[e] + m_tile * TM + (int)crank * BM;
+                const uint32_t a_bytes = a_tile_bytes(cnt - m_tile * TM);
                 const long long wrow0 = (long long)e * w_rows;
                 for (int kb = 0; kb < nkb; kb++) {
                     if (!ptx::mbar_wait_relaxed(&sm->empty[s], ph ^ 1, abort_flag, 200)) goto done;
@@ -377,8 +411,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                             tma_load_2d_pair(b_dst, &tmap_b, fbar, kb * BK, (int)(wrow0 + n_tile * 256 + 128 * (int)crank));
                         }
                     } else {
-                        ptx::mbar_expect_tx(&sm->full[s], STAGE_BYTES);
-                        ptx::tma_load_2d(a_dst, &tmap_a, &sm->full[s], kb * BK, row0);
+                        ptx::mbar_expect_tx(&sm->full[s], a_bytes + B_BYTES);
+                        load_a_rows(a_dst, &tmap_a, &tmap_a32, &sm->full[s], kb * BK, row0, a_bytes);
                         if (p.packed) {
                             // the tile's K block is one contiguous 32 KB piece of the packed weights
                             ptx::tma_load_2d(b_dst, &tmap_b, &sm->full[s], 0, (((e * NT + n_tile) * nkb) + kb) * BN);
@@ -574,11 +608,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                     uint32_t packed[AC / 4];
 #pragma unroll
                     for (int i = 0; i < AC / 4; i++) {
-                        const float a0 = accv[4 * i], a1 = accv[4 * i + 1], a2 = accv[4 * i + 2], a3 = accv[4 * i + 3];
-                        packed[i] = (uint32_t)__nv_cvt_float_to_fp8(a0 * inv, __NV_SATFINITE, __NV_E4M3) |
-                                    ((uint32_t)__nv_cvt_float_to_fp8(a1 * inv, __NV_SATFINITE, __NV_E4M3) << 8) |
-                                    ((uint32_t)__nv_cvt_float_to_fp8(a2 * inv, __NV_SATFINITE, __NV_E4M3) << 16) |
-                                    ((uint32_t)__nv_cvt_float_to_fp8(a3 * inv, __NV_SATFINITE, __NV_E4M3) << 24);
+                        packed[i] = pack_e4m3x4(accv[4 * i] * inv, accv[4 * i + 1] * inv, accv[4 * i + 2] * inv, accv[4 * i + 3] * inv);
                     }
                     uint4* dst = reinterpret_cast<uint4*>(p.act_q + grow * p.I + n_tile * 128 + wq * AC);
 #pragma unroll
@@ -656,8 +686,8 @@ done:
 // -------------------------------------------------------------------------------------------------
 template <int MODE>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
-grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                       const GemmParams p) {
+grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_a32,
+                       const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
     static_assert(NUM_PROMO_WARPS == 8, "the block-scaled kernel is written for eight epilogue warps");
     constexpr int W_SF = W_MMA0 + 1;
     extern __shared__ uint8_t smem_raw[];
@@ -687,29 +717,15 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         sm->abort_flag = 0;
         ptx::fence_mbar_init();
     }
-    if (warp == 0) {
-        int running = 0;
-        for (int e0 = 0; e0 < p.E; e0 += 32) {
-            const int e = e0 + lane;
-            int t = 0;
-            if (e < p.E) t = ((p.offsets[e + 1] - p.offsets[e] + BM - 1) / BM) * NT;
-            int incl = t;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
-            }
-            if (e < p.E) sm->tile_prefix[e] = running + incl - t;
-            running += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (lane == 0) { sm->tile_prefix[p.E] = running; sm->total_tiles = running; }
-    }
+    count_tiles(sm, p, BM, NT);
     if (warp == W_MMA0) { ptx::tmem_alloc(&sm->tmem_base, 512); ptx::tmem_relinquish(); }
     if (warp == W_TMA && lane == 0) {
         ptx::prefetch_tensormap(&tmap_a);
+        ptx::prefetch_tensormap(&tmap_a32);
         ptx::prefetch_tensormap(&tmap_b);
     }
     ptx::tc_fence_before();
+    scan_tiles(sm, p.E);
     __syncthreads();
     if (duo) cluster_sync_all();              // the neighbour's barrier is initialised before anyone signals it
     ptx::tc_fence_after();
@@ -753,13 +769,14 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                     go_ph ^= 1;
                 }
                 const int row0 = p.offsets[e] + m_tile * BM;
+                const uint32_t a_bytes = a_tile_bytes(cnt - m_tile * BM);
                 const long long wrow0 = (long long)e * w_rows;
                 for (int kb = 0; kb < nkb; kb++) {
                     if (!ptx::mbar_wait_relaxed(&sm->empty[s], ph ^ 1, abort_flag, 200)) goto done;
                     uint8_t* a_dst = tiles + (size_t)s * STAGE_BYTES;
                     uint8_t* b_dst = a_dst + A_BYTES;
-                    ptx::mbar_expect_tx(&sm->full[s], STAGE_BYTES);
-                    ptx::tma_load_2d(a_dst, &tmap_a, &sm->full[s], kb * BK, row0);
+                    ptx::mbar_expect_tx(&sm->full[s], a_bytes + B_BYTES);
+                    load_a_rows(a_dst, &tmap_a, &tmap_a32, &sm->full[s], kb * BK, row0, a_bytes);
                     if (p.packed) {
                         ptx::tma_load_2d(b_dst, &tmap_b, &sm->full[s], 0, (((e * NT + n_tile) * nkb) + kb) * BN);
                     } else if (MODE == 1) {
@@ -938,11 +955,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                     uint32_t packed[AC / 4];
 #pragma unroll
                     for (int i = 0; i < AC / 4; i++) {
-                        const float a0 = accv[4 * i], a1 = accv[4 * i + 1], a2 = accv[4 * i + 2], a3 = accv[4 * i + 3];
-                        packed[i] = (uint32_t)__nv_cvt_float_to_fp8(a0 * inv, __NV_SATFINITE, __NV_E4M3) |
-                                    ((uint32_t)__nv_cvt_float_to_fp8(a1 * inv, __NV_SATFINITE, __NV_E4M3) << 8) |
-                                    ((uint32_t)__nv_cvt_float_to_fp8(a2 * inv, __NV_SATFINITE, __NV_E4M3) << 16) |
-                                    ((uint32_t)__nv_cvt_float_to_fp8(a3 * inv, __NV_SATFINITE, __NV_E4M3) << 24);
+                        packed[i] = pack_e4m3x4(accv[4 * i] * inv, accv[4 * i + 1] * inv, accv[4 * i + 2] * inv, accv[4 * i + 3] * inv);
                     }
                     uint4* dst = reinterpret_cast<uint4*>(p.act_q + grow * p.I + n_tile * 128 + wq * AC);
 #pragma unroll
@@ -1028,6 +1041,19 @@ reduce_rows_kernel(const float* __restrict__ rows, const int* __restrict__ pair_
     }
 }
 
+// 128 threads copy a row, four 16-byte loads in flight per thread
+__device__ __forceinline__ void copy_row(uint4* __restrict__ dst, const uint4* __restrict__ src, int n) {
+    for (int i0 = threadIdx.x; i0 < n; i0 += 512) {
+        uint4 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (i0 + 128 * j < n) v[j] = __ldg(src + i0 + 128 * j);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (i0 + 128 * j < n) dst[i0 + 128 * j] = v[j];
+    }
+}
+
 // Expert-sorted copy of the FP8 rows.  One block per sorted row, grid-stride (the number of valid
 // rows is only known on the device: slots owned by other ranks are not rows).
 __global__ void __launch_bounds__(128)
@@ -1044,7 +1070,7 @@ sort_rows_fp8_kernel(const uint8_t* __restrict__ xq, const float* __restrict__ x
         const int tok = pair / K;
         const uint4* src = reinterpret_cast<const uint4*>(xq + (size_t)tok * D);
         uint4* dst = reinterpret_cast<uint4*>(sq + (size_t)r * D);
-        for (int i = threadIdx.x; i < D / 16; i += blockDim.x) dst[i] = src[i];
+        copy_row(dst, src, D / 16);
         for (int i = threadIdx.x; i < nb; i += blockDim.x) ss[(size_t)r * nb + i] = xs[(size_t)tok * nb + i];
         if (threadIdx.x == 0) {
             row_tok[r] = tok;
@@ -1120,7 +1146,7 @@ sort_small_fp8_kernel(const uint8_t* __restrict__ xq, const float* __restrict__ 
     const int nb = D / 128;
     const uint4* src = reinterpret_cast<const uint4*>(xq + (size_t)tok * D);
     uint4* dst = reinterpret_cast<uint4*>(sq + (size_t)r * D);
-    for (int i = tid; i < D / 16; i += 128) dst[i] = src[i];
+    copy_row(dst, src, D / 16);
     for (int i = tid; i < nb; i += 128) ss[(size_t)r * nb + i] = xs[(size_t)tok * nb + i];
     if (tid == 0) {
         row_tok[r] = tok;
@@ -1279,7 +1305,7 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
     if ((cfg->flags & B200_MOE_SINGLE_CTA_TILES) || mx) pair = false;
     if (ws->sm_count < 2) pair = false;
     const unsigned grid = pair ? (unsigned)(ws->sm_count / 2) * 2 : (unsigned)ws->sm_count;
-    auto launch = [&](int mode, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p) -> int {
+    auto launch = [&](int mode, const CUtensorMap& ta, const CUtensorMap& ta32, const CUtensorMap& tb, const GemmParams& p) -> int {
         cudaLaunchConfig_t lc = {};
         lc.gridDim = dim3(grid); lc.blockDim = dim3(GEMM_THREADS); lc.stream = stream;
         lc.dynamicSmemBytes = mx ? GEMM_MX_SMEM_BYTES : GEMM_SMEM_BYTES;
@@ -1296,24 +1322,24 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
         lc.attrs = attr; lc.numAttrs = cluster2 ? 1 : 0;
         cudaError_t err;
         if (mx) {
-            if (mode == 1)      err = cudaLaunchKernelEx(&lc, grouped_gemm_mx_kernel<1>, ta, tb, p);
-            else if (mode == 2) err = cudaLaunchKernelEx(&lc, grouped_gemm_mx_kernel<2>, ta, tb, p);
-            else                err = cudaLaunchKernelEx(&lc, grouped_gemm_mx_kernel<3>, ta, tb, p);
+            if (mode == 1)      err = cudaLaunchKernelEx(&lc, grouped_gemm_mx_kernel<1>, ta, ta32, tb, p);
+            else if (mode == 2) err = cudaLaunchKernelEx(&lc, grouped_gemm_mx_kernel<2>, ta, ta32, tb, p);
+            else                err = cudaLaunchKernelEx(&lc, grouped_gemm_mx_kernel<3>, ta, ta32, tb, p);
         } else if (pair) {
-            if (mode == 1)      err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<1, true>, ta, tb, p);
-            else if (mode == 2) err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<2, true>, ta, tb, p);
-            else                err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<3, true>, ta, tb, p);
+            if (mode == 1)      err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<1, true>, ta, ta32, tb, p);
+            else if (mode == 2) err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<2, true>, ta, ta32, tb, p);
+            else                err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<3, true>, ta, ta32, tb, p);
         } else {
-            if (mode == 1)      err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<1, false>, ta, tb, p);
-            else if (mode == 2) err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<2, false>, ta, tb, p);
-            else                err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<3, false>, ta, tb, p);
+            if (mode == 1)      err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<1, false>, ta, ta32, tb, p);
+            else if (mode == 2) err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<2, false>, ta, ta32, tb, p);
+            else                err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<3, false>, ta, ta32, tb, p);
         }
         b200_count_launch(1);
         B200_CUDA_TRY(err);
         B200_CUDA_TRY(cudaGetLastError());
         return B200_OK;
     };
-    CUtensorMap ta, tb;
+    CUtensorMap ta, ta32, tb;
     GemmParams p{};
     p.offsets = s.offsets; p.E = E; p.D = D; p.I = I; p.status = ws->d_status; p.total_rows = TK;
 #ifdef B200_GEMM_TRACE
@@ -1322,6 +1348,7 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
 
     // GEMM1 (a CTA of a pair fetches half of a weight tile: boxes of 128 rows instead of 256)
     st = b200_make_tmap_u8_sw128(&ta, s.sq, (unsigned long long)TK, D, 128);
+    if (!st) st = b200_make_tmap_u8_sw128(&ta32, s.sq, (unsigned long long)TK, D, 32);
     if (st) return st;
     p.packed = packed ? 1 : 0;
     if (packed) st = b200_make_tmap_u8_sw128(&tb, w1q, (unsigned long long)E * 2 * I * (D / 128), 128, pair ? 128 : 256);
@@ -1329,13 +1356,14 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
     if (st) return st;
     p.a_scale = s.ss; p.w_scale = w1s; p.act_q = s.act_q; p.act_s = s.act_s;
     if (prof) B200_CUDA_TRY(cudaEventRecord(prof->ev[slot][0], stream));
-    st = launch(1, ta, tb, p);
+    st = launch(1, ta, ta32, tb, p);
     if (st) return st;
     if (prof) B200_CUDA_TRY(cudaEventRecord(prof->ev[slot][1], stream));
     if (!do_gemm2) return B200_OK;
 
     // GEMM2
     st = b200_make_tmap_u8_sw128(&ta, s.act_q, (unsigned long long)TK, I, 128);
+    if (!st) st = b200_make_tmap_u8_sw128(&ta32, s.act_q, (unsigned long long)TK, I, 32);
     if (st) return st;
     if (packed) st = b200_make_tmap_u8_sw128(&tb, w2q, (unsigned long long)E * D * (I / 128), 128, pair ? 128 : 256);
     else        st = b200_make_tmap_u8_sw128(&tb, w2q, (unsigned long long)E * D, I, pair ? 128 : 256);
@@ -1347,7 +1375,7 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
     if (det) {
         p.out = s.rows;
         if (prof) B200_CUDA_TRY(cudaEventRecord(prof->ev[slot][2], stream));
-        st = launch(3, ta, tb, p);
+        st = launch(3, ta, ta32, tb, p);
         if (st) return st;
         reduce_rows_kernel<<<T, 256, 0, stream>>>(s.rows, s.pair_row, ids, K, D, out);
         if (prof) { B200_CUDA_TRY(cudaEventRecord(prof->ev[slot][3], stream)); prof->calls++; }
@@ -1357,7 +1385,7 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
     }
     p.out = out;
     if (prof) B200_CUDA_TRY(cudaEventRecord(prof->ev[slot][2], stream));
-    st = launch(2, ta, tb, p);
+    st = launch(2, ta, ta32, tb, p);
     if (st) return st;
     if (prof) { B200_CUDA_TRY(cudaEventRecord(prof->ev[slot][3], stream)); prof->calls++; }
     return B200_OK;
