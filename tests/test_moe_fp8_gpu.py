@@ -334,3 +334,48 @@ def test_small_batch_router_bits(b200, cuda, T, E, D):
     oids, owts = oracle.route_grouped(xq, xs, wg, bias, 4, 4, 2, 2.5)
     assert np.array_equal(ids.cpu().numpy(), oids)
     assert np.abs(wts.cpu().numpy() - owts).max() <= 5e-7
+
+
+@pytest.mark.parametrize("counts", [[0, 1, 31, 32, 33], [96, 97, 128, 129, 0], [257, 5, 300, 0, 64],
+                                    [2, 1, 33, 7, 0, 1, 1, 64, 3]])
+@pytest.mark.parametrize("packed", [False, True])
+@pytest.mark.parametrize("pow2", [False, True])
+def test_row_groups_of_the_token_tiles(b200, cuda, counts, packed, pow2):
+    """Row counts at the edges of the 32-row groups that a tile loads and of the 128-row tiles, experts without rows, an
+    odd number of column tiles and of K blocks; both weight layouts, both scale rules and both combines; eight active
+    experts of 28 GEMM2 tiles give some CTAs a second tile (opened in front of the first one's epilogue)."""
+    rng = np.random.default_rng(sum(counts))
+    E, T, I = len(counts), sum(counts), 384
+    D = 7168 if E > 8 else 1280
+    x, wg, bias, w1, w2, xq, xs, w1q, w1s, w2q, w2s = _layer(rng, T, E, D, I, 0.02)
+    ids = rng.permutation(np.repeat(np.arange(E, dtype=np.int32), counts)).reshape(T, 1)
+    wts = rng.uniform(0.5, 1.5, (T, 1)).astype(np.float32)
+    if pow2:
+        with oracle.pow2_scales():
+            xq, xs = oracle.quant_act(x)
+            w1q, w1s = oracle.quant_weight(w1)
+            w2q, w2s = oracle.quant_weight(w2)
+    d = {k: _dev(v, cuda) for k, v in dict(xq=xq, xs=xs, ids=ids, wts=wts, w1=w1q, w1s=w1s, w2=w2q, w2s=w2s).items()}
+    call = b200.moe_fp8_experts
+    if packed:
+        for which, k in ((1, "w1"), (2, "w2")):
+            p = torch.empty_like(d[k])
+            b200.moe_fp8_pack_weights(which, d[k], p, E, D, I)
+            d[k] = p
+        call = b200.moe_fp8_experts_packed
+    rows = np.unique(np.concatenate([np.arange(min(T, 8)), rng.integers(0, T, 24)])).astype(np.int32)
+    args = (xq, xs, w1q, w1s, w2q, w2s, ids, wts, rows)
+    if pow2:
+        with oracle.pow2_scales():
+            ref = oracle.moe_fp8_experts(*args)
+    else:
+        ref = oracle.moe_fp8_experts(*args)
+    for det in (0, b200.MOE_DETERMINISTIC):
+        cfg = b200.MoeFp8Config(T, E, 1, D, I, b200.SCORE_SIGMOID_GROUPED, 1, 1, 1.0, det | (b200.MOE_POW2_SCALES if pow2 else 0))
+        out = torch.full((T, D), float("nan"), dtype=torch.float32, device=cuda)
+        call(d["xq"], d["xs"], d["ids"], d["wts"], d["w1"], d["w1s"], d["w2"], d["w2s"], out, cfg)
+        torch.cuda.synchronize()
+        assert b200.device_status() == 0
+        got = out.cpu().numpy()
+        assert np.isfinite(got).all()
+        assert not (np.abs(got[rows] - ref) > ATOL + RTOL * np.abs(ref)).any()
