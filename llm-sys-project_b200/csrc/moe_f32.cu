@@ -610,7 +610,7 @@ int b200_moe_forward_f32(b200_ws* ws, const float* x, const float* gate_w, const
                                  1.0f, stream);
         if (st) return st;
         if (!short_ids) {
-            st = launch_permute(ids, T, K, E, nullptr, true, counts, offsets, row_pair, stream);
+            st = launch_permute(ids, T, K, E, true, counts, offsets, row_pair, stream);
             if (st) return st;
         }
         B200_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(float) * (size_t)T * D, stream));   // naive_moe.cu:413

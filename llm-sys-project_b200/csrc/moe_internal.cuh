@@ -68,10 +68,10 @@ size_t moe_route_scratch_floats(int T, int E, int D);
 int moe_route_fp8_run(const RouteScratch& rs, const uint8_t* xq, const float* xs, const float* gate_w, const float* bias,
                       int* ids, float* wts, int* counts, float* logits_out, const b200_moe_fp8_config* cfg,
                       int* status, cudaStream_t stream);
-// counts_in: the router's per-expert histogram (may be NULL: counted from ids).  trusted: ids come from
-// this library's router (an expert appears at most once per token), so the duplicate check is skipped.
-int launch_permute(const int* ids, int T, int K, int E, const int* counts_in, bool trusted, int* counts,
-                   int* offsets, int* row_pair, cudaStream_t stream);
+// trusted: ids come from this library's router (an expert appears at most once per token), so the duplicate check is
+// skipped.
+int launch_permute(const int* ids, int T, int K, int E, bool trusted, int* counts, int* offsets, int* row_pair,
+                   cudaStream_t stream);
 // Same result with scratch of permute_ranges_scratch_ints integers: two launches whose work does not grow with E.
 size_t permute_ranges_scratch_ints(int T, int K, int E);
 int launch_permute_ranges(const int* ids, int T, int K, int E, bool trusted, int* range_hist, int* counts, int* offsets,

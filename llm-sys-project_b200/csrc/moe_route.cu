@@ -550,8 +550,7 @@ pair_histogram_kernel(const int* __restrict__ ids, int TK, int K, int E, int* __
 }
 
 // One block per expert.  The expert's first row (= rows owned by lower experts) comes from the
-// per-expert counts (the router's histogram, or pair_histogram_kernel for routing supplied from
-// outside); ranks inside the expert are assigned by a block scan over (token, slot) pairs in
+// per-expert counts of pair_histogram_kernel; ranks inside the expert are assigned by a block scan over (token, slot) pairs in
 // ascending order, four pairs per thread, 4096 pairs per round.
 // CHECK_DUP: a token that lists the expert twice counts once (ids supplied from outside).
 constexpr int PERMUTE_THREADS = 1024;
@@ -1156,21 +1155,19 @@ int moe_route_fp8_run(const RouteScratch& rs, const uint8_t* xq, const float* xs
                                cfg->topk_group, cfg->routed_scale, stream, exact);
 }
 
-int launch_permute(const int* ids, int T, int K, int E, const int* counts_in, bool trusted, int* counts,
-                   int* offsets, int* row_pair, cudaStream_t stream) {
+int launch_permute(const int* ids, int T, int K, int E, bool trusted, int* counts, int* offsets, int* row_pair,
+                   cudaStream_t stream) {
     const int TK = T * K;
-    if (!counts_in) {
-        // no histogram from the router: count first (all SMs), then every expert's block knows its base
-        B200_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int) * (size_t)E, stream));
-        const int blocks = max(1, min((TK + 1023) / 1024, 1184));
-        if (trusted) pair_histogram_kernel<false><<<blocks, 256, sizeof(int) * (size_t)E, stream>>>(ids, TK, K, E, counts);
-        else         pair_histogram_kernel<true><<<blocks, 256, sizeof(int) * (size_t)E, stream>>>(ids, TK, K, E, counts);
-        b200_count_launch(1);
-        B200_CUDA_TRY(cudaGetLastError());
-        counts_in = counts;       // each block rewrites its own entry with the same value at the end
-    }
+    // count first (all SMs), then every expert's block knows its base
+    B200_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int) * (size_t)E, stream));
+    const int blocks = max(1, min((TK + 1023) / 1024, 1184));
+    if (trusted) pair_histogram_kernel<false><<<blocks, 256, sizeof(int) * (size_t)E, stream>>>(ids, TK, K, E, counts);
+    else         pair_histogram_kernel<true><<<blocks, 256, sizeof(int) * (size_t)E, stream>>>(ids, TK, K, E, counts);
+    b200_count_launch(1);
+    B200_CUDA_TRY(cudaGetLastError());
+    // (each block rewrites its own entry of counts with the same value at the end)
     const cudaError_t err = b200_launch_after(trusted ? permute_kernel<false> : permute_kernel<true>, dim3(E), PERMUTE_THREADS, 0, stream,
-                                              ids, TK, K, E, counts_in, counts, offsets, row_pair);
+                                              ids, TK, K, E, counts, counts, offsets, row_pair);
     b200_count_launch(1);
     B200_CUDA_TRY(err);
     B200_CUDA_TRY(cudaGetLastError());
@@ -1283,7 +1280,7 @@ int b200_moe_permute(b200_ws*, const int* expert_ids, int T, int K, int E, int* 
                      int* row_pair, b200_stream_t stream) {
     if (!expert_ids || !counts || !offsets || !row_pair) return B200_BAD_ARG;
     if (T <= 0 || K <= 0 || E <= 0) return B200_BAD_SHAPE;
-    return launch_permute(expert_ids, T, K, E, nullptr, false, counts, offsets, row_pair, stream);
+    return launch_permute(expert_ids, T, K, E, false, counts, offsets, row_pair, stream);
 }
 
 }  // extern "C"
