@@ -20,9 +20,10 @@
 //                K block into a 4-stage shared-memory ring (128-byte swizzle, K-major).
 //   warps 9,10   MMA issuers, one per 256-column TMEM accumulator stage (K blocks alternate between
 //                them): 4 x tcgen05.mma kind::f8f6f4 (K = 32 each) per K block, started fresh for
-//                every K block.  Everything that waits next to the promotion warps sleeps between
-//                polls: a warp that spins takes issue slots from the promotion warps that share
-//                its scheduler.
+//                every K block.  The issuers wait in mbarrier.try_wait (two lanes, which the
+//                hardware suspends): with 64 ns of sleep between polls they noticed a free stage ~300 cycles
+//                late, and with 200 ns the producer an empty slot (32 experts x 1024 rows 2071 -> 2044 us,
+//                T = 4096 3168 -> 3135 us).
 //   warps 0-7    promotion + epilogue: tcgen05.ld the K block's partial sums and fold them
 //                into fp32 registers with a_scale[row,kb] * w_scale[nblk,kb] (the scales are
 //                arbitrary fp32 values, so the scaling cannot be left to the tensor core).
@@ -53,7 +54,7 @@ constexpr int QCOLS = BN / NQ;               // accumulator columns per promotio
 constexpr int GEMM_THREADS = 32 * (NUM_PROMO_WARPS + 4);   // promotion/epilogue warpgroups, then the TMA + MMA warpgroup
 constexpr int W_TMA = NUM_PROMO_WARPS, W_MMA0 = NUM_PROMO_WARPS + 1;
 constexpr int MAX_E = 1024;
-constexpr unsigned ISSUER_SLEEP_NS = 64;
+constexpr unsigned PRODUCER_SLEEP_NS = 40;
 // Register budgets after setmaxnreg.  The registers a warpgroup gives up are the only ones the others can
 // take (the pool is what the CTA was launched with: GEMM_THREADS x LAUNCH_REGS), and setmaxnreg.inc waits
 // without bound until its request is met, so the two sides must balance:
@@ -391,7 +392,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                 const uint32_t a_bytes = a_tile_bytes(cnt - m_tile * TM);
                 const long long wrow0 = (long long)e * w_rows;
                 for (int kb = 0; kb < nkb; kb++) {
-                    if (!ptx::mbar_wait_relaxed(&sm->empty[s], ph ^ 1, abort_flag, 200)) goto done;
+                    if (!ptx::mbar_wait_relaxed(&sm->empty[s], ph ^ 1, abort_flag, PRODUCER_SLEEP_NS)) goto done;
                     TRACE_STAMP(6, gk); gk++;
                     uint8_t* a_dst = tiles + (size_t)s * STAGE_BYTES;
                     uint8_t* b_dst = a_dst + A_BYTES;
@@ -447,7 +448,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                     if ((int)(g & 1) == role) {
                         // (waits on barriers that the peer CTA or tcgen05.commit signal need no cluster-scope
                         // acquire: what they hand over is a TMEM stage or TMA-written tiles, not memory data)
-                        if (!ptx::mbar_wait_relaxed(&sm->tmem_empty[role], acc_ph ^ 1, abort_flag, ISSUER_SLEEP_NS)) goto done;
+                        if (!ptx::mbar_wait(&sm->tmem_empty[role], acc_ph ^ 1, abort_flag)) goto done;
                         TRACE_STAMP(0, g);
                         if (!ptx::mbar_wait(&sm->full[s], ph, abort_flag)) goto done;
                         TRACE_STAMP(1, g);
@@ -794,7 +795,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                 const uint32_t a_bytes = a_tile_bytes(cnt - m_tile * BM);
                 const long long wrow0 = (long long)e * w_rows;
                 for (int kb = 0; kb < nkb; kb++) {
-                    if (!ptx::mbar_wait_relaxed(&sm->empty[s], ph ^ 1, abort_flag, 200)) goto done;
+                    if (!ptx::mbar_wait_relaxed(&sm->empty[s], ph ^ 1, abort_flag, PRODUCER_SLEEP_NS)) goto done;
                     uint8_t* a_dst = tiles + (size_t)s * STAGE_BYTES;
                     uint8_t* b_dst = a_dst + A_BYTES;
                     ptx::mbar_expect_tx(&sm->full[s], a_bytes + B_BYTES);
