@@ -303,7 +303,8 @@ dsa_cluster_f32_kernel(const float* __restrict__ q_nope, const float* __restrict
             for (int g = 0; g < rgs; g++) part += cluster_ld_f32(cluster_map(&acc_s[(size_t)g * FC_HB * Dc + i], r));
             o = fmaf(part, f, o);
         }
-        if (h0 + hh < H) out[((size_t)q * H + h0) * Dc + i] = L > 0.0f ? o * (1.0f / L) : 0.0f;
+        // every entry empty: o = 0 and the factor 0; a NaN score or an overflow makes o and L NaN, and the product stays NaN
+        if (h0 + hh < H) out[((size_t)q * H + h0) * Dc + i] = o * (L > 0.0f ? 1.0f / L : 0.0f);
     }
     cluster_sync();                        // nobody leaves while a neighbour still reads its shared memory
 }

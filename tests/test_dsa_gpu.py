@@ -235,3 +235,57 @@ def test_f32_cluster_split_edges(b200, cuda, Q, H, Dc, Dp, S):
             sc = torch.cat([qn[i], qp[i]], 1).double() @ torch.cat([kc[r], kp[r]], 1).double().T / (Dc + Dp) ** 0.5
             ref[i] = torch.softmax(sc, 1) @ v[r].double()
     assert (out.cpu().double() - ref).abs().max().item() < 1e-5
+
+
+@pytest.mark.parametrize("S", [20, 100, 300])
+@pytest.mark.parametrize("Dc,Dp", [(64, 16), (512, 64)])
+@pytest.mark.parametrize("what", ["nan in K", "nan in Q", "score overflow", "nan in V", "-inf score", "all -inf", "all empty", "nan not selected"])
+def test_f32_kernels_agree_on_special_values(b200, cuda, what, Dc, Dp, S):
+    """NaN, infinities and empty lists through both fp32 kernels (tensors that start 4 bytes off a 16-byte boundary take
+    the general one): the same elements are NaN or zero, the others agree.  A NaN or an overflow is never hidden."""
+    g = torch.Generator(device="cpu").manual_seed(S * 1000 + Dc)
+    Q, H, N = 3, 6, 2 * S
+    rnd = lambda *s: torch.randn(s, generator=g)
+    qn, qp, kc, kp, v = rnd(Q, H, Dc), rnd(Q, H, Dp), rnd(N, Dc), rnd(N, Dp), rnd(N, Dc)
+    qn[:, :, 0] = qn[:, :, 0].abs() + 0.5
+    idx = torch.stack([torch.randperm(N, generator=g)[:S] for _ in range(Q)]).to(torch.int32)
+    row = int(idx[0, S // 2])                                   # poisoned row: query 0 lists it, perhaps others too
+    bad = torch.zeros((Q, H), dtype=torch.bool)
+    lists = (idx == row).any(1)[:, None].expand(Q, H)
+    zero = torch.zeros((Q, H), dtype=torch.bool)
+    if what == "nan in K":
+        kc[row, 5] = float("nan")
+        bad = lists
+    elif what == "nan in Q":
+        qp[1, 2, 3] = float("nan")
+        bad[1, 2] = True
+    elif what == "score overflow":                               # finite inputs: 0.5 * 3e38 * 8 > FLT_MAX
+        kc[row], kp[row] = 0.0, 0.0
+        kc[row, 0], qn[:, :, 0] = 3e38, 8.0
+        bad = lists
+    elif what == "nan in V":
+        v[row, :] = float("nan")
+        bad = lists
+    elif what == "-inf score":                                   # weight zero, no effect on the others
+        kc[row], kp[row] = 0.0, 0.0
+        kc[row, 0] = -float("inf")
+    elif what == "all -inf":
+        kc[:, 0] = -float("inf")
+        zero[:] = True
+    elif what == "all empty":
+        idx[1] = -1
+        zero[1] = True
+    else:
+        idx[idx == row] = -1
+        kc[row], v[row] = float("nan"), float("nan")
+    got = []
+    for off in (0, 1):
+        d = lambda t: torch.empty(t.numel() + 1, device=cuda)[off:off + t.numel()].view(t.shape).copy_(t)
+        out = torch.full((Q, H, Dc), 7.0, device=cuda)
+        b200.dsa_forward(d(qn), d(qp), d(kc), d(kp), d(v), idx.to(cuda), out, b200.DsaConfig(Q, H, Dc, Dp, S, 64, N))
+        got.append(out.cpu())
+    for o in got:
+        assert torch.equal(torch.isnan(o), bad[:, :, None].expand_as(o))
+        assert (o[zero] == 0).all()
+    a, b = (torch.nan_to_num(o, nan=0.0) for o in got)
+    assert (a - b).abs().max().item() < 1e-5
