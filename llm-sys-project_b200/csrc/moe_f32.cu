@@ -352,7 +352,10 @@ grouped_gemm_f32_vec_kernel(const GvParams p) {
         // the ring is refilled (and the CTA may leave) only when nobody reads the sums any more
         if (csize > 1) cluster_sync(); else __syncthreads();
     }
-    ptx::cp_async_wait<0>();                                 // tiles requested early for an expert without rows
+    // An expert without rows never entered the loop: its early tiles belong to no group yet, and nothing may be on its way
+    // into this block's shared memory when the block leaves.
+    ptx::cp_async_commit();
+    ptx::cp_async_wait<0>();
 }
 
 // Router of the vector path: block = 8 tokens x all (at most 32) experts, thread = one (token, expert) chain in the

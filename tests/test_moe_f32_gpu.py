@@ -175,3 +175,24 @@ def test_vector_path_edges(b200, cuda, T, E, K, D, I):
     ids, wts, ref = oracle.moe_forward_f32(x, wg, w1, w2, K)
     out = _run_forward(b200, cuda, x, wg, w1, w2, K)
     assert np.abs(out - ref).max() < 1e-5 * max(1.0, np.abs(ref).max())
+
+
+@pytest.mark.parametrize("T,E,K,D,I", [(1, 32, 1, 512, 512), (3, 32, 1, 260, 516), (2, 40, 2, 512, 256)])
+def test_most_experts_without_rows(b200, cuda, T, E, K, D, I):
+    """Blocks of experts nobody chose request weight tiles and then leave without using them (they wait for the copies
+    first).  Many calls back to back, so that the next blocks take over their shared memory; every result against the
+    oracle, fp32 sums of at most 516 products."""
+    rng = np.random.default_rng(E + D)
+    x = rng.normal(0, 1, (T, D)).astype(np.float32)
+    wg = rng.normal(0, D ** -0.5, (E, D)).astype(np.float32)
+    w1 = rng.normal(0, D ** -0.5, (E, 2 * I, D)).astype(np.float32)
+    w2 = rng.normal(0, I ** -0.5, (E, D, I)).astype(np.float32)
+    _, _, ref = oracle.moe_forward_f32(x, wg, w1, w2, K)
+    d = [_dev(a, cuda) for a in (x, wg, w1, w2)]
+    cfg = b200.MoeConfig(T, E, K, D, I)
+    outs = [torch.full((T, D), float("nan"), dtype=torch.float32, device=cuda) for _ in range(50)]
+    for out in outs:
+        b200.moe_forward(*d, out, cfg)
+    torch.cuda.synchronize()
+    for out in outs:
+        assert np.abs(out.cpu().numpy() - ref).max() < 1e-5 * max(1.0, np.abs(ref).max())
