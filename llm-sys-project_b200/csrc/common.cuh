@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include "../../include/b200_moe_dsa.h"
+#include "once.h"
 
 #define B200_CUDA_TRY(expr)                                      \
     do {                                                         \
@@ -66,15 +67,20 @@ static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 // ---------------------------------------------------------------------------
 // Device-side PTX wrappers
 // ---------------------------------------------------------------------------
-// Function attributes (dynamic shared-memory limits) belong to a device: a process that drives several
-// GPUs has to set them once per device, not once per process.  Returns true the first time it is called
-// for the current device with a given flag array (64 entries, zero-initialised static storage).
-static inline bool b200_first_call_on_device(bool* done_by_device) {
+// setup() once for the current device (`once`: static storage of the caller).
+template <typename F>
+static inline int b200_once_on_device(B200PerDeviceOnce& once, F setup) {
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return true;
-    if (done_by_device[dev]) return false;
-    done_by_device[dev] = true;
-    return true;
+    B200_CUDA_TRY(cudaGetDevice(&dev));
+    return once.run(dev, setup);
+}
+// Dynamic shared memory above the default limit has to be allowed per kernel and device.
+template <typename... P>
+static inline int b200_allow_smem(B200PerDeviceOnce& once, void (*kernel)(P...), size_t bytes) {
+    return b200_once_on_device(once, [&]() -> int {
+        B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        return B200_OK;
+    });
 }
 
 // Launch with programmatic stream serialisation: the kernel may start while the kernel in front of it in the stream

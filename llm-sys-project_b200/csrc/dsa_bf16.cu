@@ -429,11 +429,9 @@ int dsa_bf16_impl(b200_ws* ws, const uint16_t* q_nope, const uint16_t* q_pe, con
         }
         return B200_OK;
     }
-    static bool attr_done[64] = {false};
-    if (b200_first_call_on_device(attr_done)) {
-        B200_CUDA_TRY(cudaFuncSetAttribute(dsa_decode_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)DSA_SMEM_BYTES));
-    }
+    static B200PerDeviceOnce smem;
+    const int st = b200_allow_smem(smem, dsa_decode_bf16_kernel, DSA_SMEM_BYTES);
+    if (st) return st;
     DsaParams p;
     p.q_nope = reinterpret_cast<const __nv_bfloat16*>(q_nope);
     p.q_pe = reinterpret_cast<const __nv_bfloat16*>(q_pe);

@@ -398,8 +398,9 @@ static int launch_dsa_f32(const float* qn, const float* qp, const float* kc, con
     while (TS > 1 && need(TS) > smem_limit) TS >>= 1;
     if (need(TS) > smem_limit) return B200_UNSUPPORTED;
     size_t smem = need(TS);
-    B200_CUDA_TRY(cudaFuncSetAttribute(dsa_fused_f32_kernel<NJ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem));
+    static B200PerDeviceOnce once;
+    const int st = b200_allow_smem(once, dsa_fused_f32_kernel<NJ>, smem_limit);
+    if (st) return st;
     dim3 grid(c->num_queries, ceil_div(c->num_heads, DSA_HB));
     float scale = 1.0f / sqrtf((float)Dk);        // naive_dsa.cu:464
     dsa_fused_f32_kernel<NJ><<<grid, DSA_HB * 32, smem, stream>>>(qn, qp, kc, kp, v, idx, out, c->num_heads, Dc, Dp,

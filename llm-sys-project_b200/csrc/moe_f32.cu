@@ -532,10 +532,9 @@ __global__ void scatter_f32_kernel(const float* __restrict__ expert_out, const i
 // one grouped GEMM launch of the vector path
 template <int MODE, int MT>
 static int launch_gemm_vec(const GvParams& p, int T, int E, int sm_count, cudaStream_t stream) {
-    static bool attr_done[64] = {false};
-    if (b200_first_call_on_device(attr_done))
-        B200_CUDA_TRY(cudaFuncSetAttribute(grouped_gemm_f32_vec_kernel<MODE, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)gv_smem_bytes<MT>()));
+    static B200PerDeviceOnce once;
+    const int st = b200_allow_smem(once, grouped_gemm_f32_vec_kernel<MODE, MT>, gv_smem_bytes<MT>());
+    if (st) return st;
     const int Kd = (MODE == 1) ? p.D : p.I, N = (MODE == 1) ? p.I : p.D;
     const int nx = ceil_div(N, (MODE == 1) ? GV_N / 2 : GV_N);
     // walkers over an expert's row tiles: one where the tile was chosen to hold the expert, else the mean and a half (a
@@ -599,10 +598,9 @@ int b200_moe_forward_f32(b200_ws* ws, const float* x, const float* gate_w, const
     const bool vec = D % 4 == 0 && I % 4 == 0 && (all & 15) == 0 && (long long)E * 4 <= 65535;
     const bool short_ids = vec && (long long)T * K <= GV_PAIRS;      // the GEMM blocks list their rows themselves
     if (vec && E <= GR_MAXE && short_ids) {
-        static bool attr_done[64] = {false};
-        if (b200_first_call_on_device(attr_done))
-            B200_CUDA_TRY(cudaFuncSetAttribute(gate_select_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)gr_smem_bytes(GR_MAXE)));
+        static B200PerDeviceOnce once;
+        st = b200_allow_smem(once, gate_select_f32_kernel, gr_smem_bytes(GR_MAXE));
+        if (st) return st;
         gate_select_f32_kernel<<<ceil_div(T, GR_T), GR_T * GR_MAXE, gr_smem_bytes(E), stream>>>(x, gate_w, ids, wts, out, T, E, K, D);
         b200_count_launch(1);
         B200_CUDA_TRY(cudaGetLastError());

@@ -1215,8 +1215,6 @@ __global__ void pack_weights_kernel(int which, const uint8_t* __restrict__ src, 
     *reinterpret_cast<uint4*>(packed + i * 16) = v;
 }
 
-bool g_regs_ok = true;
-
 struct Fp8Scratch {
     RouteScratch route; int* ids; float* wts; int* range_hist; int* counts; int* offsets; int* row_pair;
     uint8_t* sq; float* ss; int* row_tok; float* row_w; uint8_t* act_q; float* act_s;
@@ -1292,8 +1290,8 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
     b200_count_launch(1);
     B200_CUDA_TRY(cudaGetLastError());
 
-    static bool attr_done[64] = {false};
-    if (b200_first_call_on_device(attr_done)) {
+    static B200PerDeviceOnce once;
+    st = b200_once_on_device(once, []() -> int {
         const void* kernels[9] = {(const void*)grouped_gemm_fp8_kernel<1, false>, (const void*)grouped_gemm_fp8_kernel<2, false>,
                                   (const void*)grouped_gemm_fp8_kernel<3, false>, (const void*)grouped_gemm_fp8_kernel<1, true>,
                                   (const void*)grouped_gemm_fp8_kernel<2, true>, (const void*)grouped_gemm_fp8_kernel<3, true>,
@@ -1308,14 +1306,14 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
             cudaFuncAttributes a{};
             B200_CUDA_TRY(cudaFuncGetAttributes(&a, kernels[i]));
             const int n = a.numRegs;
-            if (!(n * GEMM_THREADS <= 65536 && n <= PROMO_REGS && NUM_PROMO_WARPS * (PROMO_REGS - n) <= 4 * (n - AUX_REGS)))
-                g_regs_ok = false;
+            if (!(n * GEMM_THREADS <= 65536 && n <= PROMO_REGS && NUM_PROMO_WARPS * (PROMO_REGS - n) <= 4 * (n - AUX_REGS))) {
+                b200_set_last_error_text("grouped GEMM: the compiled register count does not balance the setmaxnreg budgets");
+                return B200_UNSUPPORTED;
+            }
         }
-    }
-    if (!g_regs_ok) {
-        b200_set_last_error_text("grouped GEMM: the compiled register count does not balance the setmaxnreg budgets");
-        return B200_UNSUPPORTED;
-    }
+        return B200_OK;
+    });
+    if (st) return st;
     b200_gemm_profile* prof = (ws->gemm_prof && ws->gemm_prof->on) ? ws->gemm_prof : nullptr;
     const int slot = prof ? (int)(prof->calls % PROF_SLOTS) : 0;
     // Single-CTA 128-row tiles unless the caller asks for CTA pairs.  Measured on B200 the pair tiles (256 rows,

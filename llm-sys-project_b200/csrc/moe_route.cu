@@ -144,6 +144,7 @@ gate_logits_kernel(const void* __restrict__ x_, const float* __restrict__ xs, co
 // ---------------------------------------------------------------------------
 // selection
 // ---------------------------------------------------------------------------
+constexpr int ROUTE_MAX_E = 4096;            // 128 KB of scores for the four warps of route_select_kernel
 struct ValIdx { float v; int i; };
 __device__ __forceinline__ ValIdx better(ValIdx a, ValIdx b) {
     // larger value wins; equal values -> lower index wins; index -1 = empty
@@ -960,12 +961,9 @@ gate_logits_fp8_tile_kernel(const uint8_t* __restrict__ xq, const float* __restr
 
 constexpr int GT_MAX_T = 256;
 static int gate_tile_attr() {
-    static bool attr_done[64] = {false};
-    if (b200_first_call_on_device(attr_done)) {
-        B200_CUDA_TRY(cudaFuncSetAttribute(gate_logits_fp8_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM));
-        B200_CUDA_TRY(cudaFuncSetAttribute(gate_logits_fp8_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM));
-    }
-    return B200_OK;
+    static B200PerDeviceOnce whole, list;
+    const int st = b200_allow_smem(whole, gate_logits_fp8_tile_kernel<false>, GT_SMEM);
+    return st ? st : b200_allow_smem(list, gate_logits_fp8_tile_kernel<true>, GT_SMEM);
 }
 
 template <int TY>
@@ -1006,20 +1004,25 @@ int launch_gate_logits(const void* x, const float* xs, const float* wg, float* p
     if (fp8 && vec) {
         // Pick the token-tile height (8 * TY rows) whose tile count wastes the least of the machine:
         // tiles come in waves of (SMs x resident CTAs); cost ~ waves x rows per tile.
-        static int sms = 0;
-        static int occ[17] = {0};
-        if (!sms) {
-            int dev = 0;
-            B200_CUDA_TRY(cudaGetDevice(&dev));
-            B200_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        struct Machine { int sms, occ[17]; };
+        static B200PerDeviceOnce once;
+        static Machine machine[64];
+        int dev = 0;
+        B200_CUDA_TRY(cudaGetDevice(&dev));
+        Machine& m = machine[dev & 63];
+        const int st = once.run(dev, [&]() -> int {
             for (int ty = 8; ty <= 16; ty++) {
                 int b = 0;
                 gate_fp8_try<8>(ty, b) || gate_fp8_try<9>(ty, b) || gate_fp8_try<10>(ty, b) || gate_fp8_try<11>(ty, b) ||
                     gate_fp8_try<12>(ty, b) || gate_fp8_try<13>(ty, b) || gate_fp8_try<14>(ty, b) ||
                     gate_fp8_try<15>(ty, b) || gate_fp8_try<16>(ty, b);
-                occ[ty] = b > 0 ? b : 1;
+                m.occ[ty] = b > 0 ? b : 1;
             }
-        }
+            B200_CUDA_TRY(cudaDeviceGetAttribute(&m.sms, cudaDevAttrMultiProcessorCount, dev));
+            return B200_OK;
+        });
+        if (st) return st;
+        const int sms = m.sms, *const occ = m.occ;
         int best_ty = 16;
         double best_cost = 1e300;
         for (int ty = 16; ty >= 8; ty--) {
@@ -1078,10 +1081,12 @@ int launch_gate_logits_list(const uint8_t* xq, const float* xs, const float* wg,
 int launch_route_select(const float* partials, int n_chunks, const float* bias, int* ids, float* wts, int* counts,
                         float* logits_out, int T, int E, int K, int scoring, int n_group, int topk_group,
                         float routed_scale, cudaStream_t stream, RouteCert cert) {
-    size_t smem = (size_t)4 * 2 * E * sizeof(float);
+    auto smem_of = [](int experts) { return (size_t)4 * 2 * experts * sizeof(float); };
+    const size_t smem = smem_of(E);
     if (smem > 48 * 1024) {
-        B200_CUDA_TRY(cudaFuncSetAttribute(route_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem));
+        static B200PerDeviceOnce once;
+        const int st = b200_allow_smem(once, route_select_kernel, smem_of(ROUTE_MAX_E));
+        if (st) return st;
     }
     // list mode: the length of the list is known only on the device; a modest grid walks it with a stride
     const int blocks = cert.list ? min(ceil_div(T, 4), 4 * 148) : ceil_div(T, 4);
@@ -1181,12 +1186,11 @@ int launch_permute_ranges(const int* ids, int T, int K, int E, bool trusted, int
     if (E > PR_THREADS) return B200_UNSUPPORTED;
     const int TK = T * K, ranges = ceil_div(TK, PR_PAIRS);
     const size_t smem = (size_t)E * sizeof(int) + (size_t)(PR_THREADS / 32) * E * sizeof(unsigned short);
-    static bool attr_done[64] = {false};
-    if (b200_first_call_on_device(attr_done)) {
-        const int most = PR_THREADS * (int)(sizeof(int) + (PR_THREADS / 32) * sizeof(unsigned short));
-        B200_CUDA_TRY(cudaFuncSetAttribute(permute_ranges_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-        B200_CUDA_TRY(cudaFuncSetAttribute(permute_ranges_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    }
+    static B200PerDeviceOnce plain, checked;
+    const size_t most = PR_THREADS * (sizeof(int) + (PR_THREADS / 32) * sizeof(unsigned short));
+    const int st = trusted ? b200_allow_smem(plain, permute_ranges_kernel<false>, most)
+                           : b200_allow_smem(checked, permute_ranges_kernel<true>, most);
+    if (st) return st;
     B200_CUDA_TRY(b200_launch_after(trusted ? permute_ranges_count_kernel<false> : permute_ranges_count_kernel<true>, dim3(ranges),
                                     PR_THREADS, sizeof(int) * (size_t)E, stream, ids, TK, K, E, range_hist));
     B200_CUDA_TRY(b200_launch_after(trusted ? permute_ranges_kernel<false> : permute_ranges_kernel<true>, dim3(ranges), PR_THREADS,
@@ -1199,7 +1203,7 @@ int launch_permute_ranges(const int* ids, int T, int K, int E, bool trusted, int
 int check_route_cfg(int T, int E, int K, int D, int scoring, int n_group, int topk_group) {
     if (T <= 0 || E <= 0 || K <= 0 || D <= 0) return B200_BAD_SHAPE;
     if (K > E) return B200_BAD_SHAPE;           // the reference would leave -1 ids (never exercised)
-    if (E > 4096) return B200_UNSUPPORTED;
+    if (E > ROUTE_MAX_E) return B200_UNSUPPORTED;
     if (scoring == B200_SCORE_SIGMOID_GROUPED) {
         if (n_group <= 0 || n_group > 32 || E % n_group) return B200_BAD_SHAPE;
         if (topk_group <= 0 || topk_group > n_group) return B200_BAD_SHAPE;

@@ -312,15 +312,17 @@ int launch_gate_logits_tc(const uint8_t* xq, const float* xs, const float* wg, f
     if (st) return st;
     const int N = E;
     const size_t smem = 1024 + (size_t)NSTAGE * (2 * A_TILE + 2 * (size_t)N * KS * 4) + sizeof(TcSmem) + 64;
-    static bool attr_done[64] = {false};
+    static B200PerDeviceOnce once;
     static int sm_count[64] = {0};
     int dev = 0;
     B200_CUDA_TRY(cudaGetDevice(&dev));
-    if (b200_first_call_on_device(attr_done)) {
+    st = once.run(dev, [&]() -> int {
         B200_CUDA_TRY(cudaFuncSetAttribute(gate_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)(1024 + (size_t)NSTAGE * (2 * A_TILE + 2 * (size_t)MAX_N * KS * 4) + sizeof(TcSmem) + 64)));
         B200_CUDA_TRY(cudaDeviceGetAttribute(&sm_count[dev & 63], cudaDevAttrMultiProcessorCount, dev));
-    }
+        return B200_OK;
+    });
+    if (st) return st;
     TcPlan plan;
     plan.nblk = D / 128;
     plan.ch = min(tc_chain(), plan.nblk);
