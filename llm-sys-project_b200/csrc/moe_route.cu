@@ -164,8 +164,17 @@ __device__ __forceinline__ ValIdx warp_argmax(ValIdx x) {
     return x;
 }
 
+// A NaN score (NaN weights, bias or activations) ranks below every number, so that all lanes and both selection kernels
+// see one order: an expert with a NaN is taken only where no other is left, and its weight is NaN then.  (Volatile: with
+// fmaxf the compiler moved the eight sigmoids of a lane, and a one-token layer took 108.6 us instead of 107.8.)
+__device__ __forceinline__ float rankable(float score) {
+    asm volatile("max.f32 %0, %0, 0fFF800000;" : "+f"(score));
+    return score;
+}
+
 // The same result in three warp-wide steps instead of ten dependent shuffles, for lanes that hold ascending runs of
-// indices (ties: the lowest lane, and inside a lane the caller kept the lowest index).  x.i < 0: no candidate.
+// indices (ties: the lowest lane, and inside a lane the caller kept the lowest index).  x.i < 0: no candidate.  The
+// scores are rankable: a NaN would order above every number here.
 __device__ __forceinline__ ValIdx warp_argmax_ordered(ValIdx x) {
     const unsigned u = __float_as_uint(x.v + 0.0f);                       // -0 counts as +0
     const unsigned key = x.i < 0 ? 0u : ((u & 0x80000000u) ? ~u : (u | 0x80000000u));
@@ -246,7 +255,8 @@ route_select_row(const float* __restrict__ partials, int n_chunks, const float* 
         for (int e = lane; e < E; e += 32) ss = fmaf(s[e], s[e], ss);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        tau *= fmaxf(1.0f, sqrtf(ss / (float)E));
+        const float rms = sqrtf(ss / (float)E);
+        if (!(rms <= 1.0f)) tau *= rms;          // a NaN logit makes the threshold NaN: the exact pass decides
     }
     for (int e = lane; e < E; e += 32) {
         // exact logits: correctly rounded sigmoid; approximate logits: the fp32 formula (its error, about 1e-7,
@@ -254,7 +264,7 @@ route_select_row(const float* __restrict__ partials, int n_chunks, const float* 
         float sg = (cert.tau > 0.0f) ? __fdividef(1.0f, 1.0f + __expf(-s[e]))
                                      : (float)(1.0 / (1.0 + exp(-(double)s[e])));
         s[e] = sg;
-        c[e] = __fadd_rn(sg, bias ? bias[e] : 0.0f);
+        c[e] = rankable(__fadd_rn(sg, bias ? bias[e] : 0.0f));
     }
     __syncwarp();
     const int gs = E / n_group;
@@ -270,7 +280,7 @@ route_select_row(const float* __restrict__ partials, int n_chunks, const float* 
             for (int j = lane; j < gs; j += 32)
                 if (j != b1.i) b2 = better(b2, ValIdx{c[g * gs + j], j});
             b2 = warp_argmax(b2);
-            sc = __fadd_rn(b1.v, b2.v);
+            sc = rankable(__fadd_rn(b1.v, b2.v));
         }
         if (lane == g) my_gscore = sc;
     }
@@ -387,7 +397,8 @@ route_select_row_regs(const float* __restrict__ partials, int n_chunks, const fl
         for (int j = 0; j < PER; j++) ss = fmaf(lg[j], lg[j], ss);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        tau *= fmaxf(1.0f, sqrtf(ss / (float)E));
+        const float rms = sqrtf(ss / (float)E);
+        if (!(rms <= 1.0f)) tau *= rms;          // a NaN logit makes the threshold NaN: the exact pass decides
     }
     float sg[PER], c[PER];
 #pragma unroll
@@ -396,6 +407,8 @@ route_select_row_regs(const float* __restrict__ partials, int n_chunks, const fl
                                   : (float)(1.0 / (1.0 + exp(-(double)lg[j])));
         c[j] = __fadd_rn(sg[j], bias ? bias[e_lo + j] : 0.0f);
     }
+#pragma unroll
+    for (int j = 0; j < PER; j++) c[j] = rankable(c[j]);
     // ---- group scores: best two selection scores of every group ----
     const int gs = E / n_group, lpg = gs / PER, g = lane / lpg;
     ValIdx b1 = {0.0f, -1}, b2 = {0.0f, -1};
@@ -414,7 +427,7 @@ route_select_row_regs(const float* __restrict__ partials, int n_chunks, const fl
         b2 = (top.i == b1.i) ? better(b2, o1) : better(b1, o2);
         b1 = top;
     }
-    const float gscore = (gs > 1) ? __fadd_rn(b1.v, b2.v) : b1.v;
+    const float gscore = (gs > 1) ? rankable(__fadd_rn(b1.v, b2.v)) : b1.v;
     // ---- kept groups: group g stays if fewer than topk_group groups beat it (ties: the lower group wins) ----
     int beaten_by = 0;
     for (int h = 0; h < n_group; h++) {

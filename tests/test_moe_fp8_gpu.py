@@ -379,3 +379,42 @@ def test_row_groups_of_the_token_tiles(b200, cuda, counts, packed, pow2):
         got = out.cpu().numpy()
         assert np.isfinite(got).all()
         assert not (np.abs(got[rows] - ref) > ATOL + RTOL * np.abs(ref)).any()
+
+
+@pytest.mark.parametrize("T,E,K", [(5, 256, 8), (5, 40, 4), (300, 256, 8), (300, 48, 4)])
+@pytest.mark.parametrize("what", ["bias", "gate row", "token"])
+def test_nan_scores_are_never_preferred(b200, cuda, T, E, K, what):
+    """Grouped selection with NaN among the scores, both selection kernels, exact and certified logits: a NaN score ranks
+    like -inf, so the other experts are chosen as if that expert had a bias of -inf; a token whose scores are all NaN still
+    gets K different experts, and its weights are NaN."""
+    rng = np.random.default_rng(E + T)
+    D = 1024
+    x = rng.normal(0, 1, (T, D)).astype(np.float32)
+    wg = rng.normal(0, D ** -0.5, (E, D)).astype(np.float32)
+    bias = rng.normal(0, 0.01, E).astype(np.float32)
+    xq, xs = oracle.quant_act(x)
+    poisoned = [0, 5, 8, 17, E - 1]                     # first and later experts of a lane's run
+    as_if = bias.copy()
+    if what != "token":
+        as_if[poisoned] = -np.inf
+    ref_ids, ref_w = oracle.route_grouped(xq, xs, wg, as_if, K, 4, 2, 2.5)
+    xs = xs.copy()
+    if what == "bias":
+        bias[poisoned] = np.nan
+    elif what == "gate row":
+        wg[poisoned, 7] = np.nan
+    else:
+        xs[2, 1] = np.nan
+    cfg = b200.MoeFp8Config(T, E, K, D, 128, b200.SCORE_SIGMOID_GROUPED, 4, 2, 2.5)
+    ids = torch.empty((T, K), dtype=torch.int32, device=cuda)
+    wts = torch.empty((T, K), dtype=torch.float32, device=cuda)
+    b200.moe_route_fp8(_dev(xq, cuda), _dev(xs, cuda), _dev(wg, cuda), _dev(bias, cuda), ids, wts, cfg)
+    ids, wts = ids.cpu().numpy(), wts.cpu().numpy()
+    ok = np.ones(T, bool)
+    if what == "token":
+        ok[2] = False
+        assert len(set(ids[2].tolist())) == K and ids[2].min() >= 0 and ids[2].max() < E
+        assert np.isnan(wts[2]).all()
+    assert np.array_equal(ids[ok], ref_ids[ok])
+    # the certified logits of 256 tokens and more carry the tensor cores' error: the bound of the router's own tests
+    assert np.abs(wts[ok] - ref_w[ok]).max() <= (5e-7 if T < 256 else 2e-5)
