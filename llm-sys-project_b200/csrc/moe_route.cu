@@ -570,8 +570,8 @@ pair_histogram_kernel(const int* __restrict__ ids, int TK, int K, int E, int* __
 constexpr int PERMUTE_THREADS = 1024;
 template <bool CHECK_DUP>
 __global__ void __launch_bounds__(PERMUTE_THREADS)
-permute_kernel(const int* __restrict__ ids, int TK, int K, int E, const int* __restrict__ counts_in,
-               int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ row_pair) {
+permute_kernel(const int* __restrict__ ids, int TK, int K, int E, const int* __restrict__ counts, int* __restrict__ offsets,
+               int* __restrict__ row_pair) {
     ptx::grid_wait();
     ptx::grid_release();
     constexpr int NW = PERMUTE_THREADS / 32;
@@ -585,7 +585,7 @@ permute_kernel(const int* __restrict__ ids, int TK, int K, int E, const int* __r
         return true;
     };
     int lt = 0;
-    for (int i = threadIdx.x; i < e; i += PERMUTE_THREADS) lt += counts_in[i];
+    for (int i = threadIdx.x; i < e; i += PERMUTE_THREADS) lt += counts[i];
     for (int o = 16; o > 0; o >>= 1) lt += __shfl_xor_sync(0xffffffffu, lt, o);
     if (lane == 0) warp_sums[warp] = lt;
     __syncthreads();
@@ -637,7 +637,6 @@ permute_kernel(const int* __restrict__ ids, int TK, int K, int E, const int* __r
         running += total;
     }
     if (threadIdx.x == 0) {
-        counts[e] = running;
         offsets[e] = base;
         if (e == E - 1) offsets[E] = base + running;
     }
@@ -1183,9 +1182,8 @@ int launch_permute(const int* ids, int T, int K, int E, bool trusted, int* count
     else         pair_histogram_kernel<true><<<blocks, 256, sizeof(int) * (size_t)E, stream>>>(ids, TK, K, E, counts);
     b200_count_launch(1);
     B200_CUDA_TRY(cudaGetLastError());
-    // (each block rewrites its own entry of counts with the same value at the end)
     const cudaError_t err = b200_launch_after(trusted ? permute_kernel<false> : permute_kernel<true>, dim3(E), PERMUTE_THREADS, 0, stream,
-                                              ids, TK, K, E, counts, counts, offsets, row_pair);
+                                              ids, TK, K, E, counts, offsets, row_pair);
     b200_count_launch(1);
     B200_CUDA_TRY(err);
     B200_CUDA_TRY(cudaGetLastError());
