@@ -133,10 +133,11 @@ grouped_gemm_f32_kernel(const float* __restrict__ a_src,     // MODE 1: x [T,D];
 //     per thread the T = 128 case below took 68 us;
 //   * where the tiles do not fill the machine the reduction is split over a cluster of up to four CTAs and added in
 //     rank order through distributed shared memory, so an output still receives one addition per (token, expert).
-// T = 32, E = 8, K = 2, D = 128, I = 256: 66 -> 16 us a call; T = 128, E = 16, K = 2, D = 512, I = 1024: 355 -> 68 us
-// (100 MB of weights); error against 64-bit arithmetic 9.2e-7 -> 5.2e-7.
+// T = 32, E = 8, K = 2, D = 128, I = 256: 67 -> 15 us a call; T = 128, E = 16, K = 2, D = 512, I = 1024: 350 -> 65 us
+// (100 MB of weights); error against 64-bit arithmetic 9.2e-7 -> 5.0e-7.
 // ---------------------------------------------------------------------------------------------
-constexpr int GV_KT = 64, GV_LD = GV_KT + 4, GV_ST = 4, GV_N = 64, GV_THREADS = 256, GV_PAIRS = 2048;
+constexpr int GV_KT = 64, GV_LD = GV_KT + 4, GV_ST = 4, GV_N = 64, GV_THREADS = 256, GV_PAIRS = 2048, GV_IDS = GV_PAIRS / GV_THREADS;
+constexpr int GV_MAXE = 4096;                                 // experts
 constexpr int GV_W = GV_THREADS / 32, GV_RLD = GV_N + 8;      // warps; row stride of the warps' sums
 
 __device__ __forceinline__ void gv_cp16(float* dst, const float* src, bool ok) {
@@ -151,96 +152,216 @@ struct GvParams {
     const int* row_pair;
     const float* wts;        // MODE 2
     float* dst;              // MODE 1: act [rows,I]; MODE 2: out [T,D]
-    int TK, K, D, I;
+    int TK, K, D, I, E;
 };
 
 template <int MT>
 constexpr size_t gv_smem_bytes() { return sizeof(float) * (size_t)GV_ST * (GV_N + MT) * GV_LD; }
 
-// grid: (ceil(N / tile columns), row-tile walkers, E * cluster size); MT rows x 64 weight rows per tile
-template <int MODE, int MT>
+// MT rows x 64 weight rows per tile.  Which rows a block works on:
+//   WALK  grid (ceil(N / tile columns), ny, E * cluster size): block (y, expert) takes the expert's row tiles y, y + ny, ...
+//         and asks for the first one's weights before the routing is known where that tile is likely to exist.
+//   DEAL  the same grid, for batches whose routing can leave an expert many tiles: those beyond its first ny are dealt out,
+//         one each, to the E * ny blocks of the column, first to the ones without a tile (ny * MT is at least the mean row
+//         count, so there are never more of them than blocks).  2048 rows on one of 128 experts (K = 1, D = 256, I = 512):
+//         walked in series 1382 us, dealt out 256 us (347 us in the 32 x 32-tile kernels above, which have a block per
+//         tile that may exist).
+//   LIST  grid (ceil(N / tile columns), walkers, cluster size), long id lists with 32 rows and more per expert: the row
+//         tiles of all experts in one list, taken in turn.  T = 8192, E = 16, K = 2, D = 128, I = 256: 360 us with a block
+//         per tile that may exist, 225 us.
+enum GvRows { WALK, DEAL, LIST };
+template <int MODE, int MT, GvRows ROWS>
 __global__ void __launch_bounds__(GV_THREADS, 2)
 grouped_gemm_f32_vec_kernel(const GvParams p) {
     extern __shared__ __align__(16) float gv_smem[];
     __shared__ int s_pair[GV_PAIRS];
-    __shared__ int s_warp[GV_THREADS / 32];
+    __shared__ int s_scan[2][GV_W], s_rank, s_job[2];
     constexpr int RT = MT / 4;                               // rows per thread
     constexpr int STG = (GV_N + MT) * GV_LD;                 // floats per stage: weights, then activations
     static_assert(GV_W * MT * GV_RLD <= GV_ST * STG, "the warps' sums reuse the ring");
     uint32_t crank, csize;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(crank));
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(csize));
-    const int e = blockIdx.z / csize;
+    const int E = p.E, own = blockIdx.z / csize, y = blockIdx.y, ny = ROWS == LIST ? 0 : gridDim.y;
     const int Kd = (MODE == 1) ? p.D : p.I, N = (MODE == 1) ? p.I : p.D;
     const int n0 = blockIdx.x * ((MODE == 1) ? GV_N / 2 : GV_N);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nkt = (Kd + GV_KT - 1) / GV_KT, per = (nkt + (int)csize - 1) / (int)csize;
     const int kt_b = min(nkt, (int)crank * per), nk = min(nkt, kt_b + per) - kt_b;
 
-    const float* we = p.w + (size_t)e * ((MODE == 1) ? (size_t)2 * p.I * p.D : (size_t)p.D * p.I);
     // this thread's 16-byte pieces of a weight tile: tile rows tid / 16 + 16 i
     const int lr = tid >> 4, lk = (tid & 15) * 4;
     const float* wsrc[4];
     bool wok[4];
+    auto weights_of = [&](int e) {
+        const float* we = p.w + (size_t)e * ((MODE == 1) ? (size_t)2 * p.I * p.D : (size_t)p.D * p.I);
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int c = lr + 16 * i;
-        const int n = (MODE == 1) ? n0 + (c & 31) : n0 + c;
-        wok[i] = n < N;
-        wsrc[i] = we + (size_t)((MODE == 1 && c >= 32) ? p.I + (wok[i] ? n : 0) : (wok[i] ? n : 0)) * Kd;
-    }
+        for (int i = 0; i < 4; i++) {
+            const int c = lr + 16 * i;
+            const int n = (MODE == 1) ? n0 + (c & 31) : n0 + c;
+            wok[i] = n < N;
+            wsrc[i] = we + (size_t)((MODE == 1 && c >= 32) ? p.I + (wok[i] ? n : 0) : (wok[i] ? n : 0)) * Kd;
+        }
+    };
     auto load_w = [&](int j) {                               // k-tile kt_b + j into ring slot j % GV_ST
         const int k = (kt_b + j) * GV_KT + lk;
         float* d = gv_smem + (j % GV_ST) * STG + lr * GV_LD + lk;
 #pragma unroll
         for (int i = 0; i < 4; i++) gv_cp16(d + 16 * i * GV_LD, wsrc[i] + (k < Kd ? k : 0), wok[i] && k < Kd);
     };
-    // the weights do not depend on the kernel in front: the first tiles are requested before waiting for it
-    const bool early = blockIdx.y == 0;
-    if (early)
+    // The weights do not depend on the kernel in front: the first tiles are requested before waiting for it, where the block
+    // is likely to have rows (T = 1, E = 256, K = 8, D = 512, I = 1024: 315 us with all experts' first tiles, 277 us without).
+    bool requested = ROWS != LIST && (y == 0 ? 2 * p.TK > E : y * MT < p.TK / E);
+    weights_of(own);
+    if (requested)
         for (int j = 0; j < GV_ST - 1; j++)
             if (j < nk) load_w(j);
+    // counts of all experts (short id list) in the ring's last slot, which nothing is on its way to before the main loop
+    int* const hist = reinterpret_cast<int*>(gv_smem + (GV_ST - 1) * STG);
+    static_assert(STG >= GV_MAXE, "a count per expert");
+    if (ROWS == DEAL && !p.row_pair)
+        for (int i = tid; i < E; i += GV_THREADS) hist[i] = 0;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    // rows of this expert (ascending pairs) and, for the sorted position, the rows of lower experts
+    // A short id list: thread = one pair, or GV_IDS consecutive ones.
+    static_assert(GV_IDS * GV_THREADS == GV_PAIRS, "the whole list");
+    const bool many = p.TK > GV_THREADS;
+    const int pair0 = many ? tid * GV_IDS : tid;
+    int id[GV_IDS];
+    auto load_ids = [&]() {
+#pragma unroll
+        for (int i = 0; i < GV_IDS; i++) {
+            if (i > 0 && !many) break;
+            id[i] = (pair0 + i < p.TK) ? p.ids[pair0 + i] : -1;
+        }
+    };
+    // Rows of an expert (ascending pairs) and, for the sorted position, the rows of lower experts
     int cnt = 0, base = 0;
     const int* rows = s_pair;
-    if (p.row_pair) {
-        base = p.offsets[e];
-        cnt = p.offsets[e + 1] - base;
-        rows = p.row_pair + base;
-    } else {
-        int lower = 0;
-        for (int p0 = 0; p0 < p.TK; p0 += GV_THREADS) {
-            const int id = (p0 + tid < p.TK) ? p.ids[p0 + tid] : -1;
-            const unsigned hit = __ballot_sync(0xffffffffu, id == e);
-            lower += (id >= 0 && id < e) ? 1 : 0;
-            if (lane == 0) s_warp[warp] = __popc(hit);
-            __syncthreads();
-            int before = 0, total = 0;
+    auto list_rows = [&](int e) {
+        if (ROWS == LIST || p.row_pair) {
+            base = p.offsets[e];
+            cnt = p.offsets[e + 1] - base;
+            rows = p.row_pair + base;
+            return;
+        }
+        int c = 0, lower = 0;
 #pragma unroll
-            for (int w = 0; w < GV_THREADS / 32; w++) {
-                const int n = s_warp[w];
-                before += (w < warp) ? n : 0;
-                total += n;
-            }
-            if (id == e) s_pair[cnt + before + __popc(hit & ((1u << lane) - 1))] = p0 + tid;
-            cnt += total;
-            __syncthreads();
+        for (int i = 0; i < GV_IDS; i++) {
+            if (i > 0 && !many) break;
+            c += id[i] == e ? 1 : 0;
+            lower += id[i] >= 0 && id[i] < e ? 1 : 0;
+        }
+        int at = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int n = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= o) at += n;
+        }
+        lower = __reduce_add_sync(0xffffffffu, lower);
+        if (lane == 31) { s_scan[0][warp] = at; s_scan[1][warp] = lower; }
+        __syncthreads();
+        at -= c;
+        cnt = base = 0;
+#pragma unroll
+        for (int w = 0; w < GV_W; w++) {
+            at += w < warp ? s_scan[0][w] : 0;
+            cnt += s_scan[0][w];
+            base += s_scan[1][w];
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) lower += __shfl_xor_sync(0xffffffffu, lower, o);
-        if (lane == 0) s_warp[warp] = lower;
-        __syncthreads();
+        for (int i = 0; i < GV_IDS; i++) {
+            if (i > 0 && !many) break;
+            if (id[i] == e) s_pair[at++] = pair0 + i;
+        }
+        // (a barrier of the caller's makes the list visible)
+    };
+    auto tiles_of = [&](int e) { return ((ROWS == LIST || p.row_pair ? p.offsets[e + 1] - p.offsets[e] : hist[e]) + MT - 1) / MT; };
+    // DEAL, LIST: the row tiles beyond each expert's first ny (LIST: all), numbered in order of (expert, tile); thread = a run of
+    // experts.  idle: blocks without a tile of their own.
+    const int run = (E + GV_THREADS - 1) / GV_THREADS, e_lo = min(E, tid * run), e_hi = min(E, e_lo + run);
+    int mine = 0, before = 0, idle_before = 0, all = 0, idle_all = 0;
+    auto number_tiles = [&]() {
+        int idle = 0;
+        for (int e = e_lo; e < e_hi; e++) {
+            const int t = tiles_of(e);
+            mine += max(0, t - ny);
+            idle += max(0, ny - t);
+        }
+        before = mine; idle_before = idle;
 #pragma unroll
-        for (int w = 0; w < GV_THREADS / 32; w++) base += s_warp[w];
+        for (int o = 1; o < 32; o <<= 1) {
+            const int a = __shfl_up_sync(0xffffffffu, before, o), b = __shfl_up_sync(0xffffffffu, idle_before, o);
+            if (lane >= o) { before += a; idle_before += b; }
+        }
+        if (lane == 31) { s_scan[0][warp] = before; s_scan[1][warp] = idle_before; }
+        __syncthreads();
+        before -= mine; idle_before -= idle;
+#pragma unroll
+        for (int w = 0; w < GV_W; w++) {
+            const int a = s_scan[0][w], b = s_scan[1][w];
+            if (w < warp) { before += a; idle_before += b; }
+            all += a; idle_all += b;
+        }
+    };
+    auto find_tile = [&](int n) {                            // s_job = expert and tile of number n
+        if (n >= before && n < before + mine) {
+            int left = n - before;
+            for (int e = e_lo; e < e_hi; e++) {
+                const int x = max(0, tiles_of(e) - ny);
+                if (left < x) { s_job[0] = e; s_job[1] = ny + left; break; }
+                left -= x;
+            }
+        }
+        __syncthreads();
+    };
+
+    int m0 = y * MT, next = y;                               // the block's tile: rows m0 .. m0 + MT - 1 of the list
+    bool more = false;
+    if (ROWS == LIST) {
+        number_tiles();
+        if (next >= all) return;
+        find_tile(next);
+        weights_of(s_job[0]);
+        list_rows(s_job[0]);
+        m0 = s_job[1] * MT;
+        __syncthreads();
+    } else {
+        if (!p.row_pair) load_ids();
+        list_rows(own);
+        bool over = false;                                   // any expert with more than ny tiles
+        if (ROWS == DEAL) {
+            if (!p.row_pair) {                               // (list_rows' barrier lies between clearing and counting)
+#pragma unroll
+                for (int i = 0; i < GV_IDS; i++) {
+                    if (i > 0 && !many) break;
+                    if (id[i] >= 0) atomicAdd(&hist[id[i]], 1);
+                }
+                __syncthreads();
+            }
+            for (int i = tid; i < E; i += GV_THREADS) over |= tiles_of(i) > ny;
+        }
+        if (ROWS == WALK) {
+            __syncthreads();
+        } else if (__syncthreads_or(over)) {
+            number_tiles();
+            if (own >= e_lo && own < e_hi) {                 // this block's turn: idle ones first, in order of (expert, y)
+                int b = idle_before;
+                for (int e = e_lo; e < own; e++) b += max(0, ny - tiles_of(e));
+                const int t = min(ny, tiles_of(own));
+                s_rank = y >= t ? b + y - t : idle_all + own * ny - b + y;
+            }
+            __syncthreads();
+            more = s_rank < all;
+            if (more) find_tile(s_rank);
+        }
     }
 
     const int tx = lane & 7, ty = lane >> 3;
     constexpr int AR = (MT + 15) / 16;                       // activation rows per loader thread
-    bool first = early;
-    for (int m0 = blockIdx.y * MT; m0 < cnt; m0 += gridDim.y * MT) {
+    for (;;) {
+        const bool live = m0 < cnt;
         const float* asrc[AR];
 #pragma unroll
         for (int i = 0; i < AR; i++) {
@@ -260,102 +381,120 @@ grouped_gemm_f32_vec_kernel(const GvParams p) {
         };
 #pragma unroll
         for (int j = 0; j < GV_ST - 1; j++) {
-            if (j < nk) {
-                if (!first) load_w(j);
+            if (live && j < nk) {
+                if (!requested) load_w(j);
                 load_a(j);
             }
-            ptx::cp_async_commit();
+            ptx::cp_async_commit();                          // (early weights of an expert without rows are in a group too)
         }
-        first = false;
-        float acc[RT][8];
+        requested = false;
+        if (live) {
+            float acc[RT][8];
 #pragma unroll
-        for (int i = 0; i < RT; i++)
+            for (int i = 0; i < RT; i++)
 #pragma unroll
-            for (int j = 0; j < 8; j++) acc[i][j] = 0.0f;
-        for (int j = 0; j < nk; j++) {
-            ptx::cp_async_wait<GV_ST - 2>();
-            __syncthreads();
-            const float* sb = gv_smem + (j % GV_ST) * STG;
-            const float* sa = sb + GV_N * GV_LD;
+                for (int j = 0; j < 8; j++) acc[i][j] = 0.0f;
+            for (int j = 0; j < nk; j++) {
+                ptx::cp_async_wait<GV_ST - 2>();
+                __syncthreads();
+                const float* sb = gv_smem + (j % GV_ST) * STG;
+                const float* sa = sb + GV_N * GV_LD;
 #pragma unroll
-            for (int h = 0; h < GV_KT / 4 / GV_W; h++) {
-                const int k = (warp + GV_W * h) * 4;
-                float4 b[8];
+                for (int h = 0; h < GV_KT / 4 / GV_W; h++) {
+                    const int k = (warp + GV_W * h) * 4;
+                    float4 b[8];
 #pragma unroll
-                for (int c = 0; c < 8; c++) b[c] = *reinterpret_cast<const float4*>(sb + (tx + 8 * c) * GV_LD + k);
+                    for (int c = 0; c < 8; c++) b[c] = *reinterpret_cast<const float4*>(sb + (tx + 8 * c) * GV_LD + k);
 #pragma unroll
-                for (int i = 0; i < RT; i++) {
-                    const float4 a = *reinterpret_cast<const float4*>(sa + (ty + 4 * i) * GV_LD + k);
+                    for (int i = 0; i < RT; i++) {
+                        const float4 a = *reinterpret_cast<const float4*>(sa + (ty + 4 * i) * GV_LD + k);
 #pragma unroll
-                    for (int c = 0; c < 8; c++) {
-                        acc[i][c] = fmaf(a.x, b[c].x, acc[i][c]); acc[i][c] = fmaf(a.y, b[c].y, acc[i][c]);
-                        acc[i][c] = fmaf(a.z, b[c].z, acc[i][c]); acc[i][c] = fmaf(a.w, b[c].w, acc[i][c]);
+                        for (int c = 0; c < 8; c++) {
+                            acc[i][c] = fmaf(a.x, b[c].x, acc[i][c]); acc[i][c] = fmaf(a.y, b[c].y, acc[i][c]);
+                            acc[i][c] = fmaf(a.z, b[c].z, acc[i][c]); acc[i][c] = fmaf(a.w, b[c].w, acc[i][c]);
+                        }
                     }
                 }
+                if (j + GV_ST - 1 < nk) { load_w(j + GV_ST - 1); load_a(j + GV_ST - 1); }
+                ptx::cp_async_commit();
             }
-            if (j + GV_ST - 1 < nk) { load_w(j + GV_ST - 1); load_a(j + GV_ST - 1); }
-            ptx::cp_async_commit();
+            ptx::cp_async_wait<0>();
+            __syncthreads();                                     // the ring is free: sums [warp][row][column]
+#pragma unroll
+            for (int i = 0; i < RT; i++)
+#pragma unroll
+                for (int c = 0; c < 8; c++) gv_smem[(warp * MT + ty + 4 * i) * GV_RLD + tx + 8 * c] = acc[i][c];
+            __syncthreads();
+            // add the warps' sums in place; thread = 4 consecutive columns
+            for (int o = tid; o < MT * GV_N / 4; o += GV_THREADS) {
+                float* q = gv_smem + (o >> 4) * GV_RLD + 4 * (o & 15);
+                float4 s = *reinterpret_cast<const float4*>(q);
+#pragma unroll
+                for (int g = 1; g < GV_W; g++) {
+                    const float4 v = *reinterpret_cast<const float4*>(q + g * MT * GV_RLD);
+                    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+                }
+                *reinterpret_cast<float4*>(q) = s;
+            }
+            if (csize > 1) cluster_sync(); else __syncthreads();
+            auto total4 = [&](int m, int c4) -> float4 {         // the CTAs of the cluster in rank order
+                const float* q = gv_smem + m * GV_RLD + 4 * c4;
+                if (csize == 1) return *reinterpret_cast<const float4*>(q);
+                float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+                for (uint32_t r = 0; r < csize; r++) {
+                    const float4 v = cluster_ld_f32x4(cluster_map(q, r));
+                    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+                }
+                return s;
+            };
+            if (MODE == 1) {
+                for (int o = (int)crank * GV_THREADS + tid; o < MT * GV_N / 8; o += (int)csize * GV_THREADS) {
+                    const int m = o >> 3, c4 = o & 7;            // row, 4 activation columns: gate at 4 c4, up 32 further
+                    if (m0 + m >= cnt || n0 + 4 * c4 >= N) continue;
+                    const float4 g = total4(m, c4), u = total4(m, 8 + c4);
+                    float4 r;
+                    r.x = __fdiv_rn(g.x, 1.0f + expf(-g.x)) * u.x;   // silu as naive_moe.cu:308
+                    r.y = __fdiv_rn(g.y, 1.0f + expf(-g.y)) * u.y;
+                    r.z = __fdiv_rn(g.z, 1.0f + expf(-g.z)) * u.z;
+                    r.w = __fdiv_rn(g.w, 1.0f + expf(-g.w)) * u.w;
+                    *reinterpret_cast<float4*>(p.dst + (size_t)(base + m0 + m) * p.I + n0 + 4 * c4) = r;
+                }
+            } else {
+                for (int o = (int)crank * GV_THREADS + tid; o < MT * GV_N / 4; o += (int)csize * GV_THREADS) {
+                    const int m = o >> 4, c4 = o & 15;
+                    if (m0 + m >= cnt || n0 + 4 * c4 >= N) continue;
+                    const float4 s = total4(m, c4);
+                    const int pair = rows[m0 + m];
+                    const float wv = p.wts[pair];
+                    float* d = p.dst + (size_t)(pair / p.K) * p.D + n0 + 4 * c4;
+                    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(d), "f"(wv * s.x), "f"(wv * s.y), "f"(wv * s.z), "f"(wv * s.w)
+                                 : "memory");
+                }
+            }
+            // the ring is refilled (and the CTA may leave) only when nobody reads the sums any more
+            if (csize > 1) cluster_sync(); else __syncthreads();
         }
+        // nothing may be on its way into this block's shared memory when the ring is used again or the block leaves
         ptx::cp_async_wait<0>();
-        __syncthreads();                                     // the ring is free: sums [warp][row][column]
-#pragma unroll
-        for (int i = 0; i < RT; i++)
-#pragma unroll
-            for (int c = 0; c < 8; c++) gv_smem[(warp * MT + ty + 4 * i) * GV_RLD + tx + 8 * c] = acc[i][c];
-        __syncthreads();
-        // add the warps' sums in place; thread = 4 consecutive columns
-        for (int o = tid; o < MT * GV_N / 4; o += GV_THREADS) {
-            float* q = gv_smem + (o >> 4) * GV_RLD + 4 * (o & 15);
-            float4 s = *reinterpret_cast<const float4*>(q);
-#pragma unroll
-            for (int g = 1; g < GV_W; g++) {
-                const float4 v = *reinterpret_cast<const float4*>(q + g * MT * GV_RLD);
-                s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-            }
-            *reinterpret_cast<float4*>(q) = s;
+        if (ROWS == WALK) {
+            m0 += ny * MT;
+            if (m0 >= cnt) return;
+            continue;
         }
-        if (csize > 1) cluster_sync(); else __syncthreads();
-        auto total4 = [&](int m, int c4) -> float4 {         // the CTAs of the cluster in rank order
-            const float* q = gv_smem + m * GV_RLD + 4 * c4;
-            if (csize == 1) return *reinterpret_cast<const float4*>(q);
-            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (uint32_t r = 0; r < csize; r++) {
-                const float4 v = cluster_ld_f32x4(cluster_map(q, r));
-                s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-            }
-            return s;
-        };
-        if (MODE == 1) {
-            for (int o = (int)crank * GV_THREADS + tid; o < MT * GV_N / 8; o += (int)csize * GV_THREADS) {
-                const int m = o >> 3, c4 = o & 7;            // row, 4 activation columns: gate at 4 c4, up 32 further
-                if (m0 + m >= cnt || n0 + 4 * c4 >= N) continue;
-                const float4 g = total4(m, c4), u = total4(m, 8 + c4);
-                float4 r;
-                r.x = __fdiv_rn(g.x, 1.0f + expf(-g.x)) * u.x;   // silu as naive_moe.cu:308
-                r.y = __fdiv_rn(g.y, 1.0f + expf(-g.y)) * u.y;
-                r.z = __fdiv_rn(g.z, 1.0f + expf(-g.z)) * u.z;
-                r.w = __fdiv_rn(g.w, 1.0f + expf(-g.w)) * u.w;
-                *reinterpret_cast<float4*>(p.dst + (size_t)(base + m0 + m) * p.I + n0 + 4 * c4) = r;
-            }
-        } else {
-            for (int o = (int)crank * GV_THREADS + tid; o < MT * GV_N / 4; o += (int)csize * GV_THREADS) {
-                const int m = o >> 4, c4 = o & 15;
-                if (m0 + m >= cnt || n0 + 4 * c4 >= N) continue;
-                const float4 s = total4(m, c4);
-                const int pair = rows[m0 + m];
-                const float wv = p.wts[pair];
-                float* d = p.dst + (size_t)(pair / p.K) * p.D + n0 + 4 * c4;
-                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(d), "f"(wv * s.x), "f"(wv * s.y), "f"(wv * s.z), "f"(wv * s.w)
-                             : "memory");
-            }
+        if (ROWS == LIST) {
+            next += gridDim.y;
+            more = next < all;
         }
-        // the ring is refilled (and the CTA may leave) only when nobody reads the sums any more
-        if (csize > 1) cluster_sync(); else __syncthreads();
+        if (!more) return;
+        more = false;
+        __syncthreads();                                     // all threads' copies are over, s_job and the row list have been read
+        if (ROWS == LIST) find_tile(next);
+        weights_of(s_job[0]);
+        if (ROWS == DEAL && !p.row_pair) load_ids();
+        list_rows(s_job[0]);
+        m0 = s_job[1] * MT;
+        __syncthreads();                                     // the list is there, s_job has been read
     }
-    // An expert without rows never entered the loop: its early tiles belong to no group yet, and nothing may be on its way
-    // into this block's shared memory when the block leaves.
-    ptx::cp_async_commit();
-    ptx::cp_async_wait<0>();
 }
 
 // Router of the vector path: block = 8 tokens x all (at most 32) experts, thread = one (token, expert) chain in the
@@ -530,22 +669,22 @@ __global__ void scatter_f32_kernel(const float* __restrict__ expert_out, const i
 }
 
 // one grouped GEMM launch of the vector path
-template <int MODE, int MT>
-static int launch_gemm_vec(const GvParams& p, int T, int E, int sm_count, cudaStream_t stream) {
+template <int MODE, int MT, GvRows ROWS>
+static int launch_gemm_vec(const GvParams& p, int ny, int sm_count, cudaStream_t stream) {
     static B200PerDeviceOnce once;
-    const int st = b200_allow_smem(once, grouped_gemm_f32_vec_kernel<MODE, MT>, gv_smem_bytes<MT>());
+    const int st = b200_allow_smem(once, grouped_gemm_f32_vec_kernel<MODE, MT, ROWS>, gv_smem_bytes<MT>());
     if (st) return st;
     const int Kd = (MODE == 1) ? p.D : p.I, N = (MODE == 1) ? p.I : p.D;
     const int nx = ceil_div(N, (MODE == 1) ? GV_N / 2 : GV_N);
-    // walkers over an expert's row tiles: one where the tile was chosen to hold the expert, else the mean and a half (a
-    // block loops over the tiles beyond)
-    const int ny = MT < 32 ? 1 : max(1, min(ceil_div(T, MT), ceil_div(3 * (p.TK / E + 1), 2 * MT)));
+    // the list's TK / 32 + E tiles at most are walked by eight rounds of resident blocks (two per SM) or fewer
+    if (ROWS == LIST) ny = (int)min((long long)p.TK / MT + p.E, (long long)max(1, 16 * sm_count / nx));
+    const int nz = ROWS == LIST ? 1 : p.E;
     // cluster over k: until there are about two blocks per SM (what fits at a time)
     const int nkt = ceil_div(Kd, GV_KT);
     int cs = 1;
-    while (cs < 4 && (long long)nx * E * cs * 2 <= 2ll * sm_count && nkt >= 2 * cs) cs *= 2;
+    while (cs < 4 && (long long)nx * (ROWS == LIST ? ny : p.E) * cs * 2 <= 2ll * sm_count && nkt >= 2 * cs) cs *= 2;
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(nx, ny, E * cs);
+    lc.gridDim = dim3(nx, ny, nz * cs);
     lc.blockDim = dim3(GV_THREADS);
     lc.dynamicSmemBytes = gv_smem_bytes<MT>();
     lc.stream = stream;
@@ -555,7 +694,7 @@ static int launch_gemm_vec(const GvParams& p, int T, int E, int sm_count, cudaSt
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = attr; lc.numAttrs = 2;
-    B200_CUDA_TRY(cudaLaunchKernelEx(&lc, grouped_gemm_f32_vec_kernel<MODE, MT>, p));
+    B200_CUDA_TRY(cudaLaunchKernelEx(&lc, grouped_gemm_f32_vec_kernel<MODE, MT, ROWS>, p));
     b200_count_launch(1);
     B200_CUDA_TRY(cudaGetLastError());
     return B200_OK;
@@ -618,7 +757,7 @@ int b200_moe_forward_f32(b200_ws* ws, const float* x, const float* gate_w, const
     }
     if (vec) {
         GvParams p{};
-        p.ids = ids; p.wts = wts; p.TK = T * K; p.K = K; p.D = D; p.I = I;
+        p.ids = ids; p.wts = wts; p.TK = T * K; p.K = K; p.D = D; p.I = I; p.E = E;
         if (!short_ids) { p.offsets = offsets; p.row_pair = row_pair; }
         // Row tiles of 8 .. 32: the smallest that holds the mean row count and twice its spread (binomial: at most
         // sqrt(mean)), because a second tile streams the weights again and an empty row costs as much as a full one.
@@ -626,10 +765,22 @@ int b200_moe_forward_f32(b200_ws* ws, const float* x, const float* gate_w, const
         const int fit = min(T, (int)(mean + 2.0f * sqrtf(mean) + 0.999f));
         auto gemm = [&](auto mode) -> int {
             constexpr int M = decltype(mode)::value;
-            if (fit <= 8) return launch_gemm_vec<M, 8>(p, T, E, ws->sm_count, stream);
-            if (fit <= 16) return launch_gemm_vec<M, 16>(p, T, E, ws->sm_count, stream);
-            if (fit <= 24) return launch_gemm_vec<M, 24>(p, T, E, ws->sm_count, stream);
-            return launch_gemm_vec<M, 32>(p, T, E, ws->sm_count, stream);
+            auto own_blocks = [&](auto rows) -> int {
+                constexpr int MT = decltype(rows)::value;
+                // blocks per expert: one where the tile was chosen to hold the expert, else for the mean and a half
+                const int ny = MT < 32 ? 1 : max(1, min(ceil_div(T, MT), ceil_div(3 * (p.TK / E + 1), 2 * MT)));
+                // Knowing the other experts' counts costs a block 0.4 us (T = 32, E = 8, D = 128: 12.4 -> 13.2 us a call), so
+                // tiles are dealt out where an expert could otherwise have more than four in series (T = 128, E = 16,
+                // K = 2, D = 512, I = 1024: 69.6 -> 64.9 us), with 32 rows more than eight (at six, T = 300, E = 16,
+                // D = 256, I = 512 took 55 us instead of 50).
+                if (T > (MT < 32 ? 4 : 8) * ny * MT) return launch_gemm_vec<M, MT, DEAL>(p, ny, ws->sm_count, stream);
+                return launch_gemm_vec<M, MT, WALK>(p, ny, ws->sm_count, stream);
+            };
+            if (fit <= 8) return own_blocks(std::integral_constant<int, 8>{});
+            if (fit <= 16) return own_blocks(std::integral_constant<int, 16>{});
+            if (fit <= 24) return own_blocks(std::integral_constant<int, 24>{});
+            if (short_ids) return own_blocks(std::integral_constant<int, 32>{});
+            return launch_gemm_vec<M, 32, LIST>(p, 0, ws->sm_count, stream);
         };
         p.a = x; p.w = w1; p.dst = act;
         st = gemm(std::integral_constant<int, 1>{});

@@ -196,3 +196,29 @@ def test_most_experts_without_rows(b200, cuda, T, E, K, D, I):
     torch.cuda.synchronize()
     for out in outs:
         assert np.abs(out.cpu().numpy() - ref).max() < 1e-5 * max(1.0, np.abs(ref).max())
+
+
+@pytest.mark.parametrize("T,E,K,D,I", [
+    (100, 16, 1, 512, 1024), (100, 16, 2, 64, 132), (90, 16, 3, 260, 260),      # an expert's tiles walked by its own block
+    (100, 4, 1, 512, 512),                                                      # ... of a cluster of four, two blocks per expert
+    (600, 300, 1, 128, 64), (200, 60, 2, 68, 36), (1000, 128, 2, 64, 64), (2048, 40, 1, 68, 36),   # dealt out: 8, 16, 24, 32 rows
+    (600, 16, 1, 512, 64), (600, 16, 1, 64, 512),                               # ... to clusters of four in one of the two GEMMs
+    (2500, 300, 1, 20, 36),                                                     # ... from the permuted (long) list
+    (700, 8, 3, 64, 68), (4100, 4, 1, 64, 1024)])                               # one list of all tiles, one and two per block
+@pytest.mark.parametrize("share", [1.0, 0.5])
+def test_uneven_routing(b200, cuda, T, E, K, D, I, share):
+    """All or half of the tokens choose the same K experts, so those experts have more row tiles than blocks of their own.
+    A tile that runs twice or not at all is off by far more than fp32 sums of at most 1024 products."""
+    rng = np.random.default_rng(T + E)
+    x = rng.normal(0, 1, (T, D)).astype(np.float32)
+    wg = rng.normal(0, D ** -0.5, (E, D)).astype(np.float32)
+    hot = rng.permutation(E)[:K]
+    x[:, 0] = np.where(np.arange(T) < share * T, 10.0, 0.0)
+    wg[:, 0] = 0.0
+    wg[hot, 0] = 5.0
+    w1 = rng.normal(0, D ** -0.5, (E, 2 * I, D)).astype(np.float32)
+    w2 = rng.normal(0, I ** -0.5, (E, D, I)).astype(np.float32)
+    ids, wts, ref = oracle.moe_forward_f32(x, wg, w1, w2, K)
+    assert np.bincount(ids.reshape(-1), minlength=E)[hot].min() >= share * T
+    out = _run_forward(b200, cuda, x, wg, w1, w2, K)
+    assert np.abs(out - ref).max() < 1e-5 * max(1.0, np.abs(ref).max())
