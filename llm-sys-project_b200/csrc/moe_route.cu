@@ -971,7 +971,7 @@ gate_logits_fp8_tile_kernel(const uint8_t* __restrict__ xq, const float* __restr
     }
 }
 
-constexpr int GT_MAX_T = 256;
+constexpr int GT_MAX_T = 256, GT_MAX_BLOCKS = 1120;
 static int gate_tile_attr() {
     static B200PerDeviceOnce whole, list;
     const int st = b200_allow_smem(whole, gate_logits_fp8_tile_kernel<false>, GT_SMEM);
@@ -1002,12 +1002,16 @@ int launch_gate_logits(const void* x, const float* xs, const float* wg, float* p
     const bool vec = (D % 16 == 0) && (chunk % 16 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0) &&
                      ((reinterpret_cast<uintptr_t>(wg) & 15) == 0);
     // Small batches: the 64 .. 128-token tiles below would leave most of the SMs idle (T = 128, E = 256, D = 7168: 28
-    // tiles), the 16 x 32 ones give 448 blocks.
-    if (fp8 && T < GT_MAX_T && vec && D % 128 == 0) {
+    // tiles), the 16 x 32 ones give 448 blocks (routing 102 -> 52 us).  Those read a weight row once per 32 tokens and
+    // are no longer ahead where they fill the machine nearly four times over (two blocks per SM): 980 .. 1120 blocks
+    // 1.03 .. 1.06 times as fast, 1176 0.95, 1344 0.90 .. 0.93, 3584 (T = 255, E = 1024) 0.57.  One tile
+    // of tokens reads every weight once in any case.
+    dim3 tiles(ceil_div(E, GT_E), n_chunks, ceil_div(T, GT_T));
+    const bool few = T <= GT_T || (long long)tiles.x * tiles.y * tiles.z <= GT_MAX_BLOCKS;
+    if (fp8 && T < GT_MAX_T && few && vec && D % 128 == 0) {
         const int st = gate_tile_attr();
         if (st) return st;
-        dim3 grid(ceil_div(E, GT_E), n_chunks, ceil_div(T, GT_T));
-        gate_logits_fp8_tile_kernel<false><<<grid, GT_THREADS, GT_SMEM, stream>>>(static_cast<const uint8_t*>(x), xs, wg, partials,
+        gate_logits_fp8_tile_kernel<false><<<tiles, GT_THREADS, GT_SMEM, stream>>>(static_cast<const uint8_t*>(x), xs, wg, partials,
                                                                                 nullptr, nullptr, T, E, D, chunk);
         b200_count_launch(1);
         B200_CUDA_TRY(cudaGetLastError());

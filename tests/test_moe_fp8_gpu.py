@@ -418,3 +418,18 @@ def test_nan_scores_are_never_preferred(b200, cuda, T, E, K, what):
     assert np.array_equal(ids[ok], ref_ids[ok])
     # the certified logits of 256 tokens and more carry the tensor cores' error: the bound of the router's own tests
     assert np.abs(wts[ok] - ref_w[ok]).max() <= (5e-7 if T < 256 else 2e-5)
+
+
+@pytest.mark.parametrize("T,E,D", [(1, 4096, 1024), (32, 2304, 7168), (160, 512, 7168), (192, 512, 7168), (255, 1024, 1152)])
+def test_router_bits_where_the_tiles_end(b200, cuda, T, E, D):
+    """Both sides of the line between the 16 x 32 router tiles and the tuned kernel (1120 blocks, one tile of tokens):
+    the same fixed-order chains, so the oracle's logits bit for bit."""
+    rng = np.random.default_rng(T * 3 + E)
+    xq, xs = oracle.quant_act(rng.normal(0, 1, (T, D)).astype(np.float32))
+    wg = rng.normal(0, D ** -0.5, (E, D)).astype(np.float32)
+    cfg = b200.MoeFp8Config(T, E, 4, D, 128, b200.SCORE_SIGMOID_GROUPED, 4, 2, 2.5)
+    ids = torch.empty((T, 4), dtype=torch.int32, device=cuda)
+    wts = torch.empty((T, 4), dtype=torch.float32, device=cuda)
+    logits = torch.empty((T, E), dtype=torch.float32, device=cuda)
+    b200.moe_route_fp8(_dev(xq, cuda), _dev(xs, cuda), _dev(wg, cuda), None, ids, wts, cfg, logits_out=logits)
+    assert np.array_equal(logits.cpu().numpy(), oracle.gate_logits_fp8(xq, xs, wg))
