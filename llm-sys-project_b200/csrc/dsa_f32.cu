@@ -414,10 +414,17 @@ template <int NG>
 static int launch_dsa_f32_cluster(const float* qn, const float* qp, const float* kc, const float* kp, const float* v,
                                   const int* idx, float* out, const b200_dsa_config* c, int sm_count, cudaStream_t stream) {
     const int head_blocks = ceil_div(c->num_heads, FC_HB), tiles = ceil_div(c->num_selected_kv, FC_TR);
-    // One tile of 32 rows per CTA where the grid has room (latency), up to the portable cluster size; batches that
-    // fill the machine several times over keep their rows in fewer CTAs (less merging).
+    // One tile of 32 rows per CTA, up to the portable cluster size, until the grid has two CTAs per SM (latency); beyond
+    // that a CTA keeps eight tiles or more, and grids of six times that are cut once at most (less merging).
+    // 256 queries x 8 heads, Dc = 512: S = 128 99 us split in four, 66 us not at all; S = 2048 736 us in four, 690 us in
+    // two, 752 us not at all; 512 queries, Dc = 128, S = 2048: 638 us in two, 706 us not at all.
+    const long long ctas = (long long)c->num_queries * head_blocks;
+    auto room = [&](int cs) {
+        return ctas * cs < 2ll * sm_count || (ctas * cs < 6ll * sm_count && tiles >= 16 * cs) ||
+               (ctas < 8ll * sm_count && cs == 1 && tiles >= 32);
+    };
     int cs = 1;
-    while (cs < 8 && cs < tiles && (long long)c->num_queries * head_blocks * cs < 8ll * sm_count) cs *= 2;
+    while (cs < 8 && cs < tiles && room(cs)) cs *= 2;
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(cs, head_blocks, c->num_queries);
     lc.blockDim = dim3(FC_THREADS);
@@ -432,6 +439,28 @@ static int launch_dsa_f32_cluster(const float* qn, const float* qp, const float*
     b200_count_launch(1);
     B200_CUDA_TRY(cudaGetLastError());
     return B200_OK;
+}
+
+// Where the general kernel stays: batches that fill the machine with little work per (query, head).  Its eight heads share
+// one staged tile, the cluster kernel's four fetch their rows themselves and pay for the cluster and the merge.  Measured
+// with H a multiple of 8 (time of the general kernel / time of the cluster kernel; N = 8192; ctas = queries x groups
+// of four heads):
+//   ctas = 512    Dc = 16 0.90 .. 1.0, Dc = 32 from S = 64 on 1.1 and more, Dc = 128 S = 8 0.84, S = 32 1.1 and more
+//   ctas = 1024   Dc = 16 0.66 .. 0.83, Dc = 32 0.69 (S = 8) 0.97 (128) 1.08 (512), Dc = 64 0.71 (8) 0.94 (32) 1.08 (64)
+//   ctas = 4096   Dc = 32 0.42 (8) .. 0.91 (2048), Dc = 64 0.55 (8) 0.95 (64) 1.10 (128), Dc = 128 0.48 (8) 0.82 (32) 1.08
+//                 (64), Dc = 256 0.86 (8) 1.7 (32), Dc = 512 2.4 (8)
+// Heads that leave the general kernel's blocks partly empty shift the line: H = 2, ctas = 2048, Dc = 16 0.56 (8) 0.88 (64)
+// 1.06 (128), Dc = 64 0.86 (8) 1.27 (32), Dc = 128 0.87 (8), Dc = 256 1.2 (1); H = 12, ctas = 1536 Dc = 16 0.50 .. 0.90,
+// Dc = 32 0.94 (64), Dc = 64 0.70 (8), Dc = 128 0.66 (8), above 1 (32).
+static bool dsa_f32_general_pays(const b200_dsa_config* c) {
+    const int H = c->num_heads, Dc = c->head_dim_compressed;
+    const long long ctas = (long long)c->num_queries * ceil_div(H, FC_HB), work = (long long)c->num_selected_kv * Dc;
+    if (Dc > 256 || ctas < 512) return false;
+    if (H <= 4) return ctas >= 2048 && Dc <= 128 && work <= 1024;
+    if (Dc <= 16) return true;
+    if (H >= 9 && H <= 12) return work <= (Dc <= 128 ? 2048 : 1024);
+    if (Dc <= 32) return ctas >= 2048 || work <= 4096;
+    return work <= (Dc <= 128 && ctas >= 2048 ? 4096 : 2048);
 }
 
 extern "C" {
@@ -452,7 +481,7 @@ int b200_dsa_forward_f32(b200_ws* ws, const float* q_nope, const float* q_pe, co
     const uintptr_t all = reinterpret_cast<uintptr_t>(q_nope) | reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(v) |
                           (Dp > 0 ? reinterpret_cast<uintptr_t>(q_pe) | reinterpret_cast<uintptr_t>(kp) : 0);
     if (Dc % 4 == 0 && Dp % 4 == 0 && Dc <= 512 && Dc + Dp <= 640 && (all & 15) == 0 && cfg->num_queries <= 65535 &&
-        cfg->num_heads <= 65535 * FC_HB) {
+        cfg->num_heads <= 65535 * FC_HB && !dsa_f32_general_pays(cfg)) {
         const int ng = ceil_div(Dc + Dp, 128);
         if (ng <= 1) return launch_dsa_f32_cluster<1>(q_nope, q_pe, kc, kp, v, idx, out, cfg, ws->sm_count, stream);
         if (ng <= 2) return launch_dsa_f32_cluster<2>(q_nope, q_pe, kc, kp, v, idx, out, cfg, ws->sm_count, stream);

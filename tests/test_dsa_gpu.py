@@ -289,3 +289,25 @@ def test_f32_kernels_agree_on_special_values(b200, cuda, what, Dc, Dp, S):
         assert (o[zero] == 0).all()
     a, b = (torch.nan_to_num(o, nan=0.0) for o in got)
     assert (a - b).abs().max().item() < 1e-5
+
+
+@pytest.mark.parametrize("Q,H,Dc,Dp,S", [(512, 5, 16, 4, 40), (512, 4, 16, 4, 40), (2048, 2, 16, 4, 64), (2049, 1, 16, 8, 65), (400, 8, 32, 4, 128),
+                                         (400, 8, 32, 4, 129), (1024, 8, 64, 0, 64), (1024, 8, 64, 0, 65), (200, 12, 128, 8, 16),
+                                         (200, 12, 128, 8, 17), (300, 8, 256, 4, 8), (300, 8, 256, 4, 9), (300, 8, 64, 8, 512)])
+def test_f32_both_sides_of_the_kernel_choice(b200, cuda, Q, H, Dc, Dp, S):
+    """Large batches on both sides of the lines between the two fp32 kernels and of the cluster sizes, against 64-bit
+    arithmetic, with empty entries and rows listed twice.  fp32 sums of up to 264 products and 512 rows stay within
+    1e-5 of the result's scale."""
+    g = torch.Generator(device="cpu").manual_seed(Q + S)
+    N = 300
+    qn, qp, kc, kp, v = (torch.randn(s, generator=g).to(cuda) for s in ((Q, H, Dc), (Q, H, Dp), (N, Dc), (N, Dp), (N, Dc)))
+    idx = torch.randint(-3, N, (Q, S), generator=g).to(torch.int32).to(cuda)
+    idx[:, 0] = 7
+    out = torch.full((Q, H, Dc), float("nan"), device=cuda)
+    b200.dsa_forward(qn, qp if Dp else None, kc, kp if Dp else None, v, idx, out, b200.DsaConfig(Q, H, Dc, Dp, S, 64, N))
+    k, q = torch.cat([kc, kp], 1).double(), torch.cat([qn, qp], 2).double()
+    sc = torch.einsum("qhd,nd->qhn", q, k) / (Dc + Dp) ** 0.5
+    sc = torch.gather(sc, 2, idx.clamp(min=0).long()[:, None, :].expand(Q, H, S)).masked_fill((idx < 0)[:, None, :], -float("inf"))
+    p = torch.zeros((Q, H, N), dtype=torch.float64, device=cuda)
+    p.scatter_add_(2, idx.clamp(min=0).long()[:, None, :].expand(Q, H, S).contiguous(), torch.softmax(sc, 2))
+    assert (out.double() - p @ v.double()).abs().max().item() < 1e-5
