@@ -580,7 +580,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS128, 1) dsa_d
         // ===================== gather producers: NKW warps for K rows, NVW warps for V rows =====================
         const int pt = threadIdx.x - 160;
         const int s_begin = t_begin * TKV;
-        // the ids of the first tile are looked up (up to four dependent loads with a block table) behind the copies of Q
         constexpr int RPW = KROWS / NKW;                          // K rows per warp
         const int kw = pt >> 5;                                   // K warp: rows RPW kw .. RPW kw + RPW - 1 of this CTA's 64
         constexpr int VPW = TKV / NVW;                            // V rows per warp
@@ -588,7 +587,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS128, 1) dsa_d
         const int vw = (pt - 32 * NKW) >> 5;                      // V warp: rows vw, vw + NVW, ... of the tile's 128
         const bool k_warp = pt < 32 * NKW;
         const int my = k_warp ? (int)rank * KROWS + RPW * kw + (lane % RPW) : vw + NVW * lane;
-        int id_n = (nt > 0) ? dsa_resolve(p.ix, b, s_begin + my) : -1;
         // Q: this CTA's 64 heads x 72 sixteen-byte chunks; heads >= H are zero
         for (int i = pt; i < HPC * 72; i += NPROD) {
             const int r = i / 72, ch = i - r * 72;
@@ -606,6 +604,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS128, 1) dsa_d
         // while Q is on its way
         __threadfence_block();
         ptx::cp_async_arrive_noinc(&sm->q_full);
+        // the ids of the first tile (up to four dependent loads with a block table) are looked up behind the copies of Q:
+        // in front of them they delayed the whole block (200 queries, H = 128, S = 128: 51.4 instead of 50.1 us)
+        int id_n = (nt > 0) ? dsa_resolve(p.ix, b, s_begin + my) : -1;
 
         // A warp instruction always covers 512 contiguous bytes of one row (DRAM serves such pieces at
         // more than twice the rate of scattered 128-byte ones).  Each lane fetches the ids of the rows
