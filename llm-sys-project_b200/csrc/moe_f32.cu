@@ -736,7 +736,10 @@ int b200_moe_forward_f32(b200_ws* ws, const float* x, const float* gate_w, const
                           reinterpret_cast<uintptr_t>(w2) | reinterpret_cast<uintptr_t>(out);
     const bool vec = D % 4 == 0 && I % 4 == 0 && (all & 15) == 0 && (long long)E * 4 <= 65535;
     const bool short_ids = vec && (long long)T * K <= GV_PAIRS;      // the GEMM blocks list their rows themselves
-    if (vec && E <= GR_MAXE && short_ids) {
+    // (the fused router clears the output while it reads its weights)
+    const uintptr_t o0 = reinterpret_cast<uintptr_t>(out), g0 = reinterpret_cast<uintptr_t>(gate_w);
+    const bool shared = o0 < g0 + sizeof(float) * (size_t)E * D && g0 < o0 + sizeof(float) * (size_t)T * D;
+    if (vec && E <= GR_MAXE && short_ids && !shared) {
         static B200PerDeviceOnce once;
         st = b200_allow_smem(once, gate_select_f32_kernel, gr_smem_bytes(GR_MAXE));
         if (st) return st;

@@ -1273,13 +1273,24 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
               I = cfg->intermediate_dim;
     const long long TK = (long long)T * K;
     const bool det = (cfg->flags & B200_MOE_DETERMINISTIC) != 0 && do_gemm2;
+    // The output is cleared early (the one-launch sort does it on the way), unless it shares memory with something that
+    // the kernels in front of GEMM2 still read.
+    const bool clear = do_gemm2 && !det && zero_out;
+    const size_t out_bytes = sizeof(float) * (size_t)T * D, w1_blocks = (size_t)E * (2 * I / 128) * (D / 128);
+    auto shares = [&](const void* p, size_t n) {
+        const uintptr_t a = reinterpret_cast<uintptr_t>(out), b = reinterpret_cast<uintptr_t>(p);
+        return a < b + n && b < a + out_bytes;
+    };
+    const bool late = clear && (shares(xq, (size_t)T * D) || shares(xs, sizeof(float) * (size_t)T * (D / 128)) ||
+                                shares(ids, sizeof(int) * (size_t)TK) || shares(wts, sizeof(float) * (size_t)TK) ||
+                                shares(w1q, w1_blocks * 128 * 128) || shares(w1s, sizeof(float) * w1_blocks));
     int st = B200_OK;
     if (trusted && TK <= SMALL_PAIRS) {
         B200_CUDA_TRY(b200_launch_after(sort_small_fp8_kernel, dim3((unsigned)TK + 1), 128, 0, stream, xq, xs, ids, wts, (int)TK, E, K, D,
                                         s.offsets, s.sq, s.ss, s.row_tok, s.row_w, det ? s.pair_row : nullptr,
-                                        do_gemm2 && !det && zero_out ? out : nullptr));
+                                        clear && !late ? out : nullptr));
     } else {
-        if (do_gemm2 && !det && zero_out) B200_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(float) * (size_t)T * D, stream));
+        if (clear && !late) B200_CUDA_TRY(cudaMemsetAsync(out, 0, out_bytes, stream));
         st = launch_permute_ranges(ids, T, K, E, trusted, s.range_hist, s.counts, s.offsets, s.row_pair, stream);
         if (st) return st;
         if (det) B200_CUDA_TRY(cudaMemsetAsync(s.pair_row, 0xFF, sizeof(int) * (size_t)TK, stream));
@@ -1405,6 +1416,7 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
         return B200_OK;
     }
     p.out = out;
+    if (late) B200_CUDA_TRY(cudaMemsetAsync(out, 0, out_bytes, stream));
     if (prof) B200_CUDA_TRY(cudaEventRecord(prof->ev[slot][2], stream));
     st = launch(2, ta, ta32, tb, p);
     if (st) return st;

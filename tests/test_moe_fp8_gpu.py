@@ -433,3 +433,39 @@ def test_router_bits_where_the_tiles_end(b200, cuda, T, E, D):
     logits = torch.empty((T, E), dtype=torch.float32, device=cuda)
     b200.moe_route_fp8(_dev(xq, cuda), _dev(xs, cuda), _dev(wg, cuda), None, ids, wts, cfg, logits_out=logits)
     assert np.array_equal(logits.cpu().numpy(), oracle.gate_logits_fp8(xq, xs, wg))
+
+
+@pytest.mark.parametrize("T", [5, 600])
+@pytest.mark.parametrize("entry", ["forward", "experts"])
+def test_output_over_the_inputs(b200, cuda, T, entry):
+    """The output may lie over the activations, their scales and the given routing: nothing in front of GEMM2 finds them
+    cleared (short and long id lists).  Same kernels and routing, so the same sums up to the order of K additions."""
+    rng = np.random.default_rng(T)
+    E, K, D, I = 16, 4, 512, 256
+    x, wg, bias, w1, w2, xq, xs, w1q, w1s, w2q, w2s = _layer(rng, T, E, D, I)
+    ids = np.stack([rng.permutation(E)[:K] for _ in range(T)]).astype(np.int32)
+    wts = rng.uniform(0.5, 1.5, (T, K)).astype(np.float32)
+    d = [_dev(a, cuda) for a in (w1q, w1s, w2q, w2s)]
+    dg, db = _dev(wg, cuda), _dev(bias, cuda)
+    cfg = b200.MoeFp8Config(T, E, K, D, I, b200.SCORE_SIGMOID_GROUPED, 4, 2, 2.5)
+    got = []
+    for over in (False, True):
+        out = torch.full((T, D), float("nan"), dtype=torch.float32, device=cuda)
+        room = (out if over else torch.empty_like(out)).view(-1).view(torch.uint8)
+        at = 0
+        parts = []
+        for a in (xq, xs, ids, wts):
+            t = _dev(a, cuda)
+            n = t.numel() * t.element_size()
+            v = room[at:at + n].view(t.dtype).view(t.shape)
+            v.copy_(t)
+            parts.append(v)
+            at += (n + 255) & ~255
+        if entry == "forward":
+            b200.moe_fp8_forward(parts[0], parts[1], dg, db, *d, out, cfg)
+        else:
+            b200.moe_fp8_experts(*parts, *d, out, cfg)
+        torch.cuda.synchronize()
+        got.append(out.cpu().numpy())
+    assert np.isfinite(got[0]).all()
+    assert np.abs(got[0] - got[1]).max() <= 4 * K * 2.0 ** -24 * np.abs(got[0]).max()
