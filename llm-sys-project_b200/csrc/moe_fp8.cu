@@ -1034,8 +1034,6 @@ done:
 __global__ void __launch_bounds__(256)
 reduce_rows_kernel(const float* __restrict__ rows, const int* __restrict__ pair_row, const int* __restrict__ ids,
                    int K, int D, float* __restrict__ out) {
-    ptx::grid_wait();
-    ptx::grid_release();
     const int t = blockIdx.x;
     __shared__ int order[64];
     if (threadIdx.x == 0) {

@@ -72,7 +72,7 @@ int moe_route_fp8_run(const RouteScratch& rs, const uint8_t* xq, const float* xs
 // skipped.
 int launch_permute(const int* ids, int T, int K, int E, bool trusted, int* counts, int* offsets, int* row_pair,
                    cudaStream_t stream);
-// Same result with scratch of permute_ranges_scratch_ints integers: two launches whose work does not grow with E.
+// Same result with scratch of permute_ranges_scratch_ints integers: two launches that read the ids once each.
 size_t permute_ranges_scratch_ints(int T, int K, int E);
 int launch_permute_ranges(const int* ids, int T, int K, int E, bool trusted, int* range_hist, int* counts, int* offsets,
                           int* row_pair, cudaStream_t stream);

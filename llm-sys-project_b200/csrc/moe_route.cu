@@ -642,13 +642,13 @@ permute_kernel(const int* __restrict__ ids, int TK, int K, int E, const int* __r
     }
 }
 
-// The same permutation for callers with scratch, in two launches whose work does not grow with E: the list is cut
-// into ranges of PR_PAIRS pairs, one block each.  permute_ranges_count_kernel writes a range's rows per expert;
-// permute_ranges_kernel adds the experts' totals and the earlier ranges' rows itself (E x ranges integers) and gives
+// The same permutation for callers with scratch, in two launches that read the list once each instead of once per expert:
+// it is cut into ranges of PR_PAIRS pairs, one block each.  permute_ranges_count_kernel writes a range's rows per
+// expert; permute_ranges_kernel adds the experts' totals and the earlier ranges' rows itself (E x ranges integers per
+// block, so E x ranges^2 over the grid: 131 KB for 131072 ids and 32 experts, 1 GB for 4 million and 256) and gives
 // every pair of its range its row: a warp owns 128 consecutive pairs, equal ids of a 32-pair step find each other by
-// match, and per-warp counters (scanned over the warps) keep the order stable.  The kernel above scans the whole
-// list once per expert: 131072 ids x 32 experts 67 us.  Here 12 us together (a
-// layer of 32 experts and 16384 rows: 2530 -> 2475 us).
+// match, and per-warp counters (32 x E of them, scanned over the warps) keep the order stable.  131072 ids x 32 experts
+// 67 us in the kernel above, 12 us here (a layer of 32 experts and 16384 rows: 2530 -> 2475 us).
 constexpr int PR_PAIRS = 4096, PR_THREADS = 1024;
 static_assert(PR_PAIRS == (PR_THREADS / 32) * 128, "128 pairs per warp");
 

@@ -363,7 +363,12 @@ def test_row_groups_of_the_token_tiles(b200, cuda, counts, packed, pow2):
             b200.moe_fp8_pack_weights(which, d[k], p, E, D, I)
             d[k] = p
         call = b200.moe_fp8_experts_packed
-    rows = np.unique(np.concatenate([np.arange(min(T, 8)), rng.integers(0, T, 24)])).astype(np.int32)
+    # compared with the oracle: the first and last row of every expert and of each of its 32-row groups, and a few more
+    edges = []
+    for e in range(E):
+        p = np.nonzero(ids[:, 0] == e)[0]                     # ascending: the order of the sorted rows
+        edges += [p[j] for j in range(len(p)) if j % 32 in (0, 31) or j == len(p) - 1]
+    rows = np.unique(np.concatenate([np.array(edges), rng.integers(0, T, 24)])).astype(np.int32)
     args = (xq, xs, w1q, w1s, w2q, w2s, ids, wts, rows)
     if pow2:
         with oracle.pow2_scales():
