@@ -114,6 +114,20 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
     return t;
 }
 
+// ---- warp-uniform single-lane instructions ---------------------------------------
+// A tcgen05.mma, tcgen05.commit or TMA instruction takes its descriptors and addresses from uniform registers.  Where one
+// lane of a diverged warp issues it, every operand is computed in vector registers and moved over first (measured in a
+// grouped GEMM: 85 cycles per MMA); a whole warp that walks the loop together and elects a lane for the instruction
+// alone needs 38.  So issuing warps stay together: loop bounds through uniform(), waits through whole_warp().
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+// true only if no lane gave up: the warp leaves a bounded wait as a whole
+__device__ __forceinline__ bool whole_warp(bool ok) { return __all_sync(0xffffffffu, ok); }
+
 // ---- mbarrier -------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(DSA_THREADS, 1) dsa_decode_bf16_kernel(const D
     volatile int* abort_flag = &sm->abort_flag;
 
     const int hv = blockIdx.x, sp = blockIdx.y, b = blockIdx.z;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = ptx::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int nt_total = p.S / TKV;
     const int t_begin = sp * p.tiles_per_split;
     const int t_end = min(nt_total, t_begin + p.tiles_per_split);
@@ -187,46 +187,48 @@ __global__ void __launch_bounds__(DSA_THREADS, 1) dsa_decode_bf16_kernel(const D
         for (int u = max(0, total_units - LAG); u < total_units; u++) ptx::mbar_arrive(bar_of(u));
     } else if (warp == 4) {
         // ===================== MMA issuer =====================
-        if (lane == 0 && nt > 0) {
+        if (nt > 0) {
             constexpr uint32_t idesc_qk = ptx::make_idesc(1, 1, 0, 0, HEADS, TKV);
             constexpr uint32_t idesc_pv = ptx::make_idesc(1, 1, 0, 1, HEADS, DVH);
             const uint32_t q_addr = ptx::smem_u32(sQ), k_addr = ptx::smem_u32(sK), v_addr = ptx::smem_u32(sV),
                            p_addr = ptx::smem_u32(sP);
             auto issue_pv = [&](int i) -> bool {
                 const int vb = i & 1;
-                if (!ptx::mbar_wait(&sm->p_full, (uint32_t)(i & 1), abort_flag)) return false;
-                if (!ptx::mbar_wait(&sm->v_full[vb], (uint32_t)((i >> 1) & 1), abort_flag)) return false;
+                if (!ptx::whole_warp(ptx::mbar_wait(&sm->p_full, (uint32_t)(i & 1), abort_flag))) return false;
+                if (!ptx::whole_warp(ptx::mbar_wait(&sm->v_full[vb], (uint32_t)((i >> 1) & 1), abort_flag))) return false;
                 ptx::tc_fence_after();
+                const uint64_t ad = ptx::make_smem_desc(p_addr, P_CHUNK_BYTES, 128, 0);
+                const uint64_t bd = ptx::make_smem_desc(v_addr + vb * V_BYTES, VCHUNK_BYTES, 1024, 2);
+                if (ptx::elect_one()) {
 #pragma unroll
-                for (int k2 = 0; k2 < 2; k2++) {
-                    uint64_t ad = ptx::make_smem_desc(p_addr + k2 * 2 * P_CHUNK_BYTES, P_CHUNK_BYTES, 128, 0);
-                    uint64_t bd = ptx::make_smem_desc(v_addr + vb * V_BYTES + k2 * 2048, VCHUNK_BYTES, 1024, 2);
-                    ptx::mma_f16(tmem + O_COL, ad, bd, idesc_pv, (i > 0 || k2 > 0) ? 1u : 0u);
+                    for (int k2 = 0; k2 < 2; k2++)
+                        ptx::mma_f16(tmem + O_COL, ad + k2 * (2 * P_CHUNK_BYTES / 16), bd + k2 * (2048 / 16), idesc_pv, (i > 0 || k2 > 0) ? 1u : 0u);
+                    ptx::tc_commit(&sm->v_empty[vb]);
+                    ptx::tc_commit(&sm->p_empty);
                 }
-                ptx::tc_commit(&sm->v_empty[vb]);
-                ptx::tc_commit(&sm->p_empty);
                 return true;
             };
-            if (!ptx::mbar_wait(&sm->q_full, 0, abort_flag)) goto done;
+            if (!ptx::whole_warp(ptx::mbar_wait(&sm->q_full, 0, abort_flag))) goto done;
             for (int j = 0; j < nt; j++) {
                 const int sb = j & 1;
-                if (!ptx::mbar_wait(&sm->s_empty[sb], (uint32_t)(((j >> 1) & 1) ^ 1), abort_flag)) goto done;
+                if (!ptx::whole_warp(ptx::mbar_wait(&sm->s_empty[sb], (uint32_t)(((j >> 1) & 1) ^ 1), abort_flag))) goto done;
                 for (int c = 0; c < KBLK; c++) {
-                    if (!ptx::mbar_wait(&sm->k_full[c], (uint32_t)(j & 1), abort_flag)) goto done;
+                    if (!ptx::whole_warp(ptx::mbar_wait(&sm->k_full[c], (uint32_t)(j & 1), abort_flag))) goto done;
                     ptx::tc_fence_after();
+                    const uint64_t ad = ptx::make_smem_desc(q_addr + c * Q_BLK_BYTES, 16, 1024, 2);
+                    const uint64_t bd = ptx::make_smem_desc(k_addr + c * KSLOT_BYTES, 16, 1024, 2);
+                    if (ptx::elect_one()) {
 #pragma unroll
-                    for (int k4 = 0; k4 < 4; k4++) {
-                        uint64_t ad = ptx::make_smem_desc(q_addr + c * Q_BLK_BYTES + k4 * 32, 16, 1024, 2);
-                        uint64_t bd = ptx::make_smem_desc(k_addr + c * KSLOT_BYTES + k4 * 32, 16, 1024, 2);
-                        ptx::mma_f16(tmem + S_COL + sb * TKV, ad, bd, idesc_qk, (c > 0 || k4 > 0) ? 1u : 0u);
+                        for (int k4 = 0; k4 < 4; k4++)
+                            ptx::mma_f16(tmem + S_COL + sb * TKV, ad + 2 * k4, bd + 2 * k4, idesc_qk, (c > 0 || k4 > 0) ? 1u : 0u);
+                        ptx::tc_commit(&sm->k_empty[c]);
                     }
-                    ptx::tc_commit(&sm->k_empty[c]);
                 }
-                ptx::tc_commit(&sm->s_full[sb]);
+                if (ptx::elect_one()) ptx::tc_commit(&sm->s_full[sb]);
                 if (j > 0 && !issue_pv(j - 1)) goto done;
             }
             if (!issue_pv(nt - 1)) goto done;
-            ptx::tc_commit(&sm->o_done);
+            if (ptx::elect_one()) ptx::tc_commit(&sm->o_done);
         }
     } else {
         // ===================== softmax / correction / epilogue (warps 0-3) =====================

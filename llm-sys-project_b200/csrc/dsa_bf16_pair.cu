@@ -169,9 +169,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) dsa_deco
     Smem* sm = reinterpret_cast<Smem*>(sP + P_BYTES);
     volatile int* abort_flag = &sm->abort_flag;
 
-    const uint32_t rank = cluster_rank();          // 0 = leader
+    const uint32_t rank = (uint32_t)ptx::uniform((int)cluster_rank());          // 0 = leader
     const int sp = blockIdx.y, b = blockIdx.z;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = ptx::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int nt_total = p.S / TKV;
     const int t_begin = sp * p.tiles_per_split;
     const int nt = max(0, min(nt_total, t_begin + p.tiles_per_split) - t_begin);
@@ -301,9 +301,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) dsa_deco
         ptx::cp_async_wait<0>();           // nothing of this thread is in flight when the CTA winds down
     } else if (warp == 4) {
         // ===================== MMA issuer (leader) / barrier relay (peer) =====================
-        // Both threads walk the same sequence of waits.  The peer's thread forwards each completed
-        // local barrier to its twin in the leader; the leader waits for its own barrier and the twin.
-        if (lane == 0 && nt > 0) {
+        // Both warps walk the same sequence of waits.  The peer's forwards each completed local barrier to its twin in the
+        // leader; the leader waits for its own barrier and the twin.
+        if (nt > 0) {
             const bool leader = (rank == 0);
             constexpr uint32_t idesc_qk = ptx::make_idesc(1, 1, 0, 0, HEADS, TKV);
             constexpr uint32_t idesc_pv = ptx::make_idesc(1, 1, 0, 1, HEADS, 256);
@@ -313,58 +313,56 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) dsa_deco
             // st.shared) and is read by the tensor core through the async proxy: fence after waiting.
             auto forward_or_wait = [&](uint64_t* peer, uint32_t par_peer) -> bool {
                 ptx::fence_proxy_async_smem();
-                if (leader) return mbar_wait_cluster(peer, par_peer, abort_flag);
-                mbar_arrive_cta(peer, 0);
+                if (leader) return ptx::whole_warp(mbar_wait_cluster(peer, par_peer, abort_flag));
+                if (ptx::elect_one()) mbar_arrive_cta(peer, 0);
                 return true;
             };
             auto issue_pv = [&](int i) -> bool {
                 const int st = i & 1;
                 const uint32_t par = (uint32_t)((i >> 1) & 1);
-                if (!ptx::mbar_wait(&sm->p_full, (uint32_t)(i & 1), abort_flag)) return false;
-                if (!ptx::mbar_wait(&sm->v_full[st], par, abort_flag)) return false;
+                if (!ptx::whole_warp(ptx::mbar_wait(&sm->p_full, (uint32_t)(i & 1), abort_flag))) return false;
+                if (!ptx::whole_warp(ptx::mbar_wait(&sm->v_full[st], par, abort_flag))) return false;
                 if (!forward_or_wait(&sm->pv_peer[st], par)) return false;
                 if (!leader) return true;
                 ptx::tc_fence_after();
+                const uint64_t ad = ptx::make_smem_desc(p_addr, P_CHUNK_BYTES, 128, 0), bd = ptx::make_smem_desc(v_addr + st * V_STAGE_BYTES, VCHUNK_BYTES, 1024, 2);
+                if (ptx::elect_one()) {
 #pragma unroll
-                for (int inst = 0; inst < 2; inst++) {
+                    for (int inst = 0; inst < 2; inst++)
 #pragma unroll
-                    for (int ks = 0; ks < 4; ks++) {
-                        uint64_t ad = ptx::make_smem_desc(p_addr + ks * 2 * P_CHUNK_BYTES, P_CHUNK_BYTES, 128, 0);
-                        uint64_t bd = ptx::make_smem_desc(v_addr + st * V_STAGE_BYTES + 2 * inst * VCHUNK_BYTES + ks * 2048,
-                                                          VCHUNK_BYTES, 1024, 2);
-                        mma2_f16(tmem + O_COL + 128 * inst, ad, bd, idesc_pv, (i > 0 || ks > 0) ? 1u : 0u);
-                    }
+                        for (int ks = 0; ks < 4; ks++)
+                            mma2_f16(tmem + O_COL + 128 * inst, ad + ks * (2 * P_CHUNK_BYTES / 16), bd + (2 * inst * VCHUNK_BYTES + ks * 2048) / 16,
+                                     idesc_pv, (i > 0 || ks > 0) ? 1u : 0u);
+                    commit_both(&sm->v_empty[st]);
+                    commit_both(&sm->p_empty);
                 }
-                commit_both(&sm->v_empty[st]);
-                commit_both(&sm->p_empty);
                 return true;
             };
-            if (!ptx::mbar_wait(&sm->q_full, 0, abort_flag)) goto done;
+            if (!ptx::whole_warp(ptx::mbar_wait(&sm->q_full, 0, abort_flag))) goto done;
             for (int j = 0; j < nt; j++) {
                 const int st = j & 1;                           // K stage and S buffer of this tile
                 const uint32_t par = (uint32_t)((j >> 1) & 1);
-                if (!ptx::mbar_wait(&sm->s_empty[st], par ^ 1, abort_flag)) goto done;   // passes at once on first use
-                if (!ptx::mbar_wait(&sm->k_full[st], par, abort_flag)) goto done;
+                if (!ptx::whole_warp(ptx::mbar_wait(&sm->s_empty[st], par ^ 1, abort_flag))) goto done;   // passes at once on first use
+                if (!ptx::whole_warp(ptx::mbar_wait(&sm->k_full[st], par, abort_flag))) goto done;
                 if (!forward_or_wait(&sm->qk_peer[st], par)) goto done;
                 if (leader) {
                     ptx::tc_fence_after();
+                    const uint64_t ad = ptx::make_smem_desc(q_addr, 16, 1024, 2), bd = ptx::make_smem_desc(k_addr + st * K_STAGE_BYTES, 16, 1024, 2);
+                    if (ptx::elect_one()) {
 #pragma unroll
-                    for (int c = 0; c < KBLK; c++) {
+                        for (int c = 0; c < KBLK; c++)
 #pragma unroll
-                        for (int k4 = 0; k4 < 4; k4++) {
-                            uint64_t ad = ptx::make_smem_desc(q_addr + c * Q_BLK_BYTES + k4 * 32, 16, 1024, 2);
-                            uint64_t bd = ptx::make_smem_desc(k_addr + st * K_STAGE_BYTES + c * KSLOT_BYTES + k4 * 32,
-                                                              16, 1024, 2);
-                            mma2_f16(tmem + S_COL + st * 32, ad, bd, idesc_qk, (c > 0 || k4 > 0) ? 1u : 0u);
-                        }
+                            for (int k4 = 0; k4 < 4; k4++)
+                                mma2_f16(tmem + S_COL + st * 32, ad + (c * Q_BLK_BYTES + k4 * 32) / 16, bd + (c * KSLOT_BYTES + k4 * 32) / 16,
+                                         idesc_qk, (c > 0 || k4 > 0) ? 1u : 0u);
+                        commit_both(&sm->k_empty[st]);
+                        commit_both(&sm->s_full[st]);
                     }
-                    commit_both(&sm->k_empty[st]);
-                    commit_both(&sm->s_full[st]);
                 }
                 if (j > 0 && !issue_pv(j - 1)) goto done;
             }
             if (!issue_pv(nt - 1)) goto done;
-            if (leader) commit_both(&sm->o_done);
+            if (leader && ptx::elect_one()) commit_both(&sm->o_done);
         }
     } else {
         // ===================== softmax / correction / epilogue (warps 0-3 of each CTA) =====================
@@ -535,9 +533,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS128, 1) dsa_d
     Smem* sm = reinterpret_cast<Smem*>(sP + P_BYTES);
     volatile int* abort_flag = &sm->abort_flag;
 
-    const uint32_t rank = cluster_rank();          // 0 = leader
+    const uint32_t rank = (uint32_t)ptx::uniform((int)cluster_rank());          // 0 = leader
     const int sp = blockIdx.y, b = blockIdx.z;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = ptx::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int nt_total = p.S / TKV;
     const int t_begin = sp * p.tiles_per_split;
     const int nt = max(0, min(nt_total, t_begin + p.tiles_per_split) - t_begin);
@@ -703,7 +701,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS128, 1) dsa_d
         ptx::cp_async_wait<0>();           // nothing of this thread is in flight when the CTA winds down
     } else if (warp == 4) {
         // ===================== MMA issuer (leader) / barrier relay (peer) =====================
-        if (lane == 0 && nt > 0) {
+        if (nt > 0) {
             const bool leader = (rank == 0);
             constexpr uint32_t idesc_qk = ptx::make_idesc(1, 1, 0, 0, HEADS, TKV);
             constexpr uint32_t idesc_pv = ptx::make_idesc(1, 1, 0, 1, HEADS, 256);
@@ -711,54 +709,54 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS128, 1) dsa_d
                            p_addr = ptx::smem_u32(sP);
             auto forward_or_wait = [&](uint64_t* peer, uint32_t par_peer) -> bool {
                 ptx::fence_proxy_async_smem();
-                if (leader) return mbar_wait_cluster(peer, par_peer, abort_flag);
-                mbar_arrive_cta(peer, 0);
+                if (leader) return ptx::whole_warp(mbar_wait_cluster(peer, par_peer, abort_flag));
+                if (ptx::elect_one()) mbar_arrive_cta(peer, 0);
                 return true;
             };
             auto issue_pv = [&](int i) -> bool {
                 const uint32_t par = (uint32_t)(i & 1);
-                if (!ptx::mbar_wait(&sm->p_full, par, abort_flag)) return false;
-                if (!ptx::mbar_wait(&sm->v_full, par, abort_flag)) return false;
+                if (!ptx::whole_warp(ptx::mbar_wait(&sm->p_full, par, abort_flag))) return false;
+                if (!ptx::whole_warp(ptx::mbar_wait(&sm->v_full, par, abort_flag))) return false;
                 if (!forward_or_wait(&sm->pv_peer, par)) return false;
                 if (!leader) return true;
                 ptx::tc_fence_after();
+                const uint64_t ad = ptx::make_smem_desc(p_addr, P_CHUNK_BYTES, 128, 0), bd = ptx::make_smem_desc(v_addr, VCHUNK_BYTES, 1024, 2);
+                if (ptx::elect_one()) {
 #pragma unroll
-                for (int inst = 0; inst < 2; inst++) {
+                    for (int inst = 0; inst < 2; inst++)
 #pragma unroll
-                    for (int ks = 0; ks < 8; ks++) {
-                        uint64_t ad = ptx::make_smem_desc(p_addr + ks * 2 * P_CHUNK_BYTES, P_CHUNK_BYTES, 128, 0);
-                        uint64_t bd = ptx::make_smem_desc(v_addr + 2 * inst * VCHUNK_BYTES + ks * 2048, VCHUNK_BYTES, 1024, 2);
-                        mma2_f16(tmem + O_COL + 128 * inst, ad, bd, idesc_pv, (i > 0 || ks > 0) ? 1u : 0u);
-                    }
+                        for (int ks = 0; ks < 8; ks++)
+                            mma2_f16(tmem + O_COL + 128 * inst, ad + ks * (2 * P_CHUNK_BYTES / 16), bd + (2 * inst * VCHUNK_BYTES + ks * 2048) / 16,
+                                     idesc_pv, (i > 0 || ks > 0) ? 1u : 0u);
+                    commit_both(&sm->v_empty);
+                    commit_both(&sm->p_empty);
                 }
-                commit_both(&sm->v_empty);
-                commit_both(&sm->p_empty);
                 return true;
             };
-            if (!ptx::mbar_wait(&sm->q_full, 0, abort_flag)) goto done;     // (fenced with the first K stage below)
+            if (!ptx::whole_warp(ptx::mbar_wait(&sm->q_full, 0, abort_flag))) goto done;     // (fenced with the first K stage below)
             for (int j = 0; j < nt; j++) {
                 const int sb = j & 1;
-                if (!ptx::mbar_wait(&sm->s_empty[sb], (uint32_t)(((j >> 1) & 1) ^ 1), abort_flag)) goto done;
-                if (!ptx::mbar_wait(&sm->k_full, (uint32_t)(j & 1), abort_flag)) goto done;
+                if (!ptx::whole_warp(ptx::mbar_wait(&sm->s_empty[sb], (uint32_t)(((j >> 1) & 1) ^ 1), abort_flag))) goto done;
+                if (!ptx::whole_warp(ptx::mbar_wait(&sm->k_full, (uint32_t)(j & 1), abort_flag))) goto done;
                 if (!forward_or_wait(&sm->qk_peer, (uint32_t)(j & 1))) goto done;
                 if (leader) {
                     ptx::tc_fence_after();
+                    const uint64_t ad = ptx::make_smem_desc(q_addr, 16, 1024, 2), bd = ptx::make_smem_desc(k_addr, 16, 1024, 2);
+                    if (ptx::elect_one()) {
 #pragma unroll
-                    for (int c = 0; c < KBLK; c++) {
+                        for (int c = 0; c < KBLK; c++)
 #pragma unroll
-                        for (int k4 = 0; k4 < 4; k4++) {
-                            uint64_t ad = ptx::make_smem_desc(q_addr + c * Q_BLK_BYTES + k4 * 32, 16, 1024, 2);
-                            uint64_t bd = ptx::make_smem_desc(k_addr + c * KSLOT_BYTES + k4 * 32, 16, 1024, 2);
-                            mma2_f16(tmem + S_COL + sb * 64, ad, bd, idesc_qk, (c > 0 || k4 > 0) ? 1u : 0u);
-                        }
+                            for (int k4 = 0; k4 < 4; k4++)
+                                mma2_f16(tmem + S_COL + sb * 64, ad + (c * Q_BLK_BYTES + k4 * 32) / 16, bd + (c * KSLOT_BYTES + k4 * 32) / 16,
+                                         idesc_qk, (c > 0 || k4 > 0) ? 1u : 0u);
+                        commit_both(&sm->k_empty);
+                        commit_both(&sm->s_full[sb]);
                     }
-                    commit_both(&sm->k_empty);
-                    commit_both(&sm->s_full[sb]);
                 }
                 if (j > 0 && !issue_pv(j - 1)) goto done;
             }
             if (!issue_pv(nt - 1)) goto done;
-            if (leader) commit_both(&sm->o_done);
+            if (leader && ptx::elect_one()) commit_both(&sm->o_done);
         }
     } else {
         // ===================== softmax / correction / epilogue (warps 0-3 of each CTA) =====================
