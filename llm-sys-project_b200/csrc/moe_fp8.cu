@@ -90,7 +90,10 @@ struct GemmSmem {
     alignas(16) float stage[NUM_PROMO_WARPS][32][SW + 4];   // per promotion warp: 32 rows x SW columns (+4 pad), output transpose
 };
 
-constexpr size_t GEMM_SMEM_BYTES = 1024 /*alignment slack*/ + (size_t)STAGES * STAGE_BYTES + sizeof(GemmSmem);
+constexpr size_t GEMM_BASE_BYTES = 1024 /*alignment slack*/ + (size_t)STAGES * STAGE_BYTES + sizeof(GemmSmem);
+// scales of four K blocks: [K block % 4][gate / up or column half][row]
+constexpr int SC_RING = 4;
+constexpr size_t GEMM_SMEM_BYTES = GEMM_BASE_BYTES + sizeof(float) * SC_RING * 2 * BM;
 static_assert(GEMM_SMEM_BYTES <= 232448, "shared memory budget of one CTA");
 // block-scaled kernel: per stage one 512-byte scale atom for the 128 rows of A and two for the 256 rows of B
 constexpr int SF_BYTES = 1536;
@@ -99,17 +102,19 @@ constexpr int SF_BYTES = 1536;
 // error on GEMM1, enough to flip one e4m3 code in a thousand at the requantisation and to push a few outputs of
 // the full-size layer past the 1e-2 absolute bound); 32 MMAs per chain keep it near fp32.
 constexpr int MX_FLUSH = 8;
-constexpr size_t GEMM_MX_SMEM_BYTES = GEMM_SMEM_BYTES + (size_t)STAGES * SF_BYTES;
+constexpr size_t GEMM_MX_SMEM_BYTES = GEMM_BASE_BYTES + (size_t)STAGES * SF_BYTES;
 static_assert(GEMM_MX_SMEM_BYTES <= 232448, "shared memory budget of one CTA (block-scaled kernel)");
 
 struct GemmParams {
-    const float* a_scale;      // [rows, nkb]
+    const float* a_scale;      // scale of sorted row r, K block kb: a_scale[kb * a_ks + r]
+    long long a_ks;
     const float* w_scale;      // MODE 1: [E, 2I/128, D/128]   MODE 2/3: [E, D/128, I/128]
     const int* offsets;        // [E+1]
     const int* row_tok;        // MODE 2
     const float* row_w;        // MODE 2/3
     uint8_t* act_q;            // MODE 1 out [rows, I]
-    float* act_s;              // MODE 1 out [rows, I/128]
+    float* act_s;              // MODE 1 out: scale of row r, block b at act_s[r * s_rs + b * s_ks]
+    long long s_rs, s_ks;
     float* out;                // MODE 2 out [T, D]; MODE 3 out [rows, D]
     int* status;
     int E, D, I;
@@ -154,7 +159,8 @@ __device__ __forceinline__ uint32_t cluster_nctarank() {
 // every tile: each arrives on the neighbour's barrier and waits on its own (bounded).
 __device__ __forceinline__ bool pair_rendezvous(uint64_t* own_bar, uint32_t peer_bar_cluster_addr, uint32_t parity,
                                                 volatile int* abort_flag) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(peer_bar_cluster_addr) : "memory");
+    if (ptx::elect_one())
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(peer_bar_cluster_addr) : "memory");
     return ptx::mbar_wait_relaxed(own_bar, parity, abort_flag, 100);
 }
 __device__ __forceinline__ void cluster_sync_all() {
@@ -311,9 +317,10 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     GemmSmem* sm = reinterpret_cast<GemmSmem*>(tiles + (size_t)STAGES * STAGE_BYTES);
+    float (*const scales)[2][BM] = reinterpret_cast<float (*)[2][BM]>(sm + 1);
     volatile int* abort_flag = &sm->abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = ptx::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int Kdim = (MODE == 1) ? p.D : p.I;
     const int nkb = Kdim / BK;
     const int NT = (MODE == 1) ? p.I / 128 : p.D / 256;     // N tiles per expert
@@ -329,7 +336,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         // arrival from every promotion warp of both CTAs
         for (int s = 0; s < STAGES; s++) { ptx::mbar_init(&sm->full[s], PAIR ? 2 : 1); ptx::mbar_init(&sm->empty[s], 1); }
         for (int a = 0; a < 2; a++) {
-            ptx::mbar_init(&sm->tmem_full[a], 1);
+            ptx::mbar_init(&sm->tmem_full[a], 2);             // the commit and the scale warp
             ptx::mbar_init(&sm->tmem_empty[a], PAIR ? 2 * NUM_PROMO_WARPS : NUM_PROMO_WARPS);
             ptx::mbar_init(&sm->amax_bar[a], NUM_PROMO_WARPS);
         }
@@ -353,7 +360,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     if (PAIR || duo) cluster_sync_all();      // the peer's barriers are initialised before anyone signals them
     ptx::tc_fence_after();
     const uint32_t tmem_base = sm->tmem_base;
-    const int total_tiles = sm->total_tiles;
+    const int total_tiles = ptx::uniform(sm->total_tiles);
 
     // tile -> (expert, m_tile, n_tile): expert-major, then n, then m, so the CTAs that run
     // together walk through one expert's weights once.
@@ -365,10 +372,10 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         }
         // experts with zero tiles repeat the prefix value; the search lands on the last
         // expert whose prefix is <= tile, which is the one that owns tiles.
-        e = lo;
-        cnt = p.offsets[e + 1] - p.offsets[e];
+        e = ptx::uniform(lo);
+        cnt = ptx::uniform(p.offsets[e + 1] - p.offsets[e]);
         int mt = (cnt + TM - 1) / TM;
-        int local = tile - sm->tile_prefix[e];
+        int local = tile - ptx::uniform(sm->tile_prefix[e]);
         n_tile = local / mt;
         m_tile = local - n_tile * mt;
     };
@@ -377,7 +384,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         ptx::setmaxnreg_dec<AUX_REGS>();
       if (warp == W_TMA) {
         // ===================== TMA producer =====================
-        if (lane == 0) {
+        {
             int s = 0; uint32_t ph = 0; int gk = 0; (void)gk;
             uint32_t go_ph = 0;
             const uint32_t peer_go = duo ? map_to_cta(&sm->pair_go, cluster_ctarank() ^ 1u) : 0u;
@@ -385,18 +392,20 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                 int e, m_tile, n_tile, cnt;
                 locate(tile, e, m_tile, n_tile, cnt);
                 if (duo && (tile | 1) < total_tiles) {        // the neighbour has a tile in this pass over the grid too
-                    if (!pair_rendezvous(&sm->pair_go, peer_go, go_ph, abort_flag)) goto done;
+                    if (!ptx::whole_warp(pair_rendezvous(&sm->pair_go, peer_go, go_ph, abort_flag))) goto done;
                     go_ph ^= 1;
                 }
-                const int row0 = p.offsets[e] + m_tile * TM + (int)crank * BM;
+                const int row0 = ptx::uniform(p.offsets[e]) + m_tile * TM + (int)crank * BM;
                 const uint32_t a_bytes = a_tile_bytes(cnt - m_tile * TM);
                 const long long wrow0 = (long long)e * w_rows;
                 for (int kb = 0; kb < nkb; kb++) {
-                    if (!ptx::mbar_wait_relaxed(&sm->empty[s], ph ^ 1, abort_flag, PRODUCER_SLEEP_NS)) goto done;
+                    if (!ptx::whole_warp(ptx::mbar_wait_relaxed(&sm->empty[s], ph ^ 1, abort_flag, PRODUCER_SLEEP_NS))) goto done;
                     TRACE_STAMP(6, gk); gk++;
                     uint8_t* a_dst = tiles + (size_t)s * STAGE_BYTES;
                     uint8_t* b_dst = a_dst + A_BYTES;
-                    if (PAIR) {
+                    if (!ptx::elect_one()) {
+                        // (the elected lane alone issues the loads)
+                    } else if (PAIR) {
                         // this CTA's 128 rows of A and its half of the weight tile (accumulator columns
                         // 128 crank .. +127); the bytes are counted on the leader's barrier
                         const uint32_t fbar = map_to_cta(&sm->full[s], 0);
@@ -438,7 +447,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         // K block's MMAs stays tied up until they have run (in the issue of the later ones and in the
         // commits); with a single issuer it came back to look at the other stage's "free" barrier
         // hundreds of cycles after the promotion warps had released it.
-        if (lane == 0 && crank == 0) {
+        if (crank == 0) {
             constexpr uint32_t idesc = ptx::make_idesc(0, 0, 0, 0, TM, BN);
             const int role = warp - W_MMA0;                 // the TMEM stage this issuer owns
             int s = 0; uint32_t ph = 0;
@@ -448,32 +457,87 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                     if ((int)(g & 1) == role) {
                         // (waits on barriers that the peer CTA or tcgen05.commit signal need no cluster-scope
                         // acquire: what they hand over is a TMEM stage or TMA-written tiles, not memory data)
-                        if (!ptx::mbar_wait(&sm->tmem_empty[role], acc_ph ^ 1, abort_flag)) goto done;
+                        if (!ptx::whole_warp(ptx::mbar_wait(&sm->tmem_empty[role], acc_ph ^ 1, abort_flag))) goto done;
                         TRACE_STAMP(0, g);
-                        if (!ptx::mbar_wait(&sm->full[s], ph, abort_flag)) goto done;
+                        if (!ptx::whole_warp(ptx::mbar_wait(&sm->full[s], ph, abort_flag))) goto done;
                         TRACE_STAMP(1, g);
                         ptx::tc_fence_after();
                         const uint32_t a_addr = ptx::smem_u32(tiles + (size_t)s * STAGE_BYTES);
-                        const uint32_t b_addr = a_addr + A_BYTES;
+                        const uint64_t ad = ptx::make_smem_desc(a_addr, 16, 1024, 2), bd = ptx::make_smem_desc(a_addr + A_BYTES, 16, 1024, 2);
                         const uint32_t d_tmem = tmem_base + role * BN;
+                        if (ptx::elect_one()) {
 #pragma unroll
-                        for (int k4 = 0; k4 < 4; k4++) {
-                            uint64_t ad = ptx::make_smem_desc(a_addr + k4 * 32, 16, 1024, 2);
-                            uint64_t bd = ptx::make_smem_desc(b_addr + k4 * 32, 16, 1024, 2);
-                            if (PAIR) mma2_f8(d_tmem, ad, bd, idesc, k4 > 0 ? 1u : 0u);
-                            else      ptx::mma_f8(d_tmem, ad, bd, idesc, k4 > 0 ? 1u : 0u);
-                        }
-                        if (PAIR) {
-                            commit_both(&sm->empty[s]);
-                            commit_both(&sm->tmem_full[role]);
-                        } else {
-                            ptx::tc_commit(&sm->empty[s]);          // smem stage reusable once the MMAs have read it
-                            ptx::tc_commit(&sm->tmem_full[role]);   // partial sums ready for promotion
+                            for (int k4 = 0; k4 < 4; k4++) {        // 32 bytes further along K: 2 in the descriptor's 16-byte units
+                                if (PAIR) mma2_f8(d_tmem, ad + 2 * k4, bd + 2 * k4, idesc, k4 > 0 ? 1u : 0u);
+                                else      ptx::mma_f8(d_tmem, ad + 2 * k4, bd + 2 * k4, idesc, k4 > 0 ? 1u : 0u);
+                            }
+                            if (PAIR) {
+                                commit_both(&sm->empty[s]);
+                                commit_both(&sm->tmem_full[role]);
+                            } else {
+                                ptx::tc_commit(&sm->empty[s]);          // smem stage reusable once the MMAs have read it
+                                ptx::tc_commit(&sm->tmem_full[role]);   // partial sums ready for promotion
+                            }
                         }
                         TRACE_STAMP(2, g);
                         acc_ph ^= 1;
                     }
                     if (++s == STAGES) { s = 0; ph ^= 1; }
+                }
+            }
+        }
+      } else {
+        // ===================== scales =====================
+        // a_scale[row, kb] * w_scale[block, kb] of the tile's 128 rows into shared memory, K block by K block.  Loaded by the
+        // promotion warps themselves one K block ahead, the scales' latency (32 rows of a row-major matrix are 32 cache lines) was
+        // longer than a K block: it held the warps back by different amounts, and the last one sets the pace.
+        const int nkb_w = Kdim / 128;
+        uint32_t g = 0;                                     // K blocks since the kernel started
+        for (int tile = walker; tile < total_tiles; tile += pair_count) {
+            int e, m_tile, n_tile, cnt;
+            locate(tile, e, m_tile, n_tile, cnt);
+            const int trow0 = m_tile * TM + (int)crank * BM, left = cnt - trow0 - lane;      // rows lane + 32 i exist for 32 i < left
+            const float* a_sc = p.a_scale + (long long)p.offsets[e] + trow0 + lane;
+            const float *w0, *w1;
+            if (MODE == 1) {
+                w0 = p.w_scale + ((size_t)e * (2 * p.I / 128) + n_tile) * nkb_w;             // gate rows' block
+                w1 = w0 + (size_t)(p.I / 128) * nkb_w;                                       // up rows' block
+            } else {
+                w0 = p.w_scale + ((size_t)e * (p.D / 128) + n_tile * 2) * nkb_w;             // columns 0 .. 127 of the tile
+                w1 = w0 + nkb_w;                                                             // columns 128 .. 255
+            }
+            // two K blocks ahead
+            float a[2][4], w[2][2];
+            auto fetch = [&](int kb, float (&av)[4], float (&wv)[2]) {
+                if (kb < nkb) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) av[i] = 32 * i < left ? a_sc[kb * p.a_ks + 32 * i] : 0.0f;
+                    wv[0] = w0[kb];
+                    wv[1] = w1[kb];
+                }
+            };
+            auto publish = [&](float (&av)[4], float (&wv)[2]) -> bool {
+                // This slot's last K block, g - 4, has been read once the MMAs of block g - 2 have run: they waited for it.
+                if (g >= 2 && !ptx::whole_warp(ptx::mbar_wait(&sm->tmem_full[g & 1], ((g >> 1) & 1) ^ 1, abort_flag))) return false;
+                float (*const sc)[BM] = scales[g % SC_RING];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    sc[0][lane + 32 * i] = av[i] * wv[0];
+                    sc[1][lane + 32 * i] = av[i] * wv[1];
+                }
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(&sm->tmem_full[g & 1]);
+                g++;
+                return true;
+            };
+            fetch(0, a[0], w[0]);
+            fetch(1, a[1], w[1]);
+            for (int kb = 0; kb < nkb; kb += 2) {
+                if (!publish(a[0], w[0])) goto done;
+                fetch(kb + 2, a[0], w[0]);
+                if (kb + 1 < nkb) {
+                    if (!publish(a[1], w[1])) goto done;
+                    fetch(kb + 3, a[1], w[1]);
                 }
             }
         }
@@ -499,7 +563,6 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
 #ifdef B200_GEMM_TRACE
         const bool trw = (threadIdx.x == p.trace_warp * 32);
 #endif
-        const int nkb_w = Kdim / 128;
         // the stage's "free" barrier lives in the leader CTA
         const uint32_t tmem_empty_addr[2] = {PAIR ? map_to_cta(&sm->tmem_empty[0], 0) : 0u,
                                              PAIR ? map_to_cta(&sm->tmem_empty[1], 0) : 0u};
@@ -507,35 +570,18 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
             if (PAIR && crank != 0) mbar_arrive_cluster(tmem_empty_addr[a]);
             else                    ptx::mbar_arrive(&sm->tmem_empty[a]);
         };
-        // What a tile needs before its first K block: where it lies, and the scales of that K block.  The next tile's is
-        // fetched in front of the epilogue of the current one: behind it, finding the tile and waiting for the scales
-        // took a good part of the gap between two tiles (a GEMM2 tile of 16 K blocks: 20500 cycles + a gap of 10000).
-        // T = 16 840 -> 819 us, T = 333 2120 -> 2055, T = 4096 3310 -> 3236, 32 experts x 1024 rows 2190 -> 2110.
+        // Where the next tile lies is looked up in front of the epilogue of the current one (behind it, that took a good part of
+        // the gap between two tiles: T = 16 840 -> 819 us, T = 4096 3310 -> 3236, 32 experts x 1024 rows 2190 -> 2110).
         struct Tile {
             int off, cnt, trow0, n_tile;               // the expert's first sorted row and row count; first row of this CTA inside it
-            const float *a_sc, *w_sc0, *w_sc1;
-            float sa, w0, w1;
         } cur, nxt;
         auto open_tile = [&](int tile, Tile& x) {
             int e, m_tile;
             locate(tile, e, m_tile, x.n_tile, x.cnt);
             x.off = p.offsets[e];
             x.trow0 = m_tile * TM + (int)crank * BM;
-            const long long grow = (long long)x.off + x.trow0 + row;
-            x.a_sc = p.a_scale + (grow < p.total_rows ? grow : 0) * nkb;
-            if (MODE == 1) {
-                const float* base = p.w_scale + (size_t)e * (2 * p.I / 128) * nkb_w;
-                x.w_sc0 = base + (size_t)x.n_tile * nkb_w;                     // gate rows' block
-                x.w_sc1 = base + (size_t)(p.I / 128 + x.n_tile) * nkb_w;       // up rows' block
-            } else {
-                const float* base = p.w_scale + (size_t)e * (p.D / 128) * nkb_w;
-                x.w_sc0 = base + (size_t)(x.n_tile * 2 + (wq * QCOLS) / 128) * nkb_w;
-                x.w_sc1 = x.w_sc0;
-            }
-            x.sa = x.trow0 + row < x.cnt ? x.a_sc[0] : 0.0f;
-            x.w0 = x.w_sc0[0];
-            x.w1 = (MODE == 1) ? x.w_sc1[0] : 0.0f;
         };
+        uint32_t gsc = 0;                                     // K blocks since the kernel started
         if (walker < total_tiles) open_tile(walker, nxt);
         for (int tile = walker; tile < total_tiles; tile += pair_count) {
             cur = nxt;
@@ -543,23 +589,13 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
             const long long grow = (long long)cur.off + trow0 + row;              // sorted row
             const bool row_ok = (trow0 + row) < cnt;
             const bool warp_valid = (trow0 + (warp & 3) * 32) < cnt;              // any valid row in this warp's 32
-            const float *const a_sc = cur.a_sc, *const w_sc0 = cur.w_sc0, *const w_sc1 = cur.w_sc1;
             const float row_weight = (MODE != 1 && row_ok) ? p.row_w[grow] : 0.0f;     // used by the epilogue
             const int row_token = (MODE == 2 && row_ok) ? p.row_tok[grow] : -1;
             float accv[QCOLS];
 #pragma unroll
             for (int i = 0; i < QCOLS; i++) accv[i] = 0.0f;
 
-            // scales of K block kb+1 are fetched while block kb is being promoted
-            float sa_n = cur.sa, w0_n = cur.w0, w1_n = cur.w1;
-            for (int kb = 0; kb < nkb; kb++) {
-                const float s0 = sa_n * w0_n;
-                const float s1 = (MODE == 1) ? sa_n * w1_n : s0;
-                if (kb + 1 < nkb) {
-                    sa_n = row_ok ? a_sc[kb + 1] : 0.0f;
-                    w0_n = w_sc0[kb + 1];
-                    if (MODE == 1) w1_n = w_sc1[kb + 1];
-                }
+            for (int kb = 0; kb < nkb; kb++, gsc++) {
                 if (!warp_wait(&sm->tmem_full[acc], acc_ph)) goto done;
 #ifdef B200_GEMM_TRACE
                 if (trw) TRACE_STAMP(3, gp);
@@ -567,6 +603,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                 if (warp_valid) {
                     // warps whose 32 rows are all padding only hand the stage back
                     ptx::tc_fence_after();
+                    const float (*const sc)[BM] = scales[gsc % SC_RING];
+                    const float s0 = (MODE == 1) ? sc[0][row] : sc[(wq * QCOLS) / 128][row], s1 = (MODE == 1) ? sc[1][row] : s0;
                     const uint32_t t0 = tmem_base + lane_addr + acc * BN + wq * QCOLS;
                     // QCOLS columns in chunks of CH, two loads in flight; columns [0, QCOLS/2) take s0 (MODE 1:
                     // gate), the rest s1 (MODE 1: up)
@@ -637,7 +675,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
 #pragma unroll
                     for (int i = 0; i < AC / 16; i++)
                         dst[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
-                    if (wq == 0) p.act_s[grow * (p.I / 128) + n_tile] = scale;
+                    if (wq == 0) p.act_s[grow * p.s_rs + n_tile * p.s_ks] = scale;
                 }
                 tile_par ^= 1;
             } else if (warp_valid) {
@@ -719,7 +757,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     GemmSmem* sm = reinterpret_cast<GemmSmem*>(sf_area + (size_t)STAGES * SF_BYTES);
     volatile int* abort_flag = &sm->abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = ptx::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int Kdim = (MODE == 1) ? p.D : p.I;
     const int nkb = Kdim / BK;
     const int NT = (MODE == 1) ? p.I / 128 : p.D / 256;     // N tiles per expert
@@ -753,7 +791,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     if (duo) cluster_sync_all();              // the neighbour's barrier is initialised before anyone signals it
     ptx::tc_fence_after();
     const uint32_t tmem_base = sm->tmem_base;
-    const int total_tiles = sm->total_tiles;
+    const int total_tiles = ptx::uniform(sm->total_tiles);
 
     auto locate = [&](int tile, int& e, int& m_tile, int& n_tile, int& cnt) {
         int lo = 0, hi = p.E;
@@ -761,10 +799,10 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
             int mid = (lo + hi) >> 1;
             if (sm->tile_prefix[mid] <= tile) lo = mid; else hi = mid;
         }
-        e = lo;
-        cnt = p.offsets[e + 1] - p.offsets[e];
+        e = ptx::uniform(lo);
+        cnt = ptx::uniform(p.offsets[e + 1] - p.offsets[e]);
         int mt = (cnt + BM - 1) / BM;
-        int local = tile - sm->tile_prefix[e];
+        int local = tile - ptx::uniform(sm->tile_prefix[e]);
         n_tile = local / mt;
         m_tile = local - n_tile * mt;
     };
@@ -781,35 +819,37 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         ptx::setmaxnreg_dec<AUX_REGS>();
       if (warp == W_TMA) {
         // ===================== TMA producer (operand tiles) =====================
-        if (lane == 0) {
+        {
             int s = 0; uint32_t ph = 0, go_ph = 0;
             const uint32_t peer_go = duo ? map_to_cta(&sm->pair_go, cluster_ctarank() ^ 1u) : 0u;
             for (int tile = walker; tile < total_tiles; tile += walkers) {
                 int e, m_tile, n_tile, cnt;
                 locate(tile, e, m_tile, n_tile, cnt);
                 if (duo && (tile | 1) < total_tiles) {        // the neighbour has a tile in this pass over the grid too
-                    if (!pair_rendezvous(&sm->pair_go, peer_go, go_ph, abort_flag)) goto done;
+                    if (!ptx::whole_warp(pair_rendezvous(&sm->pair_go, peer_go, go_ph, abort_flag))) goto done;
                     go_ph ^= 1;
                 }
-                const int row0 = p.offsets[e] + m_tile * BM;
+                const int row0 = ptx::uniform(p.offsets[e]) + m_tile * BM;
                 const uint32_t a_bytes = a_tile_bytes(cnt - m_tile * BM);
                 const long long wrow0 = (long long)e * w_rows;
                 for (int kb = 0; kb < nkb; kb++) {
-                    if (!ptx::mbar_wait_relaxed(&sm->empty[s], ph ^ 1, abort_flag, PRODUCER_SLEEP_NS)) goto done;
+                    if (!ptx::whole_warp(ptx::mbar_wait_relaxed(&sm->empty[s], ph ^ 1, abort_flag, PRODUCER_SLEEP_NS))) goto done;
                     uint8_t* a_dst = tiles + (size_t)s * STAGE_BYTES;
                     uint8_t* b_dst = a_dst + A_BYTES;
-                    ptx::mbar_expect_tx(&sm->full[s], a_bytes + B_BYTES);
-                    load_a_rows(a_dst, &tmap_a, &tmap_a32, &sm->full[s], kb * BK, row0, a_bytes);
-                    if (p.packed) {
-                        ptx::tma_load_2d(b_dst, &tmap_b, &sm->full[s], 0, (((e * NT + n_tile) * nkb) + kb) * BN);
-                    } else if (MODE == 1) {
-                        const int j0 = n_tile * 128;
+                    if (ptx::elect_one()) {
+                        ptx::mbar_expect_tx(&sm->full[s], a_bytes + B_BYTES);
+                        load_a_rows(a_dst, &tmap_a, &tmap_a32, &sm->full[s], kb * BK, row0, a_bytes);
+                        if (p.packed) {
+                            ptx::tma_load_2d(b_dst, &tmap_b, &sm->full[s], 0, (((e * NT + n_tile) * nkb) + kb) * BN);
+                        } else if (MODE == 1) {
+                            const int j0 = n_tile * 128;
 #pragma unroll
-                        for (int bx = 0; bx < 2 * NQ; bx++)
-                            ptx::tma_load_2d(b_dst + bx * (QCOLS / 2) * 128, &tmap_b, &sm->full[s], kb * BK,
-                                             (int)(wrow0 + ((bx & 1) ? p.I : 0) + j0 + (QCOLS / 2) * (bx >> 1)));
-                    } else {
-                        ptx::tma_load_2d(b_dst, &tmap_b, &sm->full[s], kb * BK, (int)(wrow0 + n_tile * 256));
+                            for (int bx = 0; bx < 2 * NQ; bx++)
+                                ptx::tma_load_2d(b_dst + bx * (QCOLS / 2) * 128, &tmap_b, &sm->full[s], kb * BK,
+                                                 (int)(wrow0 + ((bx & 1) ? p.I : 0) + j0 + (QCOLS / 2) * (bx >> 1)));
+                        } else {
+                            ptx::tma_load_2d(b_dst, &tmap_b, &sm->full[s], kb * BK, (int)(wrow0 + n_tile * 256));
+                        }
                     }
                     if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
@@ -817,36 +857,35 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         }
       } else if (warp == W_MMA0) {
         // ===================== scale copies + MMAs =====================
-        if (lane == 0) {
+        {
             int s = 0; uint32_t ph = 0, tph = 0;
             for (int tile = walker; tile < total_tiles; tile += walkers) {
               for (int kb0 = 0; kb0 < nkb; kb0 += MX_FLUSH) {
                 // the epilogue warps have added the previous segment (or tile) into their registers
-                if (!ptx::mbar_wait(&sm->tmem_empty[0], tph ^ 1, abort_flag)) goto done;
+                if (!ptx::whole_warp(ptx::mbar_wait(&sm->tmem_empty[0], tph ^ 1, abort_flag))) goto done;
                 ptx::tc_fence_after();
                 const int kb1 = min(nkb, kb0 + MX_FLUSH);
                 for (int kb = kb0; kb < kb1; kb++) {
-                    if (!ptx::mbar_wait(&sm->full[s], ph, abort_flag)) goto done;
-                    if (!ptx::mbar_wait(&sm->sf_full[s], ph, abort_flag)) goto done;
+                    if (!ptx::whole_warp(ptx::mbar_wait(&sm->full[s], ph, abort_flag))) goto done;
+                    if (!ptx::whole_warp(ptx::mbar_wait(&sm->sf_full[s], ph, abort_flag))) goto done;
                     ptx::tc_fence_after();
                     const uint32_t a_addr = ptx::smem_u32(tiles + (size_t)s * STAGE_BYTES);
-                    const uint32_t b_addr = a_addr + A_BYTES;
-                    const uint32_t sf_addr = ptx::smem_u32(sf_area + (size_t)s * SF_BYTES);
+                    const uint64_t ad = ptx::make_smem_desc(a_addr, 16, 1024, 2), bd = ptx::make_smem_desc(a_addr + A_BYTES, 16, 1024, 2);
+                    const uint64_t sd = ptx::make_smem_desc(ptx::smem_u32(sf_area + (size_t)s * SF_BYTES), 16, 128, 0);
                     const uint32_t tsfa = tmem_base + BN + 16 * s, tsfb = tsfa + 4;
-                    ptx::tmem_cp_32x128b_warpx4(tsfa, ptx::make_smem_desc(sf_addr, 16, 128, 0));
-                    ptx::tmem_cp_32x128b_warpx4(tsfb, ptx::make_smem_desc(sf_addr + 512, 16, 128, 0));
-                    ptx::tmem_cp_32x128b_warpx4(tsfb + 4, ptx::make_smem_desc(sf_addr + 1024, 16, 128, 0));
+                    if (ptx::elect_one()) {
+                        ptx::tmem_cp_32x128b_warpx4(tsfa, sd);
+                        ptx::tmem_cp_32x128b_warpx4(tsfb, sd + 512 / 16);
+                        ptx::tmem_cp_32x128b_warpx4(tsfb + 4, sd + 1024 / 16);
 #pragma unroll
-                    for (int k4 = 0; k4 < 4; k4++) {
-                        const uint64_t ad = ptx::make_smem_desc(a_addr + k4 * 32, 16, 1024, 2);
-                        const uint64_t bd = ptx::make_smem_desc(b_addr + k4 * 32, 16, 1024, 2);
-                        ptx::mma_mxf8(tmem_base, ad, bd, ptx::make_idesc_mx(BM, BN, k4, k4), tsfa, tsfb,
-                                      (kb > kb0 || k4 > 0) ? 1u : 0u);
+                        for (int k4 = 0; k4 < 4; k4++)
+                            ptx::mma_mxf8(tmem_base, ad + 2 * k4, bd + 2 * k4, ptx::make_idesc_mx(BM, BN, k4, k4), tsfa, tsfb,
+                                          (kb > kb0 || k4 > 0) ? 1u : 0u);
+                        ptx::tc_commit(&sm->empty[s]);          // operand tiles, scale atoms and their TMEM copies reusable
                     }
-                    ptx::tc_commit(&sm->empty[s]);          // operand tiles, scale atoms and their TMEM copies reusable
                     if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
-                ptx::tc_commit(&sm->tmem_full[0]);
+                if (ptx::elect_one()) ptx::tc_commit(&sm->tmem_full[0]);
                 tph ^= 1;
               }
             }
@@ -870,7 +909,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
             for (int q = 0; q < 4; q++) {
                 const int r = m_tile * BM + lane + 32 * q;
                 ok[q] = r < cnt;
-                a_sc[q] = p.a_scale + (size_t)(ok[q] ? (long long)p.offsets[e] + r : 0) * nkb;
+                a_sc[q] = p.a_scale + (ok[q] ? (long long)p.offsets[e] + r : 0);
             }
             const float* w_sc0;
             const float* w_sc1;
@@ -890,7 +929,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                 const float a0 = an[0], a1 = an[1], a2 = an[2], a3 = an[3], w0 = w0n, w1 = w1n;
                 if (kb + 1 < nkb) {
 #pragma unroll
-                    for (int q = 0; q < 4; q++) an[q] = ok[q] ? a_sc[q][kb + 1] : 1.0f;
+                    for (int q = 0; q < 4; q++) an[q] = ok[q] ? a_sc[q][(kb + 1) * p.a_ks] : 1.0f;
                     w0n = w_sc0[kb + 1];
                     w1n = w_sc1[kb + 1];
                 }
@@ -984,7 +1023,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
 #pragma unroll
                     for (int i = 0; i < AC / 16; i++)
                         dst[i] = make_uint4(packed[4 * i], packed[4 * i + 1], packed[4 * i + 2], packed[4 * i + 3]);
-                    if (wq == 0) p.act_s[grow * (p.I / 128) + n_tile] = scale;
+                    if (wq == 0) p.act_s[grow * p.s_rs + n_tile * p.s_ks] = scale;
                 }
                 tile_par ^= 1;
             } else if (warp_valid) {
@@ -1080,7 +1119,7 @@ __device__ __forceinline__ void copy_row(uint4* __restrict__ dst, const uint4* _
 __global__ void __launch_bounds__(128)
 sort_rows_fp8_kernel(const uint8_t* __restrict__ xq, const float* __restrict__ xs, const int* __restrict__ row_pair,
                      const int* __restrict__ offsets, const float* __restrict__ wts, int E, int K, int D,
-                     uint8_t* __restrict__ sq, float* __restrict__ ss, int* __restrict__ row_tok,
+                     uint8_t* __restrict__ sq, float* __restrict__ ss, long long s_ks, int* __restrict__ row_tok,
                      float* __restrict__ row_w, int* __restrict__ pair_row) {
     ptx::grid_wait();
     ptx::grid_release();
@@ -1092,7 +1131,7 @@ sort_rows_fp8_kernel(const uint8_t* __restrict__ xq, const float* __restrict__ x
         const uint4* src = reinterpret_cast<const uint4*>(xq + (size_t)tok * D);
         uint4* dst = reinterpret_cast<uint4*>(sq + (size_t)r * D);
         copy_row(dst, src, D / 16);
-        for (int i = threadIdx.x; i < nb; i += blockDim.x) ss[(size_t)r * nb + i] = xs[(size_t)tok * nb + i];
+        for (int i = threadIdx.x; i < nb; i += blockDim.x) ss[i * s_ks + r] = xs[(size_t)tok * nb + i];
         if (threadIdx.x == 0) {
             row_tok[r] = tok;
             row_w[r] = wts[pair];
@@ -1112,7 +1151,7 @@ constexpr int SMALL_PAIRS = 2048;
 __global__ void __launch_bounds__(128)
 sort_small_fp8_kernel(const uint8_t* __restrict__ xq, const float* __restrict__ xs, const int* __restrict__ ids,
                       const float* __restrict__ wts, int TK, int E, int K, int D, int* __restrict__ offsets,
-                      uint8_t* __restrict__ sq, float* __restrict__ ss, int* __restrict__ row_tok,
+                      uint8_t* __restrict__ sq, float* __restrict__ ss, long long s_ks, int* __restrict__ row_tok,
                       float* __restrict__ row_w, int* __restrict__ pair_row, float* __restrict__ out) {
     __shared__ int s_cnt[MAX_E];
     __shared__ int s_warp[4];
@@ -1168,7 +1207,7 @@ sort_small_fp8_kernel(const uint8_t* __restrict__ xq, const float* __restrict__ 
     const uint4* src = reinterpret_cast<const uint4*>(xq + (size_t)tok * D);
     uint4* dst = reinterpret_cast<uint4*>(sq + (size_t)r * D);
     copy_row(dst, src, D / 16);
-    for (int i = tid; i < nb; i += 128) ss[(size_t)r * nb + i] = xs[(size_t)tok * nb + i];
+    for (int i = tid; i < nb; i += 128) ss[i * s_ks + r] = xs[(size_t)tok * nb + i];
     if (tid == 0) {
         row_tok[r] = tok;
         row_w[r] = wts[pair];
@@ -1285,7 +1324,7 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
     int st = B200_OK;
     if (trusted && TK <= SMALL_PAIRS) {
         B200_CUDA_TRY(b200_launch_after(sort_small_fp8_kernel, dim3((unsigned)TK + 1), 128, 0, stream, xq, xs, ids, wts, (int)TK, E, K, D,
-                                        s.offsets, s.sq, s.ss, s.row_tok, s.row_w, det ? s.pair_row : nullptr,
+                                        s.offsets, s.sq, s.ss, TK, s.row_tok, s.row_w, det ? s.pair_row : nullptr,
                                         clear && !late ? out : nullptr));
     } else {
         if (clear && !late) B200_CUDA_TRY(cudaMemsetAsync(out, 0, out_bytes, stream));
@@ -1294,7 +1333,7 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
         if (det) B200_CUDA_TRY(cudaMemsetAsync(s.pair_row, 0xFF, sizeof(int) * (size_t)TK, stream));
         const unsigned sort_blocks = (unsigned)(TK < (long long)ws->sm_count * 32 ? TK : (long long)ws->sm_count * 32);
         B200_CUDA_TRY(b200_launch_after(sort_rows_fp8_kernel, dim3(sort_blocks), 128, 0, stream, xq, xs, s.row_pair, s.offsets, wts, E, K, D,
-                                        s.sq, s.ss, s.row_tok, s.row_w, det ? s.pair_row : nullptr));
+                                        s.sq, s.ss, TK, s.row_tok, s.row_w, det ? s.pair_row : nullptr));
     }
     b200_count_launch(1);
     B200_CUDA_TRY(cudaGetLastError());
@@ -1384,7 +1423,9 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
     if (packed) st = b200_make_tmap_u8_sw128(&tb, w1q, (unsigned long long)E * 2 * I * (D / 128), 128, pair ? 128 : 256);
     else        st = b200_make_tmap_u8_sw128(&tb, w1q, (unsigned long long)E * 2 * I, D, QCOLS / 2);
     if (st) return st;
-    p.a_scale = s.ss; p.w_scale = w1s; p.act_q = s.act_q; p.act_s = s.act_s;
+    // Scales of the sorted rows lie K block by K block, as the GEMMs read them; alone, GEMM1 leaves its own row by row.
+    p.a_scale = s.ss; p.a_ks = TK; p.w_scale = w1s; p.act_q = s.act_q; p.act_s = s.act_s;
+    p.s_rs = do_gemm2 ? 1 : I / 128; p.s_ks = do_gemm2 ? TK : 1;
     if (prof) B200_CUDA_TRY(cudaEventRecord(prof->ev[slot][0], stream));
     st = launch(1, ta, ta32, tb, p);
     if (st) return st;
