@@ -28,9 +28,8 @@
 //                into fp32 registers with a_scale[row,kb] * w_scale[nblk,kb] (the scales are
 //                arbitrary fp32 values, so the scaling cannot be left to the tensor core).
 //                Warp w owns TMEM lanes 32 (w % 4) .. +31 (the tile rows) and accumulator columns
-//                128 (w / 4) .. +127: 128 running sums per thread.  (A build with 16 promotion warps
-//                and 64 sums each, -DB200_GEMM_PROMO_WARPS=16, measured no faster; neither did packed
-//                fma.rn.f32x2 arithmetic, -DB200_GEMM_PACKED_FMA.)
+//                128 (w / 4) .. +127: 128 running sums per thread.
+//   warp 11      scales: a_scale[row,kb] * w_scale[nblk,kb] of the coming K blocks, and where the tile lies, into shared memory.
 // Every mbarrier wait is bounded; on give-up the CTA flags B200_TIMEOUT and winds down.
 #include "common.cuh"
 #include "moe_internal.cuh"
@@ -55,6 +54,7 @@ constexpr int GEMM_THREADS = 32 * (NUM_PROMO_WARPS + 4);   // promotion/epilogue
 constexpr int W_TMA = NUM_PROMO_WARPS, W_MMA0 = NUM_PROMO_WARPS + 1;
 constexpr int MAX_E = 1024;
 constexpr unsigned PRODUCER_SLEEP_NS = 40;
+constexpr int DIRECT_ROWS = 8;               // GEMM2: rows of a warp up to which each lane adds its own row
 // Register budgets after setmaxnreg.  The registers a warpgroup gives up are the only ones the others can
 // take (the pool is what the CTA was launched with: GEMM_THREADS x LAUNCH_REGS), and setmaxnreg.inc waits
 // without bound until its request is met, so the two sides must balance:
@@ -91,9 +91,9 @@ struct GemmSmem {
 };
 
 constexpr size_t GEMM_BASE_BYTES = 1024 /*alignment slack*/ + (size_t)STAGES * STAGE_BYTES + sizeof(GemmSmem);
-// scales of four K blocks: [K block % 4][gate / up or column half][row]
+// scales of four K blocks, [K block % 4][gate / up or column half][row], and where four tiles lie
 constexpr int SC_RING = 4;
-constexpr size_t GEMM_SMEM_BYTES = GEMM_BASE_BYTES + sizeof(float) * SC_RING * 2 * BM;
+constexpr size_t GEMM_SMEM_BYTES = GEMM_BASE_BYTES + sizeof(float) * SC_RING * 2 * BM + sizeof(int4) * SC_RING;
 static_assert(GEMM_SMEM_BYTES <= 232448, "shared memory budget of one CTA");
 // block-scaled kernel: per stage one 512-byte scale atom for the 128 rows of A and two for the 256 rows of B
 constexpr int SF_BYTES = 1536;
@@ -273,10 +273,10 @@ __device__ __forceinline__ void load_a_rows(uint8_t* dst, const CUtensorMap* map
         for (uint32_t o = 0; o < bytes; o += 32 * BK) ptx::tma_load_2d(dst + o, map32, bar, x, row0 + (int)(o / BK));
     }
 }
-// acc[0..N-1] += v[0..N-1] * s  (B200_GEMM_PACKED_FMA: as N/2 fma.rn.f32x2, same bits)
+// acc[0..N-1] += v[0..N-1] * s, two columns per instruction (the same bits as N fmaf in half the issue slots: with the scales out
+// of the loop T = 4096 3576 -> 3449 us, 32 experts x 1024 rows 2245 -> 2180 us)
 template <int N>
 __device__ __forceinline__ void promote(float* acc, const uint32_t (&v)[N], float s) {
-#ifdef B200_GEMM_PACKED_FMA
     const unsigned long long s2 = ptx::pack_f32x2(s, s);
 #pragma unroll
     for (int i = 0; i < N / 2; i++) {
@@ -284,10 +284,6 @@ __device__ __forceinline__ void promote(float* acc, const uint32_t (&v)[N], floa
                                                     ptx::pack_f32x2(acc[2 * i], acc[2 * i + 1]));
         ptx::unpack_f32x2(r, acc[2 * i], acc[2 * i + 1]);
     }
-#else
-#pragma unroll
-    for (int i = 0; i < N; i++) acc[i] = fmaf(__uint_as_float(v[i]), s, acc[i]);
-#endif
 }
 template <int N>
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[N]) {
@@ -318,6 +314,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     GemmSmem* sm = reinterpret_cast<GemmSmem*>(tiles + (size_t)STAGES * STAGE_BYTES);
     float (*const scales)[2][BM] = reinterpret_cast<float (*)[2][BM]>(sm + 1);
+    int4* const tile_at = reinterpret_cast<int4*>(scales + SC_RING);
     volatile int* abort_flag = &sm->abort_flag;
 
     const int warp = ptx::uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -492,12 +489,13 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         // promotion warps themselves one K block ahead, the scales' latency (32 rows of a row-major matrix are 32 cache lines) was
         // longer than a K block: it held the warps back by different amounts, and the last one sets the pace.
         const int nkb_w = Kdim / 128;
-        uint32_t g = 0;                                     // K blocks since the kernel started
-        for (int tile = walker; tile < total_tiles; tile += pair_count) {
+        uint32_t g = 0, tiles_done = 0;                     // K blocks, tiles since the kernel started
+        for (int tile = walker; tile < total_tiles; tile += pair_count, tiles_done++) {
             int e, m_tile, n_tile, cnt;
             locate(tile, e, m_tile, n_tile, cnt);
             const int trow0 = m_tile * TM + (int)crank * BM, left = cnt - trow0 - lane;      // rows lane + 32 i exist for 32 i < left
-            const float* a_sc = p.a_scale + (long long)p.offsets[e] + trow0 + lane;
+            const int off = p.offsets[e];
+            const float* a_sc = p.a_scale + (long long)off + trow0 + lane;
             const float *w0, *w1;
             if (MODE == 1) {
                 w0 = p.w_scale + ((size_t)e * (2 * p.I / 128) + n_tile) * nkb_w;             // gate rows' block
@@ -516,7 +514,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                     wv[1] = w1[kb];
                 }
             };
-            auto publish = [&](float (&av)[4], float (&wv)[2]) -> bool {
+            auto publish = [&](float (&av)[4], float (&wv)[2], bool first) -> bool {
                 // This slot's last K block, g - 4, has been read once the MMAs of block g - 2 have run: they waited for it.
                 if (g >= 2 && !ptx::whole_warp(ptx::mbar_wait(&sm->tmem_full[g & 1], ((g >> 1) & 1) ^ 1, abort_flag))) return false;
                 float (*const sc)[BM] = scales[g % SC_RING];
@@ -525,6 +523,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                     sc[0][lane + 32 * i] = av[i] * wv[0];
                     sc[1][lane + 32 * i] = av[i] * wv[1];
                 }
+                // (a tile has a K block at least: the slot's last tile, four tiles ago, has been read as well)
+                if (first && lane == 0) tile_at[tiles_done % SC_RING] = make_int4(off, cnt, trow0, n_tile);
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(&sm->tmem_full[g & 1]);
                 g++;
@@ -533,10 +533,10 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
             fetch(0, a[0], w[0]);
             fetch(1, a[1], w[1]);
             for (int kb = 0; kb < nkb; kb += 2) {
-                if (!publish(a[0], w[0])) goto done;
+                if (!publish(a[0], w[0], kb == 0)) goto done;
                 fetch(kb + 2, a[0], w[0]);
                 if (kb + 1 < nkb) {
-                    if (!publish(a[1], w[1])) goto done;
+                    if (!publish(a[1], w[1], false)) goto done;
                     fetch(kb + 3, a[1], w[1]);
                 }
             }
@@ -570,23 +570,14 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
             if (PAIR && crank != 0) mbar_arrive_cluster(tmem_empty_addr[a]);
             else                    ptx::mbar_arrive(&sm->tmem_empty[a]);
         };
-        // Where the next tile lies is looked up in front of the epilogue of the current one (behind it, that took a good part of
-        // the gap between two tiles: T = 16 840 -> 819 us, T = 4096 3310 -> 3236, 32 experts x 1024 rows 2190 -> 2110).
-        struct Tile {
-            int off, cnt, trow0, n_tile;               // the expert's first sorted row and row count; first row of this CTA inside it
-        } cur, nxt;
-        auto open_tile = [&](int tile, Tile& x) {
-            int e, m_tile;
-            locate(tile, e, m_tile, x.n_tile, x.cnt);
-            x.off = p.offsets[e];
-            x.trow0 = m_tile * TM + (int)crank * BM;
-        };
-        uint32_t gsc = 0;                                     // K blocks since the kernel started
-        if (walker < total_tiles) open_tile(walker, nxt);
-        for (int tile = walker; tile < total_tiles; tile += pair_count) {
-            cur = nxt;
-            const int n_tile = cur.n_tile, cnt = cur.cnt, trow0 = cur.trow0;
-            const long long grow = (long long)cur.off + trow0 + row;              // sorted row
+        uint32_t gsc = 0, tiles_done = 0;                     // K blocks, tiles since the kernel started
+        for (int tile = walker; tile < total_tiles; tile += pair_count, tiles_done++) {
+            // Where the tile lies comes with the scales of its first K block: looked up here, it took 1200 - 2500 cycles of the gap
+            // between two tiles.
+            if (!warp_wait(&sm->tmem_full[acc], acc_ph)) goto done;
+            const int4 at = tile_at[tiles_done % SC_RING];
+            const int off = at.x, cnt = at.y, trow0 = at.z, n_tile = at.w;        // trow0: first row of this CTA inside the expert
+            const long long grow = (long long)off + trow0 + row;                  // sorted row
             const bool row_ok = (trow0 + row) < cnt;
             const bool warp_valid = (trow0 + (warp & 3) * 32) < cnt;              // any valid row in this warp's 32
             const float row_weight = (MODE != 1 && row_ok) ? p.row_w[grow] : 0.0f;     // used by the epilogue
@@ -596,7 +587,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
             for (int i = 0; i < QCOLS; i++) accv[i] = 0.0f;
 
             for (int kb = 0; kb < nkb; kb++, gsc++) {
-                if (!warp_wait(&sm->tmem_full[acc], acc_ph)) goto done;
+                if (kb > 0 && !warp_wait(&sm->tmem_full[acc], acc_ph)) goto done;
 #ifdef B200_GEMM_TRACE
                 if (trw) TRACE_STAMP(3, gp);
 #endif
@@ -640,8 +631,6 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
             if (trw) TRACE_STAMP(7, gp / nkb - 1);     // end of the main loop of each tile; epilogue follows
 #endif
 
-            if (tile + pair_count < total_tiles) open_tile(tile + pair_count, nxt);
-
             if (MODE == 1) {
                 // SwiGLU on 32 activation columns, 1x128 requantisation shared with the three other quarters.
                 // Fast exp / reciprocal: the result is rounded to e4m3 next, an ulp of fp32 does not matter.
@@ -678,6 +667,18 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                     if (wq == 0) p.act_s[grow * p.s_rs + n_tile * p.s_ks] = scale;
                 }
                 tile_par ^= 1;
+            } else if (warp_valid && cnt - (trow0 + (warp & 3) * 32) <= DIRECT_ROWS) {
+                // A decode batch's few rows: each lane adds its own row (a row is a cache line per instruction, so 32 of them would
+                // be slower than the transpose below; 1 or 2 rows take 700 cycles instead of 3700)
+                if (row_ok) {
+                    float* const dst = p.out + (size_t)(MODE == 2 ? row_token : grow) * p.D + n_tile * 256 + wq * QCOLS;
+#pragma unroll
+                    for (int i = 0; i < QCOLS; i += 4) {
+                        const float4 x = make_float4(row_weight * accv[i], row_weight * accv[i + 1], row_weight * accv[i + 2], row_weight * accv[i + 3]);
+                        if (MODE == 2) red_add_v4(dst + i, x.x, x.y, x.z, x.w);
+                        else *reinterpret_cast<float4*>(dst + i) = x;
+                    }
+                }
             } else if (warp_valid) {
                 // The accumulator row of a lane is transposed through shared memory SW columns at a time so that
                 // one store / red instruction covers 32 / SEGS rows x 16 SEGS contiguous bytes instead of 32 rows
@@ -688,7 +689,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                 const int sub_row = lane / SEGS, seg = lane % SEGS;
                 const int tok = row_token;
                 // MODE 2: out[token] += w * acc.  MODE 3: rows[sorted row] = w * acc (plain stores).
-                const long long grow0 = (long long)cur.off + trow0 + (warp & 3) * 32;
+                const long long grow0 = (long long)off + trow0 + (warp & 3) * 32;
                 const int rows_ok = min(32, cnt - (trow0 + (warp & 3) * 32));
                 float* const out_col = p.out + n_tile * 256 + wq * QCOLS;
 #pragma unroll
