@@ -260,6 +260,21 @@ __device__ __forceinline__ void scan_tiles(GemmSmem* sm, int E) {
     }
 }
 
+// The GEMMs are launched programmatically, GEMM1 behind the sort, GEMM2 behind GEMM1.  The offsets are the sort's: GEMM1 waits for it
+// before it reads them.  GEMM2 starts only when every CTA of GEMM1 has passed that wait, so it may read the offsets, and fetch
+// weights, while GEMM1 drains; whoever touches GEMM1's results or the output waits with wait_for_gemm1 first.
+template <int MODE>
+__device__ __forceinline__ void wait_for_sort() {
+    if (MODE == 1) {
+        ptx::grid_wait();
+        ptx::grid_release();
+    }
+}
+template <int MODE>
+__device__ __forceinline__ void wait_for_gemm1() {
+    if (MODE != 1) ptx::grid_wait();
+}
+
 // The rows of an A tile that exist, in whole groups of 32 (what a promotion warp owns): a decode batch has a few rows
 // per expert, and a full box of 128 would bring the next experts' rows along, a third of the stage's bytes.  The rows of
 // the stage that are not loaded hold older bytes; their products go to accumulator rows that nobody reads.
@@ -341,7 +356,6 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         sm->abort_flag = 0;
         ptx::fence_mbar_init();
     }
-    count_tiles(sm, p, TM, NT);
     if (warp == W_MMA0) {
         if (PAIR) { tmem_alloc2(&sm->tmem_base, 512); tmem_relinquish2(); }
         else      { ptx::tmem_alloc(&sm->tmem_base, 512); ptx::tmem_relinquish(); }
@@ -351,6 +365,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         ptx::prefetch_tensormap(&tmap_a32);
         ptx::prefetch_tensormap(&tmap_b);
     }
+    wait_for_sort<MODE>();
+    count_tiles(sm, p, TM, NT);
     ptx::tc_fence_before();
     scan_tiles(sm, p.E);
     __syncthreads();
@@ -395,19 +411,14 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                 const int row0 = ptx::uniform(p.offsets[e]) + m_tile * TM + (int)crank * BM;
                 const uint32_t a_bytes = a_tile_bytes(cnt - m_tile * TM);
                 const long long wrow0 = (long long)e * w_rows;
-                for (int kb = 0; kb < nkb; kb++) {
-                    if (!ptx::whole_warp(ptx::mbar_wait_relaxed(&sm->empty[s], ph ^ 1, abort_flag, PRODUCER_SLEEP_NS))) goto done;
-                    TRACE_STAMP(6, gk); gk++;
-                    uint8_t* a_dst = tiles + (size_t)s * STAGE_BYTES;
-                    uint8_t* b_dst = a_dst + A_BYTES;
-                    if (!ptx::elect_one()) {
-                        // (the elected lane alone issues the loads)
-                    } else if (PAIR) {
-                        // this CTA's 128 rows of A and its half of the weight tile (accumulator columns
-                        // 128 crank .. +127); the bytes are counted on the leader's barrier
-                        const uint32_t fbar = map_to_cta(&sm->full[s], 0);
+                auto load_b = [&](int kb, int st) {              // expects the whole stage
+                    uint8_t* b_dst = tiles + (size_t)st * STAGE_BYTES + A_BYTES;
+                    if (!ptx::elect_one()) return;
+                    if (PAIR) {
+                        // this CTA's half of the weight tile (accumulator columns 128 crank .. +127); the bytes are counted on the
+                        // leader's barrier
+                        const uint32_t fbar = map_to_cta(&sm->full[st], 0);
                         mbar_expect_tx_cluster(fbar, A_BYTES + B_BYTES / 2);
-                        tma_load_2d_pair(a_dst, &tmap_a, fbar, kb * BK, row0);
                         if (p.packed) {
                             tma_load_2d_pair(b_dst, &tmap_b, fbar, 0, (((e * NT + n_tile) * nkb) + kb) * BN + (int)crank * 128);
                         } else if (MODE == 1) {
@@ -417,22 +428,39 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                         } else {
                             tma_load_2d_pair(b_dst, &tmap_b, fbar, kb * BK, (int)(wrow0 + n_tile * 256 + 128 * (int)crank));
                         }
-                    } else {
-                        ptx::mbar_expect_tx(&sm->full[s], a_bytes + B_BYTES);
-                        load_a_rows(a_dst, &tmap_a, &tmap_a32, &sm->full[s], kb * BK, row0, a_bytes);
-                        if (p.packed) {
-                            // the tile's K block is one contiguous 32 KB piece of the packed weights
-                            ptx::tma_load_2d(b_dst, &tmap_b, &sm->full[s], 0, (((e * NT + n_tile) * nkb) + kb) * BN);
-                        } else if (MODE == 1) {
-                            // 2 NQ boxes of QCOLS/2 weight rows: group g = [gate j0 + g QCOLS/2 .. | up j0 + g QCOLS/2 ..]
-                            const int j0 = n_tile * 128;
+                        return;
+                    }
+                    ptx::mbar_expect_tx(&sm->full[st], a_bytes + B_BYTES);
+                    if (p.packed) {
+                        // the tile's K block is one contiguous 32 KB piece of the packed weights
+                        ptx::tma_load_2d(b_dst, &tmap_b, &sm->full[st], 0, (((e * NT + n_tile) * nkb) + kb) * BN);
+                    } else if (MODE == 1) {
+                        // 2 NQ boxes of QCOLS/2 weight rows: group g = [gate j0 + g QCOLS/2 .. | up j0 + g QCOLS/2 ..]
+                        const int j0 = n_tile * 128;
 #pragma unroll
-                            for (int bx = 0; bx < 2 * NQ; bx++)
-                                ptx::tma_load_2d(b_dst + bx * (QCOLS / 2) * 128, &tmap_b, &sm->full[s], kb * BK,
-                                                 (int)(wrow0 + ((bx & 1) ? p.I : 0) + j0 + (QCOLS / 2) * (bx >> 1)));
-                        } else {
-                            ptx::tma_load_2d(b_dst, &tmap_b, &sm->full[s], kb * BK, (int)(wrow0 + n_tile * 256));
-                        }
+                        for (int bx = 0; bx < 2 * NQ; bx++)
+                            ptx::tma_load_2d(b_dst + bx * (QCOLS / 2) * 128, &tmap_b, &sm->full[st], kb * BK,
+                                             (int)(wrow0 + ((bx & 1) ? p.I : 0) + j0 + (QCOLS / 2) * (bx >> 1)));
+                    } else {
+                        ptx::tma_load_2d(b_dst, &tmap_b, &sm->full[st], kb * BK, (int)(wrow0 + n_tile * 256));
+                    }
+                };
+                int ready = 0;                                   // K blocks whose weights have been requested
+                if (MODE != 1 && tile == walker) {
+                    for (; ready < min(nkb, STAGES); ready++) load_b(ready, ready);
+                    wait_for_gemm1<MODE>();
+                }
+                for (int kb = 0; kb < nkb; kb++) {
+                    if (kb >= ready) {
+                        if (!ptx::whole_warp(ptx::mbar_wait_relaxed(&sm->empty[s], ph ^ 1, abort_flag, PRODUCER_SLEEP_NS))) goto done;
+                        TRACE_STAMP(6, gk);
+                        load_b(kb, s);
+                    }
+                    gk++;
+                    if (ptx::elect_one()) {
+                        uint8_t* a_dst = tiles + (size_t)s * STAGE_BYTES;
+                        if (PAIR) tma_load_2d_pair(a_dst, &tmap_a, map_to_cta(&sm->full[s], 0), kb * BK, row0);
+                        else      load_a_rows(a_dst, &tmap_a, &tmap_a32, &sm->full[s], kb * BK, row0, a_bytes);
                     }
                     if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
@@ -490,6 +518,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         // longer than a K block: it held the warps back by different amounts, and the last one sets the pace.
         const int nkb_w = Kdim / 128;
         uint32_t g = 0, tiles_done = 0;                     // K blocks, tiles since the kernel started
+        wait_for_gemm1<MODE>();
         for (int tile = walker; tile < total_tiles; tile += pair_count, tiles_done++) {
             int e, m_tile, n_tile, cnt;
             locate(tile, e, m_tile, n_tile, cnt);
@@ -571,6 +600,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
             else                    ptx::mbar_arrive(&sm->tmem_empty[a]);
         };
         uint32_t gsc = 0, tiles_done = 0;                     // K blocks, tiles since the kernel started
+        wait_for_gemm1<MODE>();
         for (int tile = walker; tile < total_tiles; tile += pair_count, tiles_done++) {
             // Where the tile lies comes with the scales of its first K block: looked up here, it took 1200 - 2500 cycles of the gap
             // between two tiles.
@@ -779,13 +809,14 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         sm->abort_flag = 0;
         ptx::fence_mbar_init();
     }
-    count_tiles(sm, p, BM, NT);
     if (warp == W_MMA0) { ptx::tmem_alloc(&sm->tmem_base, 512); ptx::tmem_relinquish(); }
     if (warp == W_TMA && lane == 0) {
         ptx::prefetch_tensormap(&tmap_a);
         ptx::prefetch_tensormap(&tmap_a32);
         ptx::prefetch_tensormap(&tmap_b);
     }
+    wait_for_sort<MODE>();
+    count_tiles(sm, p, BM, NT);
     ptx::tc_fence_before();
     scan_tiles(sm, p.E);
     __syncthreads();
@@ -833,25 +864,34 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                 const int row0 = ptx::uniform(p.offsets[e]) + m_tile * BM;
                 const uint32_t a_bytes = a_tile_bytes(cnt - m_tile * BM);
                 const long long wrow0 = (long long)e * w_rows;
-                for (int kb = 0; kb < nkb; kb++) {
-                    if (!ptx::whole_warp(ptx::mbar_wait_relaxed(&sm->empty[s], ph ^ 1, abort_flag, PRODUCER_SLEEP_NS))) goto done;
-                    uint8_t* a_dst = tiles + (size_t)s * STAGE_BYTES;
-                    uint8_t* b_dst = a_dst + A_BYTES;
-                    if (ptx::elect_one()) {
-                        ptx::mbar_expect_tx(&sm->full[s], a_bytes + B_BYTES);
-                        load_a_rows(a_dst, &tmap_a, &tmap_a32, &sm->full[s], kb * BK, row0, a_bytes);
-                        if (p.packed) {
-                            ptx::tma_load_2d(b_dst, &tmap_b, &sm->full[s], 0, (((e * NT + n_tile) * nkb) + kb) * BN);
-                        } else if (MODE == 1) {
-                            const int j0 = n_tile * 128;
+                auto load_b = [&](int kb, int st) {              // expects the whole stage
+                    uint8_t* b_dst = tiles + (size_t)st * STAGE_BYTES + A_BYTES;
+                    if (!ptx::elect_one()) return;
+                    ptx::mbar_expect_tx(&sm->full[st], a_bytes + B_BYTES);
+                    if (p.packed) {
+                        ptx::tma_load_2d(b_dst, &tmap_b, &sm->full[st], 0, (((e * NT + n_tile) * nkb) + kb) * BN);
+                    } else if (MODE == 1) {
+                        const int j0 = n_tile * 128;
 #pragma unroll
-                            for (int bx = 0; bx < 2 * NQ; bx++)
-                                ptx::tma_load_2d(b_dst + bx * (QCOLS / 2) * 128, &tmap_b, &sm->full[s], kb * BK,
-                                                 (int)(wrow0 + ((bx & 1) ? p.I : 0) + j0 + (QCOLS / 2) * (bx >> 1)));
-                        } else {
-                            ptx::tma_load_2d(b_dst, &tmap_b, &sm->full[s], kb * BK, (int)(wrow0 + n_tile * 256));
-                        }
+                        for (int bx = 0; bx < 2 * NQ; bx++)
+                            ptx::tma_load_2d(b_dst + bx * (QCOLS / 2) * 128, &tmap_b, &sm->full[st], kb * BK,
+                                             (int)(wrow0 + ((bx & 1) ? p.I : 0) + j0 + (QCOLS / 2) * (bx >> 1)));
+                    } else {
+                        ptx::tma_load_2d(b_dst, &tmap_b, &sm->full[st], kb * BK, (int)(wrow0 + n_tile * 256));
                     }
+                };
+                int ready = 0;                                   // K blocks whose weights have been requested
+                if (MODE != 1 && tile == walker) {
+                    for (; ready < min(nkb, STAGES); ready++) load_b(ready, ready);
+                    wait_for_gemm1<MODE>();
+                }
+                for (int kb = 0; kb < nkb; kb++) {
+                    if (kb >= ready) {
+                        if (!ptx::whole_warp(ptx::mbar_wait_relaxed(&sm->empty[s], ph ^ 1, abort_flag, PRODUCER_SLEEP_NS))) goto done;
+                        load_b(kb, s);
+                    }
+                    if (ptx::elect_one())
+                        load_a_rows(tiles + (size_t)s * STAGE_BYTES, &tmap_a, &tmap_a32, &sm->full[s], kb * BK, row0, a_bytes);
                     if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
             }
@@ -895,6 +935,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         // ===================== scale factors of every stage =====================
         int s = 0; uint32_t ph = 0;
         uint32_t bad = 0;
+        wait_for_gemm1<MODE>();
         auto expo = [&](float f) -> uint32_t {
             const uint32_t b = __float_as_uint(f);
             bad |= (b & 0x807FFFFFu) | (((b >> 23) == 0u) ? 1u : 0u);     // sign, mantissa bits, zero / denormal
@@ -962,6 +1003,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
         uint32_t fph = 0;
         int tile_par = 0; uint32_t amax_ph[2] = {0, 0};
+        wait_for_gemm1<MODE>();
         for (int tile = walker; tile < total_tiles; tile += walkers) {
             int e, m_tile, n_tile, cnt;
             locate(tile, e, m_tile, n_tile, cnt);
@@ -1379,9 +1421,11 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
         cudaLaunchConfig_t lc = {};
         lc.gridDim = dim3(grid); lc.blockDim = dim3(GEMM_THREADS); lc.stream = stream;
         lc.dynamicSmemBytes = mx ? GEMM_MX_SMEM_BYTES : GEMM_SMEM_BYTES;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = 2; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
 #ifndef B200_GEMM_CLUSTER2
 #define B200_GEMM_CLUSTER2 1
 #endif
@@ -1389,7 +1433,7 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
         // an expert's weight slab when it has 129..256 rows) then run on SMs of one GPC, behind the same L2
         // partition, and the slab comes from DRAM once instead of once per die.
         const bool cluster2 = pair || (B200_GEMM_CLUSTER2 && grid % 2 == 0);
-        lc.attrs = attr; lc.numAttrs = cluster2 ? 1 : 0;
+        lc.attrs = attr; lc.numAttrs = cluster2 ? 2 : 1;
         cudaError_t err;
         if (mx) {
             if (mode == 1)      err = cudaLaunchKernelEx(&lc, grouped_gemm_mx_kernel<1>, ta, ta32, tb, p);
