@@ -574,15 +574,9 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     } else {
         // ===================== promotion + epilogue (warps 0-15) =====================
         ptx::setmaxnreg_inc<PROMO_REGS>();
-        // one lane polls the barrier, the warp follows (hundreds of pollers and arrivals per K block on
-        // one shared-memory word cost more than the promotion itself)
-        auto warp_wait = [&](uint64_t* bar, uint32_t parity) -> bool {
-            int ok = 1;
-            if (lane == 0) ok = ptx::mbar_wait(bar, parity, abort_flag) ? 1 : 0;
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            __syncwarp();
-            return ok != 0;
-        };
+        // The warp polls as one instruction (one lane that polls and tells the others costs a shuffle and a reconvergence per K
+        // block: 32 experts x 1024 rows 2169 -> 2092 us, T = 4096 3130 -> 3036, T = 16 765 -> 748).
+        auto warp_wait = [&](uint64_t* bar, uint32_t parity) -> bool { return ptx::whole_warp(ptx::mbar_wait(bar, parity, abort_flag)); };
         const int wq = warp >> 2;                         // column group of the accumulator
         const int row = (warp & 3) * 32 + lane;           // TMEM lane = tile row
         const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
@@ -838,14 +832,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         n_tile = local / mt;
         m_tile = local - n_tile * mt;
     };
-    // one lane polls the barrier, the warp follows
-    auto warp_wait = [&](uint64_t* bar, uint32_t parity) -> bool {
-        int ok = 1;
-        if (lane == 0) ok = ptx::mbar_wait(bar, parity, abort_flag) ? 1 : 0;
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        __syncwarp();
-        return ok != 0;
-    };
+    auto warp_wait = [&](uint64_t* bar, uint32_t parity) -> bool { return ptx::whole_warp(ptx::mbar_wait(bar, parity, abort_flag)); };
 
     if (warp >= NUM_PROMO_WARPS) {
         ptx::setmaxnreg_dec<AUX_REGS>();
