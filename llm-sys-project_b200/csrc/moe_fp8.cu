@@ -480,16 +480,17 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
             for (int tile = walker; tile < total_tiles; tile += pair_count) {
                 for (int kb = 0; kb < nkb; kb++, g++) {
                     if ((int)(g & 1) == role) {
+                        // The operands first: they are there long before the stage is handed back, which starts the critical path.
                         // (waits on barriers that the peer CTA or tcgen05.commit signal need no cluster-scope
                         // acquire: what they hand over is a TMEM stage or TMA-written tiles, not memory data)
-                        if (!ptx::whole_warp(ptx::mbar_wait(&sm->tmem_empty[role], acc_ph ^ 1, abort_flag))) goto done;
-                        TRACE_STAMP(0, g);
                         if (!ptx::whole_warp(ptx::mbar_wait(&sm->full[s], ph, abort_flag))) goto done;
-                        TRACE_STAMP(1, g);
-                        ptx::tc_fence_after();
+                        TRACE_STAMP(0, g);
                         const uint32_t a_addr = ptx::smem_u32(tiles + (size_t)s * STAGE_BYTES);
                         const uint64_t ad = ptx::make_smem_desc(a_addr, 16, 1024, 2), bd = ptx::make_smem_desc(a_addr + A_BYTES, 16, 1024, 2);
                         const uint32_t d_tmem = tmem_base + role * BN;
+                        if (!ptx::whole_warp(ptx::mbar_wait(&sm->tmem_empty[role], acc_ph ^ 1, abort_flag))) goto done;
+                        TRACE_STAMP(1, g);
+                        ptx::tc_fence_after();
                         if (ptx::elect_one()) {
 #pragma unroll
                             for (int k4 = 0; k4 < 4; k4++) {        // 32 bytes further along K: 2 in the descriptor's 16-byte units
@@ -497,11 +498,11 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                                 else      ptx::mma_f8(d_tmem, ad + 2 * k4, bd + 2 * k4, idesc, k4 > 0 ? 1u : 0u);
                             }
                             if (PAIR) {
-                                commit_both(&sm->empty[s]);
                                 commit_both(&sm->tmem_full[role]);
+                                commit_both(&sm->empty[s]);
                             } else {
-                                ptx::tc_commit(&sm->empty[s]);          // smem stage reusable once the MMAs have read it
                                 ptx::tc_commit(&sm->tmem_full[role]);   // partial sums ready for promotion
+                                ptx::tc_commit(&sm->empty[s]);          // smem stage reusable once the MMAs have read it
                             }
                         }
                         TRACE_STAMP(2, g);
