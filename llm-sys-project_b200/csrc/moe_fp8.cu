@@ -275,18 +275,26 @@ __device__ __forceinline__ void wait_for_gemm1() {
     if (MODE != 1) ptx::grid_wait();
 }
 
-// The rows of an A tile that exist, in whole groups of 32 (what a promotion warp owns): a decode batch has a few rows
-// per expert, and a full box of 128 would bring the next experts' rows along, a third of the stage's bytes.  The rows of
-// the stage that are not loaded hold older bytes; their products go to accumulator rows that nobody reads.
-// E = 256, K = 8, D = 7168 layer: T = 1 129 -> 116 us, T = 333 2105 -> 2065 us; equal where the experts are full.
-__device__ __forceinline__ uint32_t a_tile_bytes(int rows) { return rows > BM - 32 ? (uint32_t)A_BYTES : (uint32_t)((rows + 31) >> 5) * 32u * BK; }
-__device__ __forceinline__ void load_a_rows(uint8_t* dst, const CUtensorMap* map128, const CUtensorMap* map32, uint64_t* bar, int x,
-                                            int row0, uint32_t bytes) {
+// The rows of an A tile that exist, in whole groups of eight: a decode batch has a few rows per expert, and a full box of 128
+// would bring the next experts' rows along, a third of the stage's bytes.  The rows of the stage that are not loaded hold
+// zeros until a fuller tile has been there (clear_a_tiles), then older bytes; their products go to accumulator rows that
+// nobody reads, but multiplying zeros takes less power, and under sustained load power is what sets the clock.  Groups
+// of 32 and no zeros: T = 16 748 us, T = 333 1950 us, T = 1024 2024 us; with zeros 733, 1904, 1985.
+__device__ __forceinline__ uint32_t a_tile_bytes(int rows) { return rows > BM - 8 ? (uint32_t)A_BYTES : (uint32_t)((rows + 7) >> 3) * 8u * BK; }
+__device__ __forceinline__ void load_a_rows(uint8_t* dst, const CUtensorMap* map128, const CUtensorMap* map32, const CUtensorMap* map8, uint64_t* bar,
+                                            int x, int row0, uint32_t bytes) {
     if (bytes == A_BYTES) {
         ptx::tma_load_2d(dst, map128, bar, x, row0);
     } else {
-        for (uint32_t o = 0; o < bytes; o += 32 * BK) ptx::tma_load_2d(dst + o, map32, bar, x, row0 + (int)(o / BK));
+        uint32_t o = 0;
+        for (; o + 32 * BK <= bytes; o += 32 * BK) ptx::tma_load_2d(dst + o, map32, bar, x, row0 + (int)(o / BK));
+        for (; o < bytes; o += 8 * BK) ptx::tma_load_2d(dst + o, map8, bar, x, row0 + (int)(o / BK));
     }
+}
+__device__ __forceinline__ void clear_a_tiles(uint8_t* tiles) {
+    for (int i = threadIdx.x; i < STAGES * A_BYTES / 16; i += GEMM_THREADS)
+        *reinterpret_cast<uint4*>(tiles + (size_t)(i / (A_BYTES / 16)) * STAGE_BYTES + (i % (A_BYTES / 16)) * 16) = make_uint4(0, 0, 0, 0);
+    ptx::fence_proxy_async_smem();
 }
 // acc[0..N-1] += v[0..N-1] * s, two columns per instruction (the same bits as N fmaf in half the issue slots: with the scales out
 // of the loop T = 4096 3576 -> 3449 us, 32 experts x 1024 rows 2245 -> 2180 us)
@@ -323,7 +331,7 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[N]) {
 template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_a32,
-                        const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
+                        const __grid_constant__ CUtensorMap tmap_a8, const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
     constexpr int TM = PAIR ? 2 * BM : BM;        // rows of a tile
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -363,8 +371,10 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     if (warp == W_TMA && lane == 0) {
         ptx::prefetch_tensormap(&tmap_a);
         ptx::prefetch_tensormap(&tmap_a32);
+        ptx::prefetch_tensormap(&tmap_a8);
         ptx::prefetch_tensormap(&tmap_b);
     }
+    clear_a_tiles(tiles);
     wait_for_sort<MODE>();
     count_tiles(sm, p, TM, NT);
     ptx::tc_fence_before();
@@ -460,7 +470,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                     if (ptx::elect_one()) {
                         uint8_t* a_dst = tiles + (size_t)s * STAGE_BYTES;
                         if (PAIR) tma_load_2d_pair(a_dst, &tmap_a, map_to_cta(&sm->full[s], 0), kb * BK, row0);
-                        else      load_a_rows(a_dst, &tmap_a, &tmap_a32, &sm->full[s], kb * BK, row0, a_bytes);
+                        else      load_a_rows(a_dst, &tmap_a, &tmap_a32, &tmap_a8, &sm->full[s], kb * BK, row0, a_bytes);
                     }
                     if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
@@ -774,7 +784,7 @@ done:
 template <int MODE>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_a32,
-                       const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
+                       const __grid_constant__ CUtensorMap tmap_a8, const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
     static_assert(NUM_PROMO_WARPS == 8, "the block-scaled kernel is written for eight epilogue warps");
     constexpr int W_SF = W_MMA0 + 1;
     extern __shared__ uint8_t smem_raw[];
@@ -808,8 +818,10 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     if (warp == W_TMA && lane == 0) {
         ptx::prefetch_tensormap(&tmap_a);
         ptx::prefetch_tensormap(&tmap_a32);
+        ptx::prefetch_tensormap(&tmap_a8);
         ptx::prefetch_tensormap(&tmap_b);
     }
+    clear_a_tiles(tiles);
     wait_for_sort<MODE>();
     count_tiles(sm, p, BM, NT);
     ptx::tc_fence_before();
@@ -879,7 +891,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                         load_b(kb, s);
                     }
                     if (ptx::elect_one())
-                        load_a_rows(tiles + (size_t)s * STAGE_BYTES, &tmap_a, &tmap_a32, &sm->full[s], kb * BK, row0, a_bytes);
+                        load_a_rows(tiles + (size_t)s * STAGE_BYTES, &tmap_a, &tmap_a32, &tmap_a8, &sm->full[s], kb * BK, row0, a_bytes);
                     if (++s == STAGES) { s = 0; ph ^= 1; }
                 }
             }
@@ -1405,7 +1417,7 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
     if ((cfg->flags & B200_MOE_SINGLE_CTA_TILES) || mx) pair = false;
     if (ws->sm_count < 2) pair = false;
     const unsigned grid = pair ? (unsigned)(ws->sm_count / 2) * 2 : (unsigned)ws->sm_count;
-    auto launch = [&](int mode, const CUtensorMap& ta, const CUtensorMap& ta32, const CUtensorMap& tb, const GemmParams& p) -> int {
+    auto launch = [&](int mode, const CUtensorMap& ta, const CUtensorMap& ta32, const CUtensorMap& ta8, const CUtensorMap& tb, const GemmParams& p) -> int {
         cudaLaunchConfig_t lc = {};
         lc.gridDim = dim3(grid); lc.blockDim = dim3(GEMM_THREADS); lc.stream = stream;
         lc.dynamicSmemBytes = mx ? GEMM_MX_SMEM_BYTES : GEMM_SMEM_BYTES;
@@ -1424,24 +1436,24 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
         lc.attrs = attr; lc.numAttrs = cluster2 ? 2 : 1;
         cudaError_t err;
         if (mx) {
-            if (mode == 1)      err = cudaLaunchKernelEx(&lc, grouped_gemm_mx_kernel<1>, ta, ta32, tb, p);
-            else if (mode == 2) err = cudaLaunchKernelEx(&lc, grouped_gemm_mx_kernel<2>, ta, ta32, tb, p);
-            else                err = cudaLaunchKernelEx(&lc, grouped_gemm_mx_kernel<3>, ta, ta32, tb, p);
+            if (mode == 1)      err = cudaLaunchKernelEx(&lc, grouped_gemm_mx_kernel<1>, ta, ta32, ta8, tb, p);
+            else if (mode == 2) err = cudaLaunchKernelEx(&lc, grouped_gemm_mx_kernel<2>, ta, ta32, ta8, tb, p);
+            else                err = cudaLaunchKernelEx(&lc, grouped_gemm_mx_kernel<3>, ta, ta32, ta8, tb, p);
         } else if (pair) {
-            if (mode == 1)      err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<1, true>, ta, ta32, tb, p);
-            else if (mode == 2) err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<2, true>, ta, ta32, tb, p);
-            else                err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<3, true>, ta, ta32, tb, p);
+            if (mode == 1)      err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<1, true>, ta, ta32, ta8, tb, p);
+            else if (mode == 2) err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<2, true>, ta, ta32, ta8, tb, p);
+            else                err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<3, true>, ta, ta32, ta8, tb, p);
         } else {
-            if (mode == 1)      err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<1, false>, ta, ta32, tb, p);
-            else if (mode == 2) err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<2, false>, ta, ta32, tb, p);
-            else                err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<3, false>, ta, ta32, tb, p);
+            if (mode == 1)      err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<1, false>, ta, ta32, ta8, tb, p);
+            else if (mode == 2) err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<2, false>, ta, ta32, ta8, tb, p);
+            else                err = cudaLaunchKernelEx(&lc, grouped_gemm_fp8_kernel<3, false>, ta, ta32, ta8, tb, p);
         }
         b200_count_launch(1);
         B200_CUDA_TRY(err);
         B200_CUDA_TRY(cudaGetLastError());
         return B200_OK;
     };
-    CUtensorMap ta, ta32, tb;
+    CUtensorMap ta, ta32, ta8, tb;
     GemmParams p{};
     p.offsets = s.offsets; p.E = E; p.D = D; p.I = I; p.status = ws->d_status; p.total_rows = TK;
 #ifdef B200_GEMM_TRACE
@@ -1451,6 +1463,7 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
     // GEMM1 (a CTA of a pair fetches half of a weight tile: boxes of 128 rows instead of 256)
     st = b200_make_tmap_u8_sw128(&ta, s.sq, (unsigned long long)TK, D, 128);
     if (!st) st = b200_make_tmap_u8_sw128(&ta32, s.sq, (unsigned long long)TK, D, 32);
+    if (!st) st = b200_make_tmap_u8_sw128(&ta8, s.sq, (unsigned long long)TK, D, 8);
     if (st) return st;
     p.packed = packed ? 1 : 0;
     if (packed) st = b200_make_tmap_u8_sw128(&tb, w1q, (unsigned long long)E * 2 * I * (D / 128), 128, pair ? 128 : 256);
@@ -1460,7 +1473,7 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
     p.a_scale = s.ss; p.a_ks = TK; p.w_scale = w1s; p.act_q = s.act_q; p.act_s = s.act_s;
     p.s_rs = do_gemm2 ? 1 : I / 128; p.s_ks = do_gemm2 ? TK : 1;
     if (prof) B200_CUDA_TRY(cudaEventRecord(prof->ev[slot][0], stream));
-    st = launch(1, ta, ta32, tb, p);
+    st = launch(1, ta, ta32, ta8, tb, p);
     if (st) return st;
     if (prof) B200_CUDA_TRY(cudaEventRecord(prof->ev[slot][1], stream));
     if (!do_gemm2) return B200_OK;
@@ -1468,6 +1481,7 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
     // GEMM2
     st = b200_make_tmap_u8_sw128(&ta, s.act_q, (unsigned long long)TK, I, 128);
     if (!st) st = b200_make_tmap_u8_sw128(&ta32, s.act_q, (unsigned long long)TK, I, 32);
+    if (!st) st = b200_make_tmap_u8_sw128(&ta8, s.act_q, (unsigned long long)TK, I, 8);
     if (st) return st;
     if (packed) st = b200_make_tmap_u8_sw128(&tb, w2q, (unsigned long long)E * D * (I / 128), 128, pair ? 128 : 256);
     else        st = b200_make_tmap_u8_sw128(&tb, w2q, (unsigned long long)E * D, I, pair ? 128 : 256);
@@ -1479,7 +1493,7 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
     if (det) {
         p.out = s.rows;
         if (prof) B200_CUDA_TRY(cudaEventRecord(prof->ev[slot][2], stream));
-        st = launch(3, ta, ta32, tb, p);
+        st = launch(3, ta, ta32, ta8, tb, p);
         if (st) return st;
         reduce_rows_kernel<<<T, 256, 0, stream>>>(s.rows, s.pair_row, ids, K, D, out);
         if (prof) { B200_CUDA_TRY(cudaEventRecord(prof->ev[slot][3], stream)); prof->calls++; }
@@ -1490,7 +1504,7 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
     p.out = out;
     if (late) B200_CUDA_TRY(cudaMemsetAsync(out, 0, out_bytes, stream));
     if (prof) B200_CUDA_TRY(cudaEventRecord(prof->ev[slot][2], stream));
-    st = launch(2, ta, ta32, tb, p);
+    st = launch(2, ta, ta32, ta8, tb, p);
     if (st) return st;
     if (prof) { B200_CUDA_TRY(cudaEventRecord(prof->ev[slot][3], stream)); prof->calls++; }
     return B200_OK;
