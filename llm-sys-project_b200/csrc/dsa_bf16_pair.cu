@@ -11,7 +11,7 @@
 // TMEM per CTA: O 256 columns (lanes 0-63: first 128 columns of each 256-wide MMA, lanes 64-127: the
 // other 128), S 2 x 32 columns (lanes 0-63: tile rows 0-31, lanes 64-127: rows 32-63).
 // The leader CTA (cluster rank 0) issues all MMAs.  Producers and softmax threads signal barriers of their
-// own CTA only; one relay thread in the peer forwards each completed barrier to a twin in the leader
+// own CTA only; one relay warp in the peer forwards each completed barrier to a twin in the leader
 // through the cluster address space, and tcgen05.commit signals each CTA in turn.
 // Every wait is bounded.
 #include <cfloat>
@@ -488,9 +488,11 @@ done:
 
 
 // =================================================================================================
-// 128-row tiles.  tcgen05.mma has a minimum issue interval of a few tens of nanoseconds whatever its
-// shape, so the 36 K-steps of Q K^T cost the same for 64 rows as for 128: with 64-row tiles the tensor
-// pipe, not HBM, bounded the kernel.  Here a tile is 128 selected rows (N = 128 for Q K^T, eight
+// 128-row tiles.  Issued by one lane of a diverged warp, an MMA took ~45 ns whatever its shape, so the 36 K-steps of Q K^T cost the
+// same for 64 rows as for 128: with 64-row tiles the issue, not HBM, bounded the kernel.  The warp now issues as a whole (an elected
+// lane, descriptors in uniform registers; 64 queries x 2048 rows 71.8 -> 64.0 us), and what is left of a tile is the refill of its single
+// K and V stages behind the MMAs that read them.  (Handing the stages over in halves: 5 queries 19.6 -> 18.8 us, 64 queries 72.7 us, the
+// rows then come in pieces of 512 and 256 bytes.)  Here a tile is 128 selected rows (N = 128 for Q K^T, eight
 // K-steps per P V half), which leaves room for one K stage (72 KB) and one V stage (64 KB) per CTA next
 // to Q (72 KB) and P (16 KB).  The K stage refills while P V of the previous tile and the softmax run,
 // the V stage while Q K^T of the next tile runs; K and V have their own gather warps so that neither

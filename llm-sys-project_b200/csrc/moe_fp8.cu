@@ -15,15 +15,14 @@
 //                          the bit-reproducible alternative to the scatter-add.
 //
 // GEMM structure (one CTA per SM, 384 threads, tiles 128 x 256 x 128 handed out round-robin,
-// expert-major):
+// expert-major; E = 256, K = 8, D = 7168, I = 2048, a GPU that has just begun: T = 16 813 -> 733 us a call, T = 333 2070 -> 1905,
+// T = 4096 3235 -> 3010; 32 experts x 1024 rows 2095 -> 1950, before and after what the comments below measure):
 //   warp 8       TMA producer: A tile (128 rows x 128 B) and B tile (256 rows x 128 B) per
 //                K block into a 4-stage shared-memory ring (128-byte swizzle, K-major).
 //   warps 9,10   MMA issuers, one per 256-column TMEM accumulator stage (K blocks alternate between
 //                them): 4 x tcgen05.mma kind::f8f6f4 (K = 32 each) per K block, started fresh for
-//                every K block.  The issuers wait in mbarrier.try_wait (two lanes, which the
-//                hardware suspends): with 64 ns of sleep between polls they noticed a free stage ~300 cycles
-//                late, and with 200 ns the producer an empty slot (32 experts x 1024 rows 2071 -> 2044 us,
-//                T = 4096 3168 -> 3135 us).
+//                every K block.  The issuers wait in mbarrier.try_wait: with 64 ns of sleep between polls they
+//                noticed a free stage ~300 cycles late, and with 200 ns the producer an empty slot.
 //   warps 0-7    promotion + epilogue: tcgen05.ld the K block's partial sums and fold them
 //                into fp32 registers with a_scale[row,kb] * w_scale[nblk,kb] (the scales are
 //                arbitrary fp32 values, so the scaling cannot be left to the tensor core).
@@ -44,10 +43,7 @@ constexpr int STAGES = 4;
 constexpr int A_BYTES = BM * BK;            // 16384
 constexpr int B_BYTES = BN * BK;            // 32768
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-#ifndef B200_GEMM_PROMO_WARPS
-#define B200_GEMM_PROMO_WARPS 8
-#endif
-constexpr int NUM_PROMO_WARPS = B200_GEMM_PROMO_WARPS;   // 8 or 16; one barrier arrival and one polling lane per warp
+constexpr int NUM_PROMO_WARPS = 8;           // one barrier arrival per warp
 constexpr int NQ = NUM_PROMO_WARPS / 4;      // column groups of the accumulator (TMEM lanes fix the row split at 4)
 constexpr int QCOLS = BN / NQ;               // accumulator columns per promotion thread
 constexpr int GEMM_THREADS = 32 * (NUM_PROMO_WARPS + 4);   // promotion/epilogue warpgroups, then the TMA + MMA warpgroup
@@ -60,16 +56,12 @@ constexpr int DIRECT_ROWS = 8;               // GEMM2: rows of a warp up to whic
 // without bound until its request is met, so the two sides must balance:
 // promotion threads x (PROMO_REGS - LAUNCH_REGS) <= 128 x (LAUNCH_REGS - AUX_REGS).  The launcher checks
 // the compiled register count against this before the first launch.
-constexpr int LAUNCH_REGS = (NUM_PROMO_WARPS == 8) ? 168 : 96;
-constexpr int PROMO_REGS = (NUM_PROMO_WARPS == 8) ? 232 : 112;
-constexpr int AUX_REGS = (NUM_PROMO_WARPS == 8) ? 40 : 32;
+constexpr int LAUNCH_REGS = 168;
+constexpr int PROMO_REGS = 232;
+constexpr int AUX_REGS = 40;
 // columns per promotion load (two loads in flight)
-#ifndef B200_GEMM_PROMO_CH
-#define B200_GEMM_PROMO_CH ((B200_GEMM_PROMO_WARPS == 8) ? 32 : 8)
-#endif
-constexpr int CH = B200_GEMM_PROMO_CH;
-constexpr int SW = (NUM_PROMO_WARPS == 8) ? 16 : 8;     // columns per pass of the output transpose
-static_assert(NUM_PROMO_WARPS == 8 || NUM_PROMO_WARPS == 16, "promotion warps");
+constexpr int CH = 32;
+constexpr int SW = 16;                       // columns per pass of the output transpose
 static_assert(QCOLS % (2 * CH) == 0, "promotion chunks");
 static_assert(NUM_PROMO_WARPS * (PROMO_REGS - LAUNCH_REGS) <= 4 * (LAUNCH_REGS - AUX_REGS), "setmaxnreg balance");
 static_assert(GEMM_THREADS * LAUNCH_REGS <= 65536, "register file");
@@ -583,7 +575,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         }
       }
     } else {
-        // ===================== promotion + epilogue (warps 0-15) =====================
+        // ===================== promotion + epilogue (warps 0-7) =====================
         ptx::setmaxnreg_inc<PROMO_REGS>();
         // The warp polls as one instruction (one lane that polls and tells the others costs a shuffle and a reconvergence per K
         // block: 32 experts x 1024 rows 2169 -> 2092 us, T = 4096 3130 -> 3036, T = 16 765 -> 748).
@@ -785,7 +777,6 @@ template <int MODE>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_a32,
                        const __grid_constant__ CUtensorMap tmap_a8, const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
-    static_assert(NUM_PROMO_WARPS == 8, "the block-scaled kernel is written for eight epilogue warps");
     constexpr int W_SF = W_MMA0 + 1;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
