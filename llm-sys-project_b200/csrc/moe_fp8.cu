@@ -50,7 +50,7 @@ constexpr int GEMM_THREADS = 32 * (NUM_PROMO_WARPS + 4);   // promotion/epilogue
 constexpr int W_TMA = NUM_PROMO_WARPS, W_MMA0 = NUM_PROMO_WARPS + 1;
 constexpr int MAX_E = 1024;
 constexpr unsigned PRODUCER_SLEEP_NS = 40;
-constexpr int DIRECT_ROWS = 8;               // GEMM2: rows of a warp up to which each lane adds its own row
+constexpr int DIRECT_ROWS = 16;              // GEMM2: rows of a warp up to which each lane adds its own row
 // Register budgets after setmaxnreg.  The registers a warpgroup gives up are the only ones the others can
 // take (the pool is what the CTA was launched with: GEMM_THREADS x LAUNCH_REGS), and setmaxnreg.inc waits
 // without bound until its request is met, so the two sides must balance:
@@ -695,8 +695,9 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                 }
                 tile_par ^= 1;
             } else if (warp_valid && cnt - (trow0 + (warp & 3) * 32) <= DIRECT_ROWS) {
-                // A decode batch's few rows: each lane adds its own row (a row is a cache line per instruction, so 32 of them would
-                // be slower than the transpose below; 1 or 2 rows take 700 cycles instead of 3700)
+                // Few rows: each lane adds its own row.  With 1 or 2 rows that takes 700 cycles instead of 3700; a row is a cache line
+                // per instruction, so with all 32 it is no faster than the transpose below (up to 8 / 16 / 32 rows: T = 333
+                // 1888 / 1876 / 1876 us, T = 4096 2992 / 2985 / 3012, 32 experts x 1024 rows 1919 / 1915 / 1917).
                 if (row_ok) {
                     float* const dst = p.out + (size_t)(MODE == 2 ? row_token : grow) * p.D + n_tile * 256 + wq * QCOLS;
 #pragma unroll
