@@ -1,5 +1,5 @@
-"""Grouped FP8 GEMMs at the edges of their tiles: experts with chosen row counts (none, around the groups of 8, 32 and 128
-rows in which rows are loaded, added to the output and tiled), odd and single K blocks, several tiles per CTA.  Against the
+"""Grouped FP8 GEMMs at the edges of their tiles: experts with chosen row counts (none, around the groups of 8, 16,
+32 and 128 rows in which rows are loaded, added to the output and tiled), odd and single K blocks, several tiles per CTA.  Against the
 CPU emulation with the bars of the layer's tests (2e-2 relative + 1e-2 absolute)."""
 import contextlib
 
@@ -11,7 +11,7 @@ import oracle
 
 pytestmark = pytest.mark.gpu
 RTOL, ATOL = 2e-2, 1e-2
-COUNTS = [0, 1, 7, 8, 9, 31, 32, 33, 40, 0, 120, 121, 127, 128, 129, 136, 161, 257, 0]
+COUNTS = [0, 1, 7, 8, 9, 16, 17, 31, 32, 33, 40, 0, 120, 121, 127, 128, 129, 136, 161, 257, 0]
 
 
 @pytest.mark.parametrize("option", ["none", "fixed_order", "pow2"])
