@@ -1011,10 +1011,11 @@ int launch_gate_logits(const void* x, const float* xs, const float* wg, float* p
     if (fp8 && T < GT_MAX_T && few && vec && D % 128 == 0) {
         const int st = gate_tile_attr();
         if (st) return st;
-        gate_logits_fp8_tile_kernel<false><<<tiles, GT_THREADS, GT_SMEM, stream>>>(static_cast<const uint8_t*>(x), xs, wg, partials,
-                                                                                nullptr, nullptr, T, E, D, chunk);
+        // (waits before it touches memory: its launch overlaps the quantiser in front, T = 1 94.3 -> 92.0 us a layer call)
+        const cudaError_t err = b200_launch_after(gate_logits_fp8_tile_kernel<false>, tiles, GT_THREADS, GT_SMEM, stream, static_cast<const uint8_t*>(x),
+                                                  xs, wg, partials, nullptr, nullptr, T, E, D, chunk);
         b200_count_launch(1);
-        B200_CUDA_TRY(cudaGetLastError());
+        B200_CUDA_TRY(err);
         return B200_OK;
     }
     if (fp8 && vec) {

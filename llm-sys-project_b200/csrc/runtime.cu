@@ -200,6 +200,7 @@ constexpr int QA_BLOCKS = 4;
 template <bool POW2>
 __global__ void __launch_bounds__(256)
 quant_act_1x128_kernel(const float* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scales, long long total) {
+    ptx::grid_release();        // the router that usually follows is launched programmatically and waits before it reads
     const int lane = threadIdx.x & 31;
     const long long b0 = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * QA_BLOCKS;
     if (b0 >= total) return;
