@@ -164,12 +164,10 @@ __device__ __forceinline__ uint32_t map_to_cta(const void* p, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(ptx::smem_u32(p)), "r"(rank));
     return r;
 }
-// Arrival on a barrier of the pair's other CTA.  Relaxed on purpose: what the arrival hands over is a TMEM
-// stage whose reads have completed (tcgen05.wait::ld + tcgen05.fence::before_thread_sync), no memory data, and
-// a cluster-scope release would first wait for every outstanding global load of the thread (the prefetched
-// scales), which put ~1000 cycles into every K block.
+// Arrival on a barrier of the pair's other CTA: a TMEM stage whose reads have completed (tcgen05.wait::ld +
+// tcgen05.fence::before_thread_sync) and the scales that were read with it.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void mbar_expect_tx_cluster(uint32_t cluster_addr, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_addr),
