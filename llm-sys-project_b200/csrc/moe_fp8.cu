@@ -644,6 +644,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                     }
                 } else {
                     ptx::tc_fence_before();
+                    __syncwarp();                            // (every lane has read tile_at)
                     if (lane == 0) release_stage(acc);
                 }
 #ifdef B200_GEMM_TRACE

@@ -1,6 +1,7 @@
 """Grouped FP8 GEMMs at the edges of their tiles: experts with chosen row counts (none, around the groups of 8, 16,
-32 and 128 rows in which rows are loaded, added to the output and tiled), odd and single K blocks, several tiles per CTA.  Against the
-CPU emulation with the bars of the layer's tests (2e-2 relative + 1e-2 absolute)."""
+32 and 128 rows in which rows are loaded, added to the output and tiled), odd and single K blocks, GEMM2 with one K block and two
+(D = 4096) or five (D = 8192) tiles per CTA, so that the ring in which a tile's place is handed over comes round between tiles with
+full and with padded warps.  Against the CPU emulation with the bars of the layer's tests (2e-2 relative + 1e-2 absolute)."""
 import contextlib
 
 import numpy as np
@@ -16,7 +17,7 @@ COUNTS = [0, 1, 7, 8, 9, 16, 17, 31, 32, 33, 40, 0, 120, 121, 127, 128, 129, 136
 
 @pytest.mark.parametrize("option", ["none", "fixed_order", "pow2"])
 @pytest.mark.parametrize("packed", [False, True])
-@pytest.mark.parametrize("D,I", [(768, 384), (4096, 128)])
+@pytest.mark.parametrize("D,I", [(768, 384), (4096, 128), (8192, 128)])
 def test_expert_row_counts_at_tile_edges(b200, cuda, D, I, packed, option):
     rng = np.random.default_rng(D + I)
     E, K = len(COUNTS), 2
