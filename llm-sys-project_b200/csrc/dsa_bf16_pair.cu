@@ -97,35 +97,6 @@ __device__ __forceinline__ void mbar_arrive_cta(uint64_t* bar, uint32_t rank) {
         ::"r"(ptx::smem_u32(bar)), "r"(rank)
         : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(ptx::smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-    uint64_t t0 = 0;                       // the clock is read every 1024 failed polls only (see ptx::mbar_wait)
-    uint32_t it = 0;
-    while (!mbar_try_wait_cluster(bar, parity)) {
-        if (((++it) & 1023u) == 0) {
-            if (*abort_flag) return false;
-            const uint64_t now = ptx::globaltimer_ns();
-            if (t0 == 0) {
-                t0 = now;
-            } else if (now - t0 > B200_WAIT_LIMIT_NS) {
-                *abort_flag = 1;
-                return false;
-            }
-        }
-    }
-    return true;
-}
 __device__ __forceinline__ void tmem_alloc2(uint32_t* smem_dst, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ptx::smem_u32(smem_dst)),
                  "r"(ncols)
@@ -313,7 +284,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) dsa_deco
             // st.shared) and is read by the tensor core through the async proxy: fence after waiting.
             auto forward_or_wait = [&](uint64_t* peer, uint32_t par_peer) -> bool {
                 ptx::fence_proxy_async_smem();
-                if (leader) return ptx::whole_warp(mbar_wait_cluster(peer, par_peer, abort_flag));
+                if (leader) return ptx::whole_warp(ptx::mbar_wait<true>(peer, par_peer, abort_flag));
                 if (ptx::elect_one()) mbar_arrive_cta(peer, 0);
                 return true;
             };
@@ -711,7 +682,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS128, 1) dsa_d
                            p_addr = ptx::smem_u32(sP);
             auto forward_or_wait = [&](uint64_t* peer, uint32_t par_peer) -> bool {
                 ptx::fence_proxy_async_smem();
-                if (leader) return ptx::whole_warp(mbar_wait_cluster(peer, par_peer, abort_flag));
+                if (leader) return ptx::whole_warp(ptx::mbar_wait<true>(peer, par_peer, abort_flag));
                 if (ptx::elect_one()) mbar_arrive_cta(peer, 0);
                 return true;
             };

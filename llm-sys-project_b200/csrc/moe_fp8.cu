@@ -481,14 +481,14 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                 for (int kb = 0; kb < nkb; kb++, g++) {
                     if ((int)(g & 1) == role) {
                         // The operands first: they are there long before the stage is handed back, which starts the critical path.
-                        // (waits on barriers that the peer CTA or tcgen05.commit signal need no cluster-scope
-                        // acquire: what they hand over is a TMEM stage or TMA-written tiles, not memory data)
+                        // (`full` hands over TMA-written tiles.  `tmem_empty` of a pair also hands back the peer's slots of the scale
+                        // ring, which this thread passes on with the commit: it acquires at cluster scope, and so does the scale warp.)
                         if (!ptx::whole_warp(ptx::mbar_wait(&sm->full[s], ph, abort_flag))) goto done;
                         TRACE_STAMP(0, g);
                         const uint32_t a_addr = ptx::smem_u32(tiles + (size_t)s * STAGE_BYTES);
                         const uint64_t ad = ptx::make_smem_desc(a_addr, 16, 1024, 2), bd = ptx::make_smem_desc(a_addr + A_BYTES, 16, 1024, 2);
                         const uint32_t d_tmem = tmem_base + role * BN;
-                        if (!ptx::whole_warp(ptx::mbar_wait(&sm->tmem_empty[role], acc_ph ^ 1, abort_flag))) goto done;
+                        if (!ptx::whole_warp(ptx::mbar_wait<PAIR>(&sm->tmem_empty[role], acc_ph ^ 1, abort_flag))) goto done;
                         TRACE_STAMP(1, g);
                         ptx::tc_fence_after();
                         if (ptx::elect_one()) {
@@ -546,7 +546,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
             };
             auto publish = [&](float (&av)[4], float (&wv)[2], bool first) -> bool {
                 // This slot's last K block, g - 4, has been read once the MMAs of block g - 2 have run: they waited for it.
-                if (g >= 2 && !ptx::whole_warp(ptx::mbar_wait(&sm->tmem_full[g & 1], ((g >> 1) & 1) ^ 1, abort_flag))) return false;
+                if (g >= 2 && !ptx::whole_warp(ptx::mbar_wait<PAIR>(&sm->tmem_full[g & 1], ((g >> 1) & 1) ^ 1, abort_flag))) return false;
                 float (*const sc)[BM] = scales[g % SC_RING];
 #pragma unroll
                 for (int i = 0; i < 4; i++) {

@@ -1,7 +1,8 @@
-"""Grouped FP8 GEMMs at the edges of their tiles: experts with chosen row counts (none, around the groups of 8, 16,
-32 and 128 rows in which rows are loaded, added to the output and tiled), odd and single K blocks, GEMM2 with one K block and two
-(D = 4096) or five (D = 8192) tiles per CTA, so that the ring in which a tile's place is handed over comes round between tiles with
-full and with padded warps.  Against the CPU emulation with the bars of the layer's tests (2e-2 relative + 1e-2 absolute)."""
+"""Grouped FP8 GEMMs at the edges of their tiles: experts with chosen row counts (none, around the groups of 8, 16, 32, 128 and
+256 rows in which rows are loaded, added to the output and tiled), odd and single K blocks, GEMM2 with one K block and two
+(D = 4096) or five (D = 8192) tiles per CTA, five or nine per CTA pair, so that the ring in which a tile's place is handed over
+comes round between tiles with full and with padded warps.  Against the CPU emulation with the bars of the layer's tests (2e-2
+relative + 1e-2 absolute)."""
 import contextlib
 
 import numpy as np
@@ -15,7 +16,7 @@ RTOL, ATOL = 2e-2, 1e-2
 COUNTS = [0, 1, 7, 8, 9, 16, 17, 31, 32, 33, 40, 0, 120, 121, 127, 128, 129, 136, 161, 257, 0]
 
 
-@pytest.mark.parametrize("option", ["none", "fixed_order", "pow2"])
+@pytest.mark.parametrize("option", ["none", "fixed_order", "pow2", "pairs"])
 @pytest.mark.parametrize("packed", [False, True])
 @pytest.mark.parametrize("D,I", [(768, 384), (4096, 128), (8192, 128)])
 def test_expert_row_counts_at_tile_edges(b200, cuda, D, I, packed, option):
@@ -39,7 +40,7 @@ def test_expert_row_counts_at_tile_edges(b200, cuda, D, I, packed, option):
         b200.moe_fp8_pack_weights(1, w1, p1, E, D, I)
         b200.moe_fp8_pack_weights(2, w2, p2, E, D, I)
         w1, w2, run = p1, p2, b200.moe_fp8_experts_packed
-    flags = {"none": 0, "fixed_order": b200.MOE_DETERMINISTIC, "pow2": b200.MOE_POW2_SCALES}[option]
+    flags = {"none": 0, "fixed_order": b200.MOE_DETERMINISTIC, "pow2": b200.MOE_POW2_SCALES, "pairs": b200.MOE_CTA_PAIR_TILES}[option]
     cfg = b200.MoeFp8Config(T, E, K, D, I, b200.SCORE_SIGMOID_GROUPED, 1, 1, 1.0, flags)
     out = torch.full((T, D), float("nan"), dtype=torch.float32, device=cuda)
     run(dev(xq), dev(xs), dev(ids), dev(wts), w1, dev(w1s), w2, dev(w2s), out, cfg)
