@@ -341,9 +341,9 @@ def test_small_batch_router_bits(b200, cuda, T, E, D):
 @pytest.mark.parametrize("packed", [False, True])
 @pytest.mark.parametrize("pow2", [False, True])
 def test_row_groups_of_the_token_tiles(b200, cuda, counts, packed, pow2):
-    """Row counts at the edges of the 32-row groups that a tile loads and of the 128-row tiles, experts without rows, an
-    odd number of column tiles and of K blocks; both weight layouts, both scale rules and both combines; eight active
-    experts of 28 GEMM2 tiles give some CTAs a second tile (opened in front of the first one's epilogue)."""
+    """Row counts at the edges of the 32 rows of a promotion warp (loaded in groups of eight) and of the 128-row tiles, experts
+    without rows, an odd number of column tiles and of K blocks; both weight layouts, both scale rules and both combines; eight active
+    experts of 28 GEMM2 tiles give some CTAs a second tile (whose place comes with the scales of its first K block)."""
     rng = np.random.default_rng(sum(counts))
     E, T, I = len(counts), sum(counts), 384
     D = 7168 if E > 8 else 1280

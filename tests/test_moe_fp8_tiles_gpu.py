@@ -1,7 +1,8 @@
 """Grouped FP8 GEMMs at the edges of their tiles: experts with chosen row counts (none, around the groups of 8, 16, 32, 128 and
 256 rows in which rows are loaded, added to the output and tiled), odd and single K blocks, GEMM2 with one K block and two
 (D = 4096) or five (D = 8192) tiles per CTA, five or nine per CTA pair, so that the ring in which a tile's place is handed over
-comes round between tiles with full and with padded warps.  Against the CPU emulation with the bars of the layer's tests (2e-2
+comes round between tiles with full and with padded warps, and GEMM1 with three tiles per CTA or five per pair (I = 2048), so that
+activation rows of a fuller tile are left in the stages.  Against the CPU emulation with the bars of the layer's tests (2e-2
 relative + 1e-2 absolute)."""
 import contextlib
 
@@ -18,7 +19,7 @@ COUNTS = [0, 1, 7, 8, 9, 16, 17, 31, 32, 33, 40, 0, 120, 121, 127, 128, 129, 136
 
 @pytest.mark.parametrize("option", ["none", "fixed_order", "pow2", "pairs"])
 @pytest.mark.parametrize("packed", [False, True])
-@pytest.mark.parametrize("D,I", [(768, 384), (4096, 128), (8192, 128)])
+@pytest.mark.parametrize("D,I", [(768, 384), (4096, 128), (8192, 128), (512, 2048)])
 def test_expert_row_counts_at_tile_edges(b200, cuda, D, I, packed, option):
     rng = np.random.default_rng(D + I)
     E, K = len(COUNTS), 2
