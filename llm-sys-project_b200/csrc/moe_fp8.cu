@@ -59,8 +59,7 @@ constexpr int DIRECT_ROWS = 16;              // GEMM2: rows of a warp up to whic
 constexpr int LAUNCH_REGS = 168;
 constexpr int PROMO_REGS = 232;
 constexpr int AUX_REGS = 40;
-// columns per promotion load (two loads in flight)
-constexpr int CH = 32;
+constexpr int CH = 32;                       // columns per promotion load (two loads in flight)
 constexpr int SW = 16;                       // columns per pass of the output transpose
 static_assert(QCOLS % (2 * CH) == 0, "promotion chunks");
 static_assert(NUM_PROMO_WARPS * (PROMO_REGS - LAUNCH_REGS) <= 4 * (LAUNCH_REGS - AUX_REGS), "setmaxnreg balance");
@@ -111,7 +110,6 @@ struct GemmParams {
     int* status;
     int E, D, I;
     int packed;                // weights pre-tiled: one contiguous 256 x 128-byte block per (expert, n tile, K block)
-    long long total_rows;      // capacity of the sorted row buffers
 #ifdef B200_GEMM_TRACE
     long long* trace;          // [8][TRACE_CAP] clock64 stamps of CTA 0's pipeline events (timeline builds only)
     int trace_warp;
@@ -297,12 +295,6 @@ __device__ __forceinline__ void promote(float* acc, const uint32_t (&v)[N], floa
                                                     ptx::pack_f32x2(acc[2 * i], acc[2 * i + 1]));
         ptx::unpack_f32x2(r, acc[2 * i], acc[2 * i + 1]);
     }
-}
-template <int N>
-__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[N]) {
-    if constexpr (N == 8) ptx::tmem_ld_32x8(taddr, r);
-    else if constexpr (N == 16) ptx::tmem_ld_32x16(taddr, r);
-    else ptx::tmem_ld_32x32(taddr, r);
 }
 
 // MODE 1: the tile's 256 accumulator columns are NQ groups [gate j0+g*QCOLS/2 .. | up j0+g*QCOLS/2 ..]
@@ -628,8 +620,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                     uint32_t ra[CH], rb[CH];
 #pragma unroll
                     for (int c = 0; c < NPAIR; c++) {
-                        tmem_ld_cols<CH>(t0 + 2 * c * CH, ra);
-                        tmem_ld_cols<CH>(t0 + 2 * c * CH + CH, rb);
+                        ptx::tmem_ld_32x32(t0 + 2 * c * CH, ra);
+                        ptx::tmem_ld_32x32(t0 + 2 * c * CH + CH, rb);
                         ptx::tc_wait_ld();
                         if (c == NPAIR - 1) {
                             ptx::tc_fence_before();
@@ -1446,7 +1438,7 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
     };
     CUtensorMap ta, ta32, ta8, tb;
     GemmParams p{};
-    p.offsets = s.offsets; p.E = E; p.D = D; p.I = I; p.status = ws->d_status; p.total_rows = TK;
+    p.offsets = s.offsets; p.E = E; p.D = D; p.I = I; p.status = ws->d_status;
 #ifdef B200_GEMM_TRACE
     p.trace = g_gemm_trace; p.trace_warp = g_gemm_trace_warp;
 #endif
