@@ -61,6 +61,7 @@ constexpr int PROMO_REGS = 232;
 constexpr int AUX_REGS = 40;
 constexpr int CH = 32;                       // columns per promotion load (two loads in flight)
 constexpr int SW = 16;                       // columns per pass of the output transpose
+constexpr int SC_RING = 4;                   // scales of four K blocks and the places of four tiles are in shared memory
 static_assert(QCOLS % (2 * CH) == 0, "promotion chunks");
 static_assert(NUM_PROMO_WARPS * (PROMO_REGS - LAUNCH_REGS) <= 4 * (LAUNCH_REGS - AUX_REGS), "setmaxnreg balance");
 static_assert(GEMM_THREADS * LAUNCH_REGS <= 65536, "register file");
@@ -72,6 +73,7 @@ struct GemmSmem {
     uint64_t tmem_empty[2];
     uint64_t amax_bar[2];
     uint64_t sf_full[STAGES];      // block-scaled kernel only: the stage's scale factors are in shared memory
+    uint64_t sc_free[SC_RING];     // CTA pairs: the promotion warps of this CTA have read the slot of the scale ring
     uint64_t pair_go;              // single-CTA tiles launched as clusters of two: the neighbour starts its tile
     uint32_t tmem_base;
     int abort_flag;
@@ -82,8 +84,7 @@ struct GemmSmem {
 };
 
 constexpr size_t GEMM_BASE_BYTES = 1024 /*alignment slack*/ + (size_t)STAGES * STAGE_BYTES + sizeof(GemmSmem);
-// scales of four K blocks, [K block % 4][gate / up or column half][row], and where four tiles lie
-constexpr int SC_RING = 4;
+// scales [K block % SC_RING][gate / up or column half][row], and where a tile lies [tile % SC_RING]
 constexpr size_t GEMM_SMEM_BYTES = GEMM_BASE_BYTES + sizeof(float) * SC_RING * 2 * BM + sizeof(int4) * SC_RING;
 static_assert(GEMM_SMEM_BYTES <= 232448, "shared memory budget of one CTA");
 // block-scaled kernel: per stage one 512-byte scale atom for the 128 rows of A and two for the 256 rows of B
@@ -162,10 +163,13 @@ __device__ __forceinline__ uint32_t map_to_cta(const void* p, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(ptx::smem_u32(p)), "r"(rank));
     return r;
 }
-// Arrival on a barrier of the pair's other CTA: a TMEM stage whose reads have completed (tcgen05.wait::ld +
-// tcgen05.fence::before_thread_sync) and the scales that were read with it.
+// Arrival on a barrier of the pair's other CTA.  What it hands over is a TMEM stage whose reads have completed
+// (tcgen05.wait::ld + tcgen05.fence::before_thread_sync) and no memory: the scales that were read with the stage go back inside the
+// CTA (sc_free).  With .release.cluster, which would let the leader hand the scales back too, the arrival waits until all that the warp did
+// in memory is visible to the other CTA: a K block of a pair then takes 1950 - 2280 cycles instead of 950 - 980 (32 experts x 1024
+// rows 3.75 ms against 2.40, T = 4096 6.8 against 4.4).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void mbar_expect_tx_cluster(uint32_t cluster_addr, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_addr),
@@ -342,6 +346,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
             ptx::mbar_init(&sm->tmem_empty[a], PAIR ? 2 * NUM_PROMO_WARPS : NUM_PROMO_WARPS);
             ptx::mbar_init(&sm->amax_bar[a], NUM_PROMO_WARPS);
         }
+        for (int i = 0; i < SC_RING; i++) ptx::mbar_init(&sm->sc_free[i], NUM_PROMO_WARPS);
         ptx::mbar_init(&sm->pair_go, 1);
         sm->abort_flag = 0;
         ptx::fence_mbar_init();
@@ -473,14 +478,14 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                 for (int kb = 0; kb < nkb; kb++, g++) {
                     if ((int)(g & 1) == role) {
                         // The operands first: they are there long before the stage is handed back, which starts the critical path.
-                        // (`full` hands over TMA-written tiles.  `tmem_empty` of a pair also hands back the peer's slots of the scale
-                        // ring, which this thread passes on with the commit: it acquires at cluster scope, and so does the scale warp.)
+                        // (waits on barriers that the peer CTA or tcgen05.commit signal need no cluster-scope
+                        // acquire: what they hand over is a TMEM stage or TMA-written tiles, not memory data)
                         if (!ptx::whole_warp(ptx::mbar_wait(&sm->full[s], ph, abort_flag))) goto done;
                         TRACE_STAMP(0, g);
                         const uint32_t a_addr = ptx::smem_u32(tiles + (size_t)s * STAGE_BYTES);
                         const uint64_t ad = ptx::make_smem_desc(a_addr, 16, 1024, 2), bd = ptx::make_smem_desc(a_addr + A_BYTES, 16, 1024, 2);
                         const uint32_t d_tmem = tmem_base + role * BN;
-                        if (!ptx::whole_warp(ptx::mbar_wait<PAIR>(&sm->tmem_empty[role], acc_ph ^ 1, abort_flag))) goto done;
+                        if (!ptx::whole_warp(ptx::mbar_wait(&sm->tmem_empty[role], acc_ph ^ 1, abort_flag))) goto done;
                         TRACE_STAMP(1, g);
                         ptx::tc_fence_after();
                         if (ptx::elect_one()) {
@@ -537,8 +542,11 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                 }
             };
             auto publish = [&](float (&av)[4], float (&wv)[2], bool first) -> bool {
-                // This slot's last K block, g - 4, has been read once the MMAs of block g - 2 have run: they waited for it.
-                if (g >= 2 && !ptx::whole_warp(ptx::mbar_wait<PAIR>(&sm->tmem_full[g & 1], ((g >> 1) & 1) ^ 1, abort_flag))) return false;
+                // Block g - 2 is through with this barrier, and with single-CTA tiles the slot's last K block, g - 4, has been read: the
+                // MMAs of block g - 2 waited for that.  In a pair the leader's MMAs wait on an arrival that orders no memory of the peer,
+                // so there each CTA's promotion warps hand the slot back themselves.
+                if (g >= 2 && !ptx::whole_warp(ptx::mbar_wait(&sm->tmem_full[g & 1], ((g >> 1) & 1) ^ 1, abort_flag))) return false;
+                if (PAIR && g >= SC_RING && !ptx::whole_warp(ptx::mbar_wait(&sm->sc_free[g % SC_RING], ((g / SC_RING) & 1) ^ 1, abort_flag))) return false;
                 float (*const sc)[BM] = scales[g % SC_RING];
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
@@ -582,7 +590,8 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         // the stage's "free" barrier lives in the leader CTA
         const uint32_t tmem_empty_addr[2] = {PAIR ? map_to_cta(&sm->tmem_empty[0], 0) : 0u,
                                              PAIR ? map_to_cta(&sm->tmem_empty[1], 0) : 0u};
-        auto release_stage = [&](int a) {
+        auto release_stage = [&](int a, uint32_t g) {                // one lane; all of the warp's reads are behind a __syncwarp
+            if (PAIR) ptx::mbar_arrive(&sm->sc_free[g % SC_RING]);
             if (PAIR && crank != 0) mbar_arrive_cluster(tmem_empty_addr[a]);
             else                    ptx::mbar_arrive(&sm->tmem_empty[a]);
         };
@@ -626,7 +635,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                         if (c == NPAIR - 1) {
                             ptx::tc_fence_before();
                             __syncwarp();
-                            if (lane == 0) release_stage(acc);   // the stage is in registers now
+                            if (lane == 0) release_stage(acc, gsc);   // the stage is in registers now
 #ifdef B200_GEMM_TRACE
                             if (trw) TRACE_STAMP(4, gp);
 #endif
@@ -637,7 +646,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
                 } else {
                     ptx::tc_fence_before();
                     __syncwarp();                            // (every lane has read tile_at)
-                    if (lane == 0) release_stage(acc);
+                    if (lane == 0) release_stage(acc, gsc);
                 }
 #ifdef B200_GEMM_TRACE
                 if (trw) TRACE_STAMP(5, gp);
