@@ -396,7 +396,8 @@ int dsa_bf16_impl(b200_ws* ws, const uint16_t* q_nope, const uint16_t* q_pe, con
     if (!ws) return B200_CUDA_ERROR;
 
     // The CTA-pair kernels take every shape with S % 64 == 0 (128-row tiles when S % 128 == 0, else
-    // 64-row tiles); the single-CTA kernel (32-row tiles) takes the rest.
+    // 64-row tiles); the single-CTA kernel (32-row tiles) takes the rest.  1 / 16 / 64 queries, us: 128-row tiles (S = 2048)
+    // 17 / 34 / 64, 64-row tiles 27 / 69 / 206, single CTA (S = 2016) 38 / 92 / 285.
     const bool use_pair = (S % 64 == 0);
     const int pair_tile = (S % 128 == 0) ? 128 : 64;
     // split the selected rows so that the grid covers the machine about once

@@ -459,11 +459,13 @@ done:
 
 
 // =================================================================================================
-// 128-row tiles.  Issued by one lane of a diverged warp, an MMA took ~45 ns whatever its shape, so the 36 K-steps of Q K^T cost the
-// same for 64 rows as for 128: with 64-row tiles the issue, not HBM, bounded the kernel.  The warp now issues as a whole (an elected
-// lane, descriptors in uniform registers; 64 queries x 2048 rows 71.8 -> 64.0 us), and what is left of a tile is the refill of its single
-// K and V stages behind the MMAs that read them.  (Handing the stages over in halves: 5 queries 19.6 -> 18.8 us, 64 queries 72.7 us, the
-// rows then come in pieces of 512 and 256 bytes.)  Here a tile is 128 selected rows (N = 128 for Q K^T, eight
+// 128-row tiles, wherever S allows them: at S = 2048 the 64-row kernel above takes 27 / 40 / 69 / 206 us for 1 / 5 / 16 / 64 queries
+// (launched programmatically like this one), this one 17 / 23 / 34 / 64.  The warp issues MMAs as a whole (an elected lane, descriptors in
+// uniform registers; 64 queries 71.8 -> 64.0 us against one lane of a diverged warp).  What a tile of a full batch waits for (clock
+// stamps, ~4900 - 5300 cycles): the refill of the single K stage behind the MMAs that read it -- 900 to issue them, 600 until they are
+// done, 1200 for the gather warps to request the next rows, 1000 until they are there, 1250 until the peer's half is known to the leader.
+// (Handing the stages over in halves: 5 queries 19.6 -> 18.8 us, 64 queries 72.7 us, the
+// rows then come in pieces of 512 and 256 bytes.)  A tile is 128 selected rows (N = 128 for Q K^T, eight
 // K-steps per P V half), which leaves room for one K stage (72 KB) and one V stage (64 KB) per CTA next
 // to Q (72 KB) and P (16 KB).  The K stage refills while P V of the previous tile and the softmax run,
 // the V stage while Q K^T of the next tile runs; K and V have their own gather warps so that neither

@@ -15,8 +15,8 @@
 //                          the bit-reproducible alternative to the scatter-add.
 //
 // GEMM structure (one CTA per SM, 384 threads, tiles 128 x 256 x 128 handed out round-robin,
-// expert-major; E = 256, K = 8, D = 7168, I = 2048, a GPU that has just begun: T = 16 813 -> 733 us a call, T = 333 2070 -> 1905,
-// T = 4096 3235 -> 3010; 32 experts x 1024 rows 2095 -> 1950, before and after what the comments below measure):
+// expert-major; E = 256, K = 8, D = 7168, I = 2048, a GPU that has just begun: T = 16 813 -> 733 us a call, T = 333 2070 -> 1876,
+// T = 4096 3235 -> 2985; 32 experts x 1024 rows 2095 -> 1915, before and after what the comments below measure):
 //   warp 8       TMA producer: A tile (128 rows x 128 B) and B tile (256 rows x 128 B) per
 //                K block into a 4-stage shared-memory ring (128-byte swizzle, K-major).
 //   warps 9,10   MMA issuers, one per 256-column TMEM accumulator stage (K blocks alternate between
@@ -271,7 +271,7 @@ __device__ __forceinline__ void wait_for_gemm1() {
 // would bring the next experts' rows along, a third of the stage's bytes.  The rows of the stage that are not loaded hold
 // zeros until a fuller tile has been there (clear_a_tiles), then older bytes; their products go to accumulator rows that
 // nobody reads, but multiplying zeros takes less power, and under sustained load power is what sets the clock.  Groups
-// of 32 and no zeros: T = 16 748 us, T = 333 1950 us, T = 1024 2024 us; with zeros 733, 1904, 1985.
+// of 32 and no zeros: T = 16 748 us, T = 333 1950 us, T = 1024 2024 us; with zeros 733, 1905, 2015.
 __device__ __forceinline__ uint32_t a_tile_bytes(int rows) { return rows > BM - 8 ? (uint32_t)A_BYTES : (uint32_t)((rows + 7) >> 3) * 8u * BK; }
 __device__ __forceinline__ void load_a_rows(uint8_t* dst, const CUtensorMap* map128, const CUtensorMap* map32, const CUtensorMap* map8, uint64_t* bar,
                                             int x, int row0, uint32_t bytes) {
@@ -309,11 +309,14 @@ __device__ __forceinline__ void promote(float* acc, const uint32_t (&v)[N], floa
 // PAIR: two CTAs of a cluster (two SMs) work on one tile of 256 rows with tcgen05.mma.cta_group::2: CTA r holds
 // rows 128 r .. +127 (its own A tile and accumulator) and HALF of the tile's weight rows (accumulator columns
 // 128 r .. +127), so per K block each SM writes and reads 32 KB of shared memory instead of 48 KB, and a
-// weight tile crosses L2 -> shared memory once per 256 rows.  Shared-memory bandwidth (TMA fill + MMA operand
-// reads: 96 KB per K block for a single-CTA 128 x 256 tile, 768 cycles at 128 B/clk against 546 cycles of
-// tensor time) is what bounds the single-CTA kernel.  The leader CTA (rank 0) issues the MMAs; both CTAs'
+// weight tile crosses L2 -> shared memory once per 256 rows.  The leader CTA (rank 0) issues the MMAs; both CTAs'
 // loads complete on the leader's `full` barrier, both CTAs' promotion warps release the accumulator stage on
 // the leader's `tmem_empty` barrier, and tcgen05.commit signals `empty` / `tmem_full` in both CTAs.
+//
+// What bounds a K block (GEMM1, 32 experts x 1024 rows, single-CTA tiles, clock stamps): 880 cycles as built, 880 without any TMA
+// load, 560 with the loads but promotion warps that only hand the stage back, 520 with neither, 840 without the multiplications.
+// So it is the round trip of an accumulator stage -- MMAs, commit, tcgen05.ld, release -- with two stages to hide it in, not shared
+// memory (96 KB per K block pass in the 560), the weight stream or the multiplications.
 template <int MODE, bool PAIR>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_a32,
@@ -659,7 +662,7 @@ grouped_gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
 #endif
 
             if (MODE == 1) {
-                // SwiGLU on 32 activation columns, 1x128 requantisation shared with the three other quarters.
+                // SwiGLU on 64 activation columns, 1x128 requantisation shared with the other half's warp.
                 // Fast exp / reciprocal: the result is rounded to e4m3 next, an ulp of fp32 does not matter.
                 constexpr int AC = QCOLS / 2;          // activation columns of this thread
                 float amax = 0.0f;
@@ -1401,9 +1404,10 @@ int run_experts(b200_ws* ws, const Fp8Scratch& s, const uint8_t* xq, const float
     const int slot = prof ? (int)(prof->calls % PROF_SLOTS) : 0;
     // Single-CTA 128-row tiles unless the caller asks for CTA pairs.  Measured on B200 the pair tiles (256 rows,
     // half of the weight tile per SM, a third less shared-memory traffic) are slower at every shape tried
-    // (config 3: GEMM1 3.0 vs 2.2 ms; 32 experts x 1024 rows: 1.9 vs 1.3 ms): the K-block period is set by the
-    // promotion of the accumulator stage through tcgen05.ld, which is the same per SM in both shapes, not by
-    // shared-memory bandwidth, and a pair idles half of its rows on experts with fewer than 129 rows.
+    // (E = 256, K = 8, D = 7168, I = 2048: T = 333 3.5 against 1.8 - 1.9 ms, T = 4096 4.3 - 4.5 against 3.2 - 3.4; 32 experts x 1024
+    // rows 2.4 against 2.0): the K-block period is the round trip of an accumulator stage, which is longer across two
+    // CTAs (950 - 980 against 880 cycles) and is not helped by less shared-memory traffic, and a pair idles half of its rows on
+    // experts with fewer than 129 rows.
     const bool mx = (cfg->flags & B200_MOE_POW2_SCALES) != 0;      // power-of-two scales: hardware block-scaled MMA
     bool pair = (cfg->flags & B200_MOE_CTA_PAIR_TILES) != 0;
     if ((cfg->flags & B200_MOE_SINGLE_CTA_TILES) || mx) pair = false;
